@@ -55,7 +55,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
 
 template <typename R, int ADV, bool SGS>
 struct TileShape {
-    static constexpr int TX = 32, TY = 8, NT = TX * TY;
+    // WENO in FP64 runs two threads a cell (u, v and w, theta): its planes and
+    // fluxes leave room for one CTA an SM, and eight warps of dependent FP64
+    // chains kept the pipe a third busy
+    static constexpr bool SHARE = ADV > 0 && sizeof(R) == 8;
+    static constexpr int TX = 32, TY = 8, PARTS = SHARE ? 2 : 1, NT = TX * TY * PARTS;
     static constexpr int HH = ADV ? 3 : 2;               // xy halo of the planes
     static constexpr int ZL = ADV ? 3 : (SGS ? 2 : 1);   // levels below the point
     static constexpr int ZH = ADV ? 3 : (SGS ? 2 : 1);   // levels above
@@ -76,7 +80,6 @@ struct TileShape {
     // [4][TY+1][TX], computed once per face; FP32 reconstructions are cheap
     // enough that recomputing a face in both cells (straight-line code, no
     // extra barrier) is faster
-    static constexpr bool SHARE = ADV > 0 && sizeof(R) == 8;
     static constexpr int FXN = TY * (TX + 1), FYN = (TY + 1) * TX;
     static constexpr int FPF = 576;                      // face entries per field: x 264 padded to 288, y 288
     static constexpr size_t FLUX_BYTES = SHARE ? (((size_t)4 * (FXN + FYN) * sizeof(R) + 127) / 128) * 128 : 0;
@@ -92,7 +95,7 @@ struct TileShape {
     static constexpr size_t KT_BYTE = ((SMEM - 128 + 127) / 128) * 128;
     static constexpr int KT_OFS = (int)((KT_BYTE - PLANES_BYTES) / sizeof(R));   // elements past nutp
     static constexpr size_t SMEM_AMD = KT_BYTE + NUT_BYTES + 128;
-    static_assert(!ADV || (FPF % 32 == 0 && FXN <= FPF / 2 && FYN == FPF / 2 && (4 * FPF) % NT == 0),
+    static_assert(!ADV || (FPF % 32 == 0 && FXN <= FPF / 2 && FYN == FPF / 2 && (4 * FPF) % 32 == 0),
                   "one field per warp in the face phase");
 };
 
@@ -129,7 +132,7 @@ struct NutAcc {
 // elements past the nut planes), 2 dynamic Smagorinsky (cs2 per level or
 // cell), 3 the TKE closure (tke_point; its kappa_t planes as the AMD's)
 template <typename R, int ADV, bool SGS, bool ANEL, bool UNI, int CLOS = 0>
-__global__ void __launch_bounds__(256) sweep_tile_kernel(const __grid_constant__ TileMaps maps, SweepArgs<R> a,
+__global__ void __launch_bounds__(TileShape<R, ADV, SGS>::NT) sweep_tile_kernel(const __grid_constant__ TileMaps maps, SweepArgs<R> a,
                                                          int kchunk, int* err) {
     using S = TileShape<R, ADV, SGS>;
     extern __shared__ __align__(128) unsigned char smem_tile[];
@@ -144,7 +147,8 @@ __global__ void __launch_bounds__(256) sweep_tile_kernel(const __grid_constant__
     R* lvs = reinterpret_cast<R*>(sbase + S::PLANES_BYTES + S::NUT_BYTES + S::FLUX_BYTES + S::BAR_BYTES);
 
     const Geo& g = a.g;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + S::TX * ty;
+    const int tid = threadIdx.x;
+    const int tx = tid & (S::TX - 1), ty = (tid / S::TX) & (S::TY - 1), part = tid / (S::TX * S::TY);
     const int i0 = blockIdx.x * S::TX, j0 = blockIdx.y * S::TY;
     const int kbeg = blockIdx.z * kchunk;
     const int kend = min(g.nz, kbeg + kchunk);
@@ -289,12 +293,11 @@ __global__ void __launch_bounds__(256) sweep_tile_kernel(const __grid_constant__
             const R* lp0[S::NW];
 #pragma unroll
             for (int d = 0; d < S::NW; ++d) lp0[d] = plane(k - S::ZL + d);
-#pragma unroll 3
-            for (int q = 0; q < 4 * S::FPF / S::NT; ++q) {
+#pragma unroll 2
+            for (int e = tid; e < 4 * S::FPF; e += S::NT) {
                 // branch-free: an x face and a y face differ only in the stencil
                 // stride and the advecting field (u or v); the second velocity
                 // point depends on the field only (f is warp-uniform, so is isx)
-                const int e = tid + q * S::NT;
                 const int f = e / S::FPF, r = e - f * S::FPF;
                 const bool isx = r < S::FPF / 2;
                 int rr = isx ? r : r - S::FPF / 2;
@@ -318,29 +321,55 @@ __global__ void __launch_bounds__(256) sweep_tile_kernel(const __grid_constant__
                     else fys[f * S::FYN + fj * S::TX + fi] = flux;
                 }
             }
-            __syncthreads();
+            // the z fluxes of the thread's cell and two fields, before the barrier:
+            // they need no face flux
+            R dzf[2];
             if (active) {
-                // cell phase: differences of the shared fluxes, the z fluxes carried up the column
-                const R idx = R(g.idx), idy = R(g.idy), idz = R(g.idz);
-                R adv[4];
 #pragma unroll
-                for (int f = 0; f < 4; ++f) {
+                for (int h = 0; h < 2; ++h) {
+                    const int f = 2 * part + h;
                     const SmAccF<R, S::ZL, S::PW> F{lp, f * S::PSZA};
                     const R ft = weno_zflux<R, ADV, 0>(f, W, F);
-                    const R fb = zc.valid ? zc.f[f] : weno_zflux<R, ADV, -1>(f, W, F);
-                    zc.f[f] = ft;
-                    const R* fx = fxs + f * S::FXN + ty * (S::TX + 1) + tx;
-                    const R* fy = fys + f * S::FYN + ty * S::TX + tx;
-                    adv[f] = R(0) - ((fx[1] - fx[0]) * idx + (fy[S::TX] - fy[0]) * idy + (ft - fb) * idz);
+                    const R fb = zc.valid ? zc.f[h] : weno_zflux<R, ADV, -1>(f, W, F);
+                    zc.f[h] = ft;
+                    dzf[h] = ft - fb;
                 }
                 zc.valid = true;
-                tu = adv[0]; tv = adv[1]; tw = adv[2]; tt = adv[3];
             }
-        }
-        if (active) {
-            sweep_point<R, ADV, SGS, ANEL, UNI, S::SHARE, CLOS == 1 || CLOS == 3>(m, a, g, k, U, V, W, T, N, tu, tv, tw, tt,
-                                                               (ADV > 0 && !S::SHARE) ? &zc : nullptr);
-            if (ADV > 0 && !S::SHARE) zc.valid = true;
+            __syncthreads();
+            if (active) {
+                // cell phase: differences of the shared fluxes and the thread's z fluxes
+                const R idx = R(g.idx), idy = R(g.idy), idz = R(g.idz);
+                R adv[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int f = 2 * part + h;
+                    const R* fx = fxs + f * S::FXN + ty * (S::TX + 1) + tx;
+                    const R* fy = fys + f * S::FYN + ty * S::TX + tx;
+                    adv[h] = R(0) - ((fx[1] - fx[0]) * idx + (fy[S::TX] - fy[0]) * idy + dzf[h] * idz);
+                }
+                const long long qi = iidx(g, i, j, k), q = pidx(g, i, j, k);
+                // the rest of the tendency, of the thread's two fields (the other two are dead code)
+                if (part == 0) {
+                    tu = adv[0]; tv = adv[1]; tw = tt = R(0);
+                    sweep_point<R, ADV, SGS, ANEL, UNI, true, CLOS == 1 || CLOS == 3>(m, a, g, k, U, V, W, T, N, tu, tv,
+                                                                                     tw, tt);
+                    a.us[qi] = U(0, 0, 0) + dt * tu;
+                    a.vs[qi] = V(0, 0, 0) + dt * tv;
+                } else {
+                    tu = tv = R(0); tw = adv[0]; tt = adv[1];
+                    sweep_point<R, ADV, SGS, ANEL, UNI, true, CLOS == 1 || CLOS == 3>(m, a, g, k, U, V, W, T, N, tu, tv,
+                                                                                     tw, tt);
+                    a.ws[qi] = (g.bc_z == 1 && k == 0) ? R(0) : W(0, 0, 0) + dt * tw;
+                    R tn = T(0, 0, 0) + dt * tt;
+                    if (a.stage) tn = rk_combine(a.ca, a.cb, a.th0[q], tn);
+                    a.th_out[q] = tn;
+                }
+            }
+        } else if (active) {
+            sweep_point<R, ADV, SGS, ANEL, UNI, false, CLOS == 1 || CLOS == 3>(m, a, g, k, U, V, W, T, N, tu, tv, tw, tt,
+                                                                              ADV > 0 ? &zc : nullptr);
+            if (ADV > 0) zc.valid = true;
             const long long qi = iidx(g, i, j, k), q = pidx(g, i, j, k);
             a.us[qi] = U(0, 0, 0) + dt * tu;
             a.vs[qi] = V(0, 0, 0) + dt * tv;

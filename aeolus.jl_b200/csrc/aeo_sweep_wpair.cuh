@@ -23,8 +23,7 @@
 //
 // The advecting velocity of a face and the face value multiply exactly as in
 // the FP64 shared-face form (aeo_sweep_tile.cuh), so the two precisions run
-// the same expression tree; the WENO divisions are a reciprocal and a product
-// (2 ulp; every denominator lies in the normal range, as for wdiv).
+// the same expression tree (weno5_left, aeo_sweep.cuh).
 //
 // Waits are bounded (AEO_WAIT_LIMIT): a CTA whose plane did not arrive
 // records AEO_ERR_FLAG_TMA, drains the copies it issued (bounded) and returns.
@@ -36,61 +35,19 @@
 __device__ __forceinline__ F2 ld2s(const float* p) { return F2(*reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ float2 ldf2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ F2 f2abs(F2 x) { return F2(fabsf(x.v.x), fabsf(x.v.y)); }
-// a / b as a times the approximate reciprocal of b (rcp.approx, 1 ulp; the
-// quotient within 2 ulp, as __fdividef), the two products one paired multiply
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ F2 f2wdiv(F2 a, F2 b) { return F2(a * F2(rcp_approx(b.v.x), rcp_approx(b.v.y))); }
+__device__ __forceinline__ F2 wabs(F2 x) { return f2abs(x); }
+__device__ __forceinline__ F2 wrcp(F2 x) { return F2(wrcp(x.v.x), wrcp(x.v.y)); }
+template <>
+struct WScalar<F2> { using type = float; };
 __device__ __forceinline__ F2 f2pick(bool px, bool py, F2 a, F2 b) {
     return F2(px ? a.v.x : b.v.x, py ? a.v.y : b.v.y);
-}
-
-// weno5_left (aeo_sweep.cuh) on two faces
-template <int ADV>
-__device__ __forceinline__ F2 weno5_left_f2(F2 v1, F2 v2, F2 v3, F2 v4, F2 v5) {
-    // the candidate values as the integer combinations over 6 (rounded
-    // coefficients 1/3, 7/6, 11/6 would not sum to one, and a uniform field
-    // would reconstruct with a bias that drifts the kinetic energy); the half
-    // second differences with the 1/2 folded in (exact for a uniform field)
-    const F2 s6(float(1.0 / 6.0)), two(2.f), half(0.5f), c133(float(13.0 / 3.0));
-    const F2 q0 = F2(two * v1 - F2(7.f) * v2 + F2(11.f) * v3) * s6;
-    const F2 q1 = F2(F2(5.f) * v3 - v2 + two * v4) * s6;
-    const F2 q2 = F2(two * v3 + F2(5.f) * v4 - v5) * s6;
-    const F2 d2a = half * (v1 + v3) - v2;
-    const F2 d2b = half * (v2 + v4) - v3;
-    const F2 d2c = half * (v3 + v5) - v4;
-    const F2 e0 = F2(v1 - F2(4.f) * v2 + F2(3.f) * v3) * half;
-    const F2 e1 = (v4 - v2) * half;
-    const F2 e2 = F2(F2(4.f) * v4 - F2(3.f) * v3 - v5) * half;
-    const F2 b0 = e0 * e0 + c133 * (d2a * d2a);
-    const F2 b1 = e1 * e1 + c133 * (d2b * d2b);
-    const F2 b2 = e2 * e2 + c133 * (d2c * d2c);
-    F2 a0, a1, a2;
-    if constexpr (ADV == 2) {   // WENO-Z5, p = 2, eps = eps(Float32)^2
-        const F2 eps(1.4210854715202004e-14f), one(1.f);
-        const F2 tau = f2abs(b0 - b2);
-        const F2 t0 = f2wdiv(tau, b0 + eps), t1 = f2wdiv(tau, b1 + eps), t2 = f2wdiv(tau, b2 + eps);
-        a0 = F2(0.1f) * (one + t0 * t0);
-        a1 = F2(0.6f) * (one + t1 * t1);
-        a2 = F2(0.3f) * (one + t2 * t2);
-    } else {                    // WENO-JS5, eps = 1e-6
-        const F2 e(1e-6f);
-        const F2 s0 = b0 + e, s1 = b1 + e, s2 = b2 + e;
-        a0 = f2wdiv(F2(0.1f), s0 * s0);
-        a1 = f2wdiv(F2(0.6f), s1 * s1);
-        a2 = f2wdiv(F2(0.3f), s2 * s2);
-    }
-    return f2wdiv(a0 * q0 + a1 * q1 + a2 * q2, a0 + a1 + a2);
 }
 
 // the upwinded value of two faces (weno_upwind lane by lane)
 template <int ADV>
 __device__ __forceinline__ F2 weno_upwind_f2(F2 vel, F2 f0, F2 f1, F2 f2, F2 f3, F2 f4, F2 f5) {
     const bool px = vel.v.x >= 0.f, py = vel.v.y >= 0.f;
-    return weno5_left_f2<ADV>(f2pick(px, py, f0, f5), f2pick(px, py, f1, f4), f2pick(px, py, f2, f3),
+    return weno5_left<F2, ADV>(f2pick(px, py, f0, f5), f2pick(px, py, f1, f4), f2pick(px, py, f2, f3),
                               f2pick(px, py, f3, f2), f2pick(px, py, f4, f1));
 }
 

@@ -765,23 +765,29 @@ struct Core : CoreBase {
             if (aeo_status e = lag_refresh()) return e;
         }
         if (aeo_status e = make_tensor_maps()) return e;
-        kchunk = std::min(g.nz, TileShape<R, 0, false>::KCH);
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cfg.device));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fin_per_sm, finite_check_kernel<R>, 256, 0));
         fin_per_sm = std::max(fin_per_sm, 1);
         {
-            // the paired WENO sweep: the chunk length that minimises whole waves x
-            // (levels + the 6-plane start of a chunk)
-            const long long tiles = (long long)((g.nx + WPairShape::TX - 1) / WPairShape::TX) *
-                                    ((g.ny + WPairShape::TY - 1) / WPairShape::TY);
-            const long long slots = (long long)WPairShape::CTAS_PER_SM * nsm;
-            long long best = -1;
-            for (int c : {16, 32, 64}) {
-                const int kc = std::min(c, g.nz);
-                const long long waves = (tiles * ((g.nz + kc - 1) / kc) + slots - 1) / slots;
-                const long long cost = waves * (kc + 6);
-                if (best < 0 || cost < best) { best = cost; wchunk = kc; }
-            }
+            // the tiled sweeps' chunk: CTAs of a tile column each march kc levels, so kc
+            // that minimises whole waves x (levels + what a chunk's start costs: its
+            // first planes' load, the eddy viscosity or z fluxes of two more levels).
+            // Fixed 32-level chunks gave a 64^3 grid 32 CTAs on 148 SMs.
+            auto chunk = [&](int tx, int ty, int slots, int kmax, int start) {
+                const long long tiles = (long long)((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty);
+                long long best = -1;
+                int pick = 1;
+                for (int kc = std::min(2, g.nz); kc <= std::min(kmax, g.nz); ++kc) {
+                    const long long waves = (tiles * ((g.nz + kc - 1) / kc) + slots - 1) / slots;
+                    const long long cost = waves * (kc + start);
+                    if (best < 0 || cost <= best) { best = cost; pick = kc; }
+                }
+                return pick;
+            };
+            using T0 = TileShape<R, 0, false>;
+            const int tile_ctas = cfg.advection != AEO_ADV_CENTRED ? 1 : 2;
+            kchunk = chunk(T0::TX, T0::TY, tile_ctas * nsm, T0::KCH, 2);
+            wchunk = chunk(WPairShape::TX, WPairShape::TY, WPairShape::CTAS_PER_SM * nsm, 64, 6);
         }
         CK(cudaStreamSynchronize(st));
         launches = 3 * (9 + dyn_launches()) + lag_launches() + tke_launches();
@@ -1386,7 +1392,7 @@ struct Core : CoreBase {
                 b.kofs = TS::KT_OFS;
                 cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM_AMD);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 1><<<grid, dim3(TS::TX, TS::TY), TS::SMEM_AMD, st>>>(
+                sweep_tile_kernel<R, ADV, SG, AN, UN, 1><<<grid, TS::NT, TS::SMEM_AMD, st>>>(
                     tmaps[s_in], b, kchunk, d_flag);
                 return;
             }
@@ -1397,7 +1403,7 @@ struct Core : CoreBase {
                 b.kofs = TS::KT_OFS;
                 cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 3>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM_AMD);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 3><<<grid, dim3(TS::TX, TS::TY), TS::SMEM_AMD, st>>>(
+                sweep_tile_kernel<R, ADV, SG, AN, UN, 3><<<grid, TS::NT, TS::SMEM_AMD, st>>>(
                     tmaps[s_in], b, kchunk, d_flag);
                 return;
             }
@@ -1406,14 +1412,14 @@ struct Core : CoreBase {
             if (dyncl()) {
                 cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 2><<<grid, dim3(TS::TX, TS::TY), TS::SMEM, st>>>(
+                sweep_tile_kernel<R, ADV, SG, AN, UN, 2><<<grid, TS::NT, TS::SMEM, st>>>(
                     tmaps[s_in], a, kchunk, d_flag);
                 return;
             }
         }
         const size_t sm = TS::SMEM;
         cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        sweep_tile_kernel<R, ADV, SG, AN, UN><<<grid, dim3(TS::TX, TS::TY), sm, st>>>(tmaps[s_in], a, kchunk, d_flag);
+        sweep_tile_kernel<R, ADV, SG, AN, UN><<<grid, TS::NT, sm, st>>>(tmaps[s_in], a, kchunk, d_flag);
     }
 
     aeo_status launch_sweep(int s_in, const SweepArgs<R>& a) {

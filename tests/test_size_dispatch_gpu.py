@@ -1,0 +1,77 @@
+"""The kernels chosen by size, at the sizes where they can go wrong.
+
+Tolerances: FP64 rounding of the path times a small factor (WENO steps and
+transforms 1e-11 as the parity tests), FP32-mixed 1e-5 against FP64.
+"""
+import numpy as np
+import pytest
+
+from aeolus_b200 import CoreSpec, regular_grid
+from aeolus_b200.inputs import embed, taylor_green
+from oracle.oracle import OracleSimulation
+
+pytestmark = pytest.mark.gpu
+
+
+def Sim(spec):
+    from aeolus_b200.simulation import Simulation
+    return Simulation(spec)
+
+
+def rel(a, b):
+    n = np.linalg.norm(b)
+    return np.linalg.norm(a - b) / (n if n > 0 else 1.0)
+
+
+def random_state(g, seed, amp=1.0):
+    rng = np.random.default_rng(seed)
+    f = [embed(g, amp * rng.standard_normal((g.nz, g.ny, g.nx))) for _ in range(4)]
+    if g.bc_z == "wall":
+        f[2][g.halo[2]] = 0.0
+    return f
+
+
+# ---- the tiled WENO sweeps: tiles of 32 x 8 cells, chunks of levels by the number of tiles ---------------------
+@pytest.mark.parametrize("size,bc_z", [((16, 4, 5), "wall"), ((32, 8, 2), "periodic"), ((64, 16, 13), "wall"),
+                                       ((32, 32, 64), "periodic")])
+@pytest.mark.parametrize("scheme", ["weno_js5", "weno_z5"])
+@pytest.mark.parametrize("c_s", [0.0, 0.17])
+def test_weno_steps_at_tile_and_chunk_edges(size, bc_z, scheme, c_s):
+    g = regular_grid(size, (2 * np.pi,) * 3, bc_z=bc_z)
+    kw = dict(grid=g, advection=scheme, nu=1e-3, c_s=c_s, theta0=300.0 if bc_z == "wall" else 0.0)
+    state = random_state(g, 5, 0.5)
+    o = OracleSimulation(CoreSpec(**kw))
+    s64, s32 = Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
+    for s in (o, s64, s32):
+        s.set_state(*state)
+        s.project()
+        s.step_rk3(1e-3, 3)
+    for n in ("u", "v", "w", "theta", "p"):
+        want = o.get_field(n)[g.interior]
+        assert rel(s64.get_field(n)[g.interior], want) <= 1e-11, n
+        # the pressure is phi / dt: the FP32 divergence's rounding over it
+        assert rel(s32.get_field(n)[g.interior], want) <= (1e-5 if n != "p" else 1e-3), n
+
+
+@pytest.mark.parametrize("scheme", ["weno_js5", "weno_z5"])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("fp32_mixed", 1e-6)])
+def test_weno_keeps_a_uniform_field_and_scales(scheme, precision, tol):
+    """A uniform wind carries a uniform scalar unchanged, whatever its size, and the reconstruction of a field
+    scaled by a power of two is the scaled one where its indicators stand far above eps."""
+    g = regular_grid((32, 16, 16), (1.0, 1.0, 1.0))
+    one = np.ones(g.storage_shape)
+    for scale in (1e-6, 1.0, 1e6):
+        s = Sim(CoreSpec(grid=g, advection=scheme, precision=precision))
+        s.set_state(one, 0.5 * one, -0.25 * one, scale * one)
+        s.step_rk3(1e-3, 2)
+        assert np.abs(s.get_field("theta")[g.interior] / scale - 1).max() <= tol
+        assert np.abs(s.get_field("u")[g.interior] - 1).max() <= tol
+    rng = np.random.default_rng(3)
+    th = embed(g, rng.standard_normal((g.nz, g.ny, g.nx)))
+    out = []
+    for scale in (1.0, 2.0 ** 24):
+        s = Sim(CoreSpec(grid=g, advection="weno_z5", precision=precision))
+        s.set_state(one, 0.5 * one, -0.25 * one, scale * th)
+        s.step_rk3(1e-3)
+        out.append(s.get_field("theta")[g.interior] / scale)
+    assert rel(out[1], out[0]) <= (1e-12 if precision == "fp64" else 1e-5)
