@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) cc_correct_kernel(Geo g, const R* __restr
     uo[qp] = un;
     vo[qp] = vn;
     wo[qp] = wn;
-    p[q] = R(pc / __ldg(dtp));   // p = phi/dt (_DivBy, src/Simulations.jl:1207-1211)
+    if (p) p[q] = R(pc / __ldg(dtp));   // p = phi/dt, in the stages that keep it (_DivBy, src/Simulations.jl:1207-1211)
 }
 
 // y[i] = x[i] in FP64 (the seam-2 source into the solver's right-hand side)

@@ -462,7 +462,9 @@ __global__ void wall_face_zero_kernel(Geo g, R* w) {
 // in RK3 stages 2 and 3 (_Lin2r, src/Simulations.jl:1194-1198).
 // N = 16/sizeof(R) x-consecutive cells per thread, 16-byte loads and stores;
 // the west, south and bottom neighbours of phi follow the centred-field
-// maps: periodic x and y, in z periodic or the wall mirror.
+// maps: periodic x and y, in z periodic or the wall mirror.  The kernel moves
+// its bytes at the copy rate; the stages whose pressure the next stage
+// replaces unread pass p = nullptr and move a pass less.
 template <typename R, bool UNI>
 __global__ void __launch_bounds__(256) correct_kernel(Geo g, const R* __restrict__ us, const R* __restrict__ vs,
                                                       const R* __restrict__ ws, const R* __restrict__ phi,
@@ -511,6 +513,7 @@ __global__ void __launch_bounds__(256) correct_kernel(Geo g, const R* __restrict
     vst(uo + qp, un);
     vst(vo + qp, vn);
     vst(wo + qp, wn);
+    if (!p) return;
     const R dt = R(__ldg(dtp));
 #pragma unroll
     for (int n = 0; n < N; ++n) pc[n] = pc[n] / dt;   // p = phi/dt (_DivBy, src/Simulations.jl:1207-1211)

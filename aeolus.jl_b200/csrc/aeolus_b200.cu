@@ -1530,33 +1530,36 @@ struct Core : CoreBase {
         return AEO_OK;
     }
 
-    aeo_status correct(R** out, int stage, R ca, R cb, const double* dtp, int s_u0) {
+    // keep_p: the last substage of a step writes the pressure (the stages before
+    // it would only have theirs overwritten)
+    aeo_status correct(R** out, int stage, R ca, R cb, const double* dtp, int s_u0, bool keep_p = true) {
         R** u0 = P[s_u0];
+        R* pout = keep_p ? pres : nullptr;
         if (pcg) {
             if (uni)
                 cc_correct_kernel<R, true><<<(unsigned)((g.nin + 255) / 256), 256, 0, st>>>(
-                    g, Q[0], Q[1], Q[2], mg_x, apx, apy, apz, u0[0], u0[1], u0[2], out[0], out[1], out[2], pres, dtp,
+                    g, Q[0], Q[1], Q[2], mg_x, apx, apy, apz, u0[0], u0[1], u0[2], out[0], out[1], out[2], pout, dtp,
                     ca, cb, stage, open_x ? ob.bw : nullptr, open_y ? ob.bs : nullptr);
             else
                 cc_correct_kernel<R, false><<<(unsigned)((g.nin + 255) / 256), 256, 0, st>>>(
-                    g, Q[0], Q[1], Q[2], mg_x, apx, apy, apz, u0[0], u0[1], u0[2], out[0], out[1], out[2], pres, dtp,
+                    g, Q[0], Q[1], Q[2], mg_x, apx, apy, apz, u0[0], u0[1], u0[2], out[0], out[1], out[2], pout, dtp,
                     ca, cb, stage);
             CKL();
             return AEO_OK;
         }
         if (uni)
             correct_kernel<R, true><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi, u0[0], u0[1], u0[2], out[0],
-                                                               out[1], out[2], pres, dtp, ca, cb, stage);
+                                                               out[1], out[2], pout, dtp, ca, cb, stage);
         else
             correct_kernel<R, false><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi, u0[0], u0[1], u0[2], out[0],
-                                                                out[1], out[2], pres, dtp, ca, cb, stage);
+                                                                out[1], out[2], pout, dtp, ca, cb, stage);
         CKL();
         return AEO_OK;
     }
 
     // One projected substage: set s_in -> set s_out; stage c(x, s) = ca*s + cb*x
     // with the step-start set s_u0 (stages 2, 3).
-    aeo_status substage(int s_in, int s_out, int s_u0, int stage, R ca, R cb) {
+    aeo_status substage(int s_in, int s_out, int s_u0, int stage, R ca, R cb, bool keep_p) {
         R** out = P[s_out];
         if (ob_rad) {   // the stage-start interior layers of the radiating faces
             ob_mark_kernel<R><<<ob_blocks(), 256, 0, st>>>(g, ob, P[s_in][0], P[s_in][1], P[s_in][2], P[s_in][3]);
@@ -1597,7 +1600,7 @@ struct Core : CoreBase {
         if (ob_rad)     // 7c. open boundaries: data, radiation, mass-flux correction
             if (aeo_status e = ob_update(s_in)) return e;
         if (aeo_status e = solve(nullptr)) return e;
-        if (aeo_status e = correct(out, stage, ca, cb, &d_sc->dt, s_u0)) return e;
+        if (aeo_status e = correct(out, stage, ca, cb, &d_sc->dt, s_u0, keep_p)) return e;
         if (ob_rad && stage)   // the buffers combined like the fields (combine_open_boundaries!)
             if (aeo_status e = ob_combine(ca, cb)) return e;
         mark(AEO_K_CORRECT);
@@ -1632,9 +1635,9 @@ struct Core : CoreBase {
         const R inv3 = R(1) / R(3), two3 = R(2) * inv3;
         if (ob_rad)
             if (aeo_status e = ob_prepare(c)) return e;
-        if (aeo_status e = substage(c, 2, c, 0, R(0), R(0))) return e;
-        if (aeo_status e = substage(2, 3, c, 1, R(0.75), R(0.25))) return e;
-        if (aeo_status e = substage(3, c ^ 1, c, 1, inv3, two3)) return e;
+        if (aeo_status e = substage(c, 2, c, 0, R(0), R(0), false)) return e;
+        if (aeo_status e = substage(2, 3, c, 1, R(0.75), R(0.25), false)) return e;
+        if (aeo_status e = substage(3, c ^ 1, c, 1, inv3, two3, true)) return e;
         return commit_sgs(c ^ 1);
     }
 
@@ -1778,7 +1781,7 @@ struct Core : CoreBase {
         for (int s = 0; s < n; ++s) {
             if (ob_rad)
                 if (aeo_status e = ob_prepare(cur)) return e;
-            if (aeo_status e = substage(cur, cur ^ 1, cur, 0, R(0), R(0))) return e;
+            if (aeo_status e = substage(cur, cur ^ 1, cur, 0, R(0), R(0), true)) return e;
             if (aeo_status e = commit_sgs(cur ^ 1)) return e;
             cur ^= 1;
         }
