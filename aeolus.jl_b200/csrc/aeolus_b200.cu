@@ -713,7 +713,7 @@ struct Core : CoreBase {
         }
         host_n = (long long)(c.nx + 2 * c.hx) * (c.ny + 2 * c.hy) * (c.nz + 2 * c.hz);
         if (aeo_status e = alloc(&d_stage, std::max<long long>(host_n, g.nin))) return e;
-        if (aeo_status e = alloc(&d_part, 4 * (size_t)(Nz + 1))) return e;
+        if (aeo_status e = alloc(&d_part, 4 * (size_t)AEO_LEVEL_CTAS * (Nz + 1))) return e;
         if (dyncl()) {
             dws.sx = g.nx + 2;
             dws.sy = g.ny + 2;
@@ -1616,14 +1616,22 @@ struct Core : CoreBase {
         if (dyn())
             if (aeo_status e = enqueue_dynamic(in)) return e;
         if (uni) {
-            if (sgs) cfl_levels_kernel<R, true, true><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
-            else cfl_levels_kernel<R, true, false><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
+    // CTAs a level of the diagnostics: enough for eight of 256 threads an SM, at
+    // least 4096 cells each
+    int level_ctas() const {
+        const long long want = (8LL * nsm + g.nz - 1) / g.nz, most = std::max(1LL, (long long)g.nx * g.ny / 4096);
+        return (int)std::min(std::max(want, 1LL), std::min(most, (long long)AEO_LEVEL_CTAS));
+    }
+
+            if (sgs) cfl_levels_kernel<R, true, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
+            else cfl_levels_kernel<R, true, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
+        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
         } else {
-            if (sgs) cfl_levels_kernel<R, false, true><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
-            else cfl_levels_kernel<R, false, false><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
+            if (sgs) cfl_levels_kernel<R, false, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
+            else cfl_levels_kernel<R, false, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
         }
         CKL();
-        dt_pick_kernel<<<1, 32, 0, st>>>(g, cflp, d_part, d_sc);
+        dt_pick_kernel<<<1, 256, 0, st>>>(g, cflp, d_part, level_ctas(), d_sc);
         CKL();
         return AEO_OK;
     }
@@ -1815,12 +1823,14 @@ struct Core : CoreBase {
     aeo_status guard(int s, bool* finite, double* div, double* speed) {
         R** in = P[s];
         if (anel) {
-            if (uni) guard_levels_kernel<R, true, true><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
-            else guard_levels_kernel<R, true, false><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
+            if (uni) guard_levels_kernel<R, true, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
+            else guard_levels_kernel<R, true, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
         } else {
-            if (uni) guard_levels_kernel<R, false, true><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
-            else guard_levels_kernel<R, false, false><<<g.nz, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
+            if (uni) guard_levels_kernel<R, false, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
+            else guard_levels_kernel<R, false, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
         }
+        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
+        CK(cudaMemsetAsync(d_part, 0, 3 * (size_t)g.nz * sizeof(double), st));
         CKL();
         std::vector<double> h(3 * (size_t)g.nz);
         CK(cudaMemcpyAsync(h.data(), d_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -32,7 +32,7 @@ def random_state(g, seed, amp=1.0):
 
 
 # ---- the tiled WENO sweeps: tiles of 32 x 8 cells, chunks of levels by the number of tiles ---------------------
-@pytest.mark.parametrize("size,bc_z", [((16, 4, 5), "wall"), ((32, 8, 2), "periodic"), ((64, 16, 13), "wall"),
+@pytest.mark.parametrize("size,bc_z", [((16, 4, 5), "wall"), ((32, 8, 4), "periodic"), ((64, 16, 13), "wall"),
                                        ((32, 32, 64), "periodic")])
 @pytest.mark.parametrize("scheme", ["weno_js5", "weno_z5"])
 @pytest.mark.parametrize("c_s", [0.0, 0.17])
@@ -40,6 +40,7 @@ def test_weno_steps_at_tile_and_chunk_edges(size, bc_z, scheme, c_s):
     g = regular_grid(size, (2 * np.pi,) * 3, bc_z=bc_z)
     kw = dict(grid=g, advection=scheme, nu=1e-3, c_s=c_s, theta0=300.0 if bc_z == "wall" else 0.0)
     state = random_state(g, 5, 0.5)
+    state[3][g.interior] += kw["theta0"]
     o = OracleSimulation(CoreSpec(**kw))
     s64, s32 = Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
     for s in (o, s64, s32):
@@ -75,3 +76,35 @@ def test_weno_keeps_a_uniform_field_and_scales(scheme, precision, tol):
         s.step_rk3(1e-3)
         out.append(s.get_field("theta")[g.interior] / scale)
     assert rel(out[1], out[0]) <= (1e-12 if precision == "fp64" else 1e-5)
+
+
+# ---- the diagnostics' levels, shared by several CTAs -----------------------------------------------------------
+@pytest.mark.parametrize("size", [(8, 4, 3), (64, 64, 5), (128, 64, 2), (256, 128, 4)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+def test_cfl_and_guard_over_shared_levels(size, precision):
+    from aeolus_b200.simulation import CFLConstraints
+    g = regular_grid(size, (2.0, 1.0, 0.5), bc_z="wall")
+    kw = dict(grid=g, theta0=300.0, c_s=0.17, nu=1e-3)
+    state = random_state(g, 2, 0.1)
+    # one fast cell in the last row of the middle level sets the rate
+    k = g.halo[2] + g.nz // 2
+    state[0][k, -1 - g.halo[1], -1 - g.halo[0]] = 7.0
+    state[3] += 300.0 + np.arange(g.storage_shape[0])[:, None, None]
+    o, s = OracleSimulation(CoreSpec(**kw)), Sim(CoreSpec(precision=precision, **kw))
+    for q in (o, s):
+        q.set_state(*state)
+    c = CFLConstraints(divergence_tol=1e9, max_retries=0)
+    want, got = o.adaptive_dt(c)[0], s.cfl_diagnostics(c)
+    assert abs(got["dt"] - want) <= (1e-12 if precision == "fp64" else 1e-5) * want
+    rate = 0.5 / got["advective_rate"]
+    assert rate < 0.5 * g.dx / 6.9
+    st = s.step_adaptive(c)
+    u = [s.get_field(n)[g.interior] for n in ("u", "v", "w")]
+    assert st["max_speed"] == max(np.abs(a).max() for a in u)
+    assert abs(st["max_divergence"] - s.max_divergence()) <= 1e-12 * max(1.0, st["max_divergence"])
+    bad = [a.copy() for a in state]
+    bad[3][k, g.halo[1], g.halo[0]] = np.nan
+    s.set_state(*bad)
+    from aeolus_b200._lib import NumericalFailure
+    with pytest.raises(NumericalFailure):
+        s.step_adaptive(c)
