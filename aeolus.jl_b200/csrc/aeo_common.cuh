@@ -23,8 +23,9 @@
 
 enum { LOC_C = 0, LOC_FX = 1, LOC_FY = 2, LOC_FZ = 3 };
 
+// aligned to its size, so that a load or store moves both parts at once
 template <typename R>
-struct cplx {
+struct alignas(2 * sizeof(R)) cplx {
     R x, y;
 };
 
@@ -65,6 +66,7 @@ struct Geo {
     int px, py;            // padded row / plane extents
     long long sy, sz;      // padded strides of j and k
     long long nin;         // nx*ny*nz
+    int sp;                // row pitch of the spectrum (nx/2 + 1 or more complex values)
     int bc_z;              // 0 periodic, 1 wall
     int ox, oy;            // open x / y faces (aeo_set_open): fields without planes take the mirror there
     int uniform;           // 1: uniform z metrics

@@ -10,7 +10,8 @@
 //   div        divergence of the predicted velocity (plain, or W-weighted for
 //              the sound-proof core), one cell per thread
 //              (src/FiniteVolume.jl:1869-1888, src/Anelastic.jl:1110-1120)
-//   src_fftx   r2c transform along x of an interior source (the divergence)
+//   src_fftx   r2c transform along x of an interior source, or of the divergence
+//              formed while its rows are loaded
 //   ffty       complex transform along y (forward or inverse)
 //   fftz_solve periodic z: forward transform, scale by nrm/lambda (zero mean
 //              mode), inverse transform -- one pass (src/PressureSolvers.jl:128-138,
@@ -20,15 +21,16 @@
 //              integrated (src/PressureSolvers.jl:650-661, :754-805)
 //   ifftx      c2r along x into the potential phi (interior array)
 //
-// The transforms are Stockham autosort FFTs on lines held in shared memory,
-// each pass an in-register DFT of radix 16, 8 or 4; the inter-pass twiddles
-// come from one table tw[m] = exp(-2 pi i m / NT) with NT the largest
-// transform length.
+// The transforms are Stockham autosort FFTs of in-register DFTs of radix 16, 8
+// or 4.  Lines of 32 .. 512 points (the *_reg kernels) stay in registers and
+// meet in shared memory between two passes; other lengths run on lines held
+// in shared memory.  The inter-pass twiddles come from one table tw[m] =
+// exp(-2 pi i m / NT) with NT the largest transform length.
 #pragma once
 
 #include "aeo_common.cuh"
 
-// Launch shape of every transform CTA: a CTA holds at most 2048 points (the
+// Launch shape of a shared-memory transform's CTA: it holds at most 2048 points (the
 // host sizes rows / column tiles so), PTS per thread: 128 threads x 16 points
 // (radix up to 16) in FP32, 256 x 8 (radix up to 8) in FP64, where 16
 // complex doubles would not fit the register budget.
@@ -189,103 +191,128 @@ __device__ __forceinline__ void smem_fft(cplx<R>* buf, int logn, int lognl, int 
     }
 }
 
-// ---- compile-time lengths -----------------------------------------------------------
-// The same Stockham passes with the length n = 2^LOGN and the line count
-// 2^LOGL (n 2^LOGL = 2048 points a CTA) known at compile time: every shift,
-// mask and offset of the index arithmetic folds to a constant, the pass
-// schedule unrolls, and the inter-pass twiddles come from a table of the n
-// roots W_n^m staged in shared memory by the kernel (twn).  The pass
-// schedule is smem_fft's (ceil(rest / passes left), largest first).
-template <int LOGN, int MAXLR>
-struct FftPlan {
-    static constexpr int NP = (LOGN + MAXLR - 1) / MAXLR;
-    static constexpr int ns(int p) {   // log2 Ns before pass p
-        int l = 0;
-        for (int q = 0; q < p; ++q) l += (LOGN - l + (NP - q) - 1) / (NP - q);
+// ---- compile-time lengths: transforms in registers -----------------------------
+// A line of n = 2^LOGN points (32 .. 512) is held by n/16 threads, 16 points
+// each, straight from global memory: pass p of radix 2^lr does its 16 / 2^lr
+// butterflies in registers, and only the exchange between two passes goes
+// through shared memory (one write and one read a point; 256 = 16 x 16 has one
+// exchange, 512 = 8 x 8 x 8 two).  The staged form this replaces wrote and read
+// shared memory once more before the first and after the last pass and twice in
+// each, at eight points a thread in FP64: bound by shared-memory latency and issue
+// (256^2 x 128 y transform: FP64 75 us, FP32 26 us; 34 us and 12 us of bytes at
+// the copy rate).  Stockham order: before pass p, with Ns points transformed,
+// butterfly j reads x[j + r n/R] and leaves y[(j - j mod Ns) R + j mod Ns + q Ns];
+// the last pass therefore leaves point j + q n/R in butterfly j, which is what the
+// first pass of an inverse with the radices in the opposite order reads: a
+// transform along z, the division by the eigenvalues and the inverse need no
+// exchange between them.
+template <int LOGN, bool REV>
+struct RegPlan {
+    static constexpr int NP = (LOGN + 3) / 4;
+    static constexpr int lrf(int p) {   // logs spread evenly, larger first
+        int rest = LOGN, l = 0;
+        for (int q = 0; q <= p; ++q) { l = (rest + (NP - q) - 1) / (NP - q); rest -= l; }
         return l;
     }
-    static constexpr int lr(int p) { return (LOGN - ns(p) + (NP - p) - 1) / (NP - p); }
+    static constexpr int lr(int p) { return REV ? lrf(NP - 1 - p) : lrf(p); }
+    static constexpr int logns(int p) {
+        int s = 0;
+        for (int q = 0; q < p; ++q) s += lr(q);
+        return s;
+    }
 };
 
-template <typename R, int LR, bool INV, bool LINE_FAST, int LOGN, int LOGL, int LOGNS>
-__device__ __forceinline__ void fft_pass_ct(cplx<R>* buf, const cplx<R>* twn) {
-    constexpr bool SKEW = !LINE_FAST;
-    constexpr int NTHR = FftCfg<R>::THREADS;
-    constexpr int RR = 1 << LR, KB = FftCfg<R>::PTS / RR;
-    constexpr int LOGNB = LOGN - LR, NB = 1 << LOGNB;
-    constexpr int TOTAL = NB << LOGL;
-    constexpr int NS = 1 << LOGNS;
-    constexpr int ES = LINE_FAST ? (1 << LOGL) : 1;
-    constexpr int LS = LINE_FAST ? 1 : ((1 << LOGN) + ((1 << LOGN) >> 4) + 1);
-    constexpr int TSH = LOGN - LR - LOGNS;
-    static_assert(KB * NTHR == TOTAL, "every butterfly of the pass has a thread slot");
-    const int tid = threadIdx.x;
-    cplx<R> v[KB][RR];
-    int oo[KB];
+// The shape of a register transform's CTA: THREADS x 16 points.  Lines of 512
+// points take 256 threads, so that a CTA covers eight columns (64 or 128 bytes
+// of a row of the spectrum).
+template <int LOGN>
+struct RegShape {
+    static constexpr int THREADS = LOGN >= 9 ? 256 : 128;
+    static constexpr int MINB = 512 / THREADS;           // 128 registers a thread
+    static constexpr int LOGT = LOGN - 4;                // log2 of a line's threads
+    static constexpr int LOGL = (LOGN >= 9 ? 8 : 7) - LOGT;
+    static constexpr int L = 1 << LOGL;                  // lines a CTA
+    static constexpr int N = 1 << LOGN;
+    static constexpr int ROW = N + (N >> 4);             // a skewed row: its lines start in distinct banks
+    // exchange buffer (columns: element e of line l at (e + e/16) L + l; rows: l ROW + e + e/16) and the n roots
+    static constexpr int POINTS = L * ROW + N;
+    template <typename R>
+    static constexpr size_t smem() { return (size_t)POINTS * sizeof(cplx<R>); }
+};
+
+// the radix 2^LR butterflies of the thread (t-th of its line), pass with Ns = 2^LOGNS
+template <typename R, int LOGN, int LR, int LOGNS, bool INV>
+__device__ __forceinline__ void reg_pass(cplx<R> (&v)[16], int t, const cplx<R>* twn) {
+    constexpr int RR = 1 << LR, KB = 16 / RR, TPL = 1 << (LOGN - 4);
 #pragma unroll
     for (int s = 0; s < KB; ++s) {
-        const int b = tid + s * NTHR;
-        int l, j;
-        if (LINE_FAST) { l = b & ((1 << LOGL) - 1); j = b >> LOGL; }
-        else { l = b >> LOGNB; j = b & (NB - 1); }
-        const int k = j & (NS - 1);
-        const cplx<R>* base = buf + l * LS;
+        if constexpr (LOGNS > 0) {
+            const int k = (t + s * TPL) & ((1 << LOGNS) - 1);
 #pragma unroll
-        for (int r = 0; r < RR; ++r) {
-            v[s][r] = base[sk16<SKEW>(j + r * NB) * ES];
-            if (LOGNS > 0 && r > 0) {
-                cplx<R> wv = twn[((r * k) << TSH) & ((1 << LOGN) - 1)];
-                if (INV) wv.y = -wv.y;
-                v[s][r] = cmul(v[s][r], wv);
+            for (int r = 1; r < RR; ++r) {
+                cplx<R> w = twn[(r * k) << (LOGN - LR - LOGNS)];   // r k < 2^(LR + LOGNS)
+                if (INV) w.y = -w.y;
+                v[s * RR + r] = cmul(v[s * RR + r], w);
             }
         }
-        dft_reg<R, RR, INV>(v[s]);
-        oo[s] = l * LS + (SKEW ? 0 : (((j - k) << LR) + k) * ES);
-        if (SKEW) oo[s] |= ((((j - k) << LR) + k) << 16);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < KB; ++s) {
-        if (SKEW) {
-            const int lo = oo[s] & 0xFFFF, o = oo[s] >> 16;
-#pragma unroll
-            for (int q = 0; q < RR; ++q) buf[lo + sk16<true>(o + q * NS)] = v[s][q];
-        } else {
-#pragma unroll
-            for (int q = 0; q < RR; ++q) buf[oo[s] + q * NS * ES] = v[s][q];
-        }
-    }
-    __syncthreads();
-}
-
-template <typename R, bool INV, bool LINE_FAST, int LOGN, int LOGL, int P = 0>
-__device__ __forceinline__ void smem_fft_ct(cplx<R>* buf, const cplx<R>* twn) {
-    using PL = FftPlan<LOGN, FftCfg<R>::MAXLR>;
-    if constexpr (P < PL::NP) {
-        fft_pass_ct<R, PL::lr(P), INV, LINE_FAST, LOGN, LOGL, PL::ns(P)>(buf, twn);
-        smem_fft_ct<R, INV, LINE_FAST, LOGN, LOGL, P + 1>(buf, twn);
+        dft_reg<R, RR, INV>(v + s * RR);
     }
 }
-
-// The transform of a kernel: compile-time lengths (LOGN > 0; the lines fill
-// the CTA's 2048 points) or the general form.
-template <typename R, bool INV, bool LINE_FAST, int LOGN>
-__device__ __forceinline__ void run_fft(cplx<R>* buf, int logn, int lognl, int ls, int es,
-                                        const cplx<R>* __restrict__ tw, int NT, const cplx<R>* twn) {
-    if constexpr (LOGN > 0) smem_fft_ct<R, INV, LINE_FAST, LOGN, 11 - LOGN>(buf, twn);
-    else smem_fft<R, INV, LINE_FAST>(buf, logn, lognl, ls, es, tw, NT);
+// point r of the thread's butterfly s before (IN) or after the pass
+template <int LOGN, int LR, int LOGNS, bool IN>
+__device__ __forceinline__ int reg_point(int t, int s, int r) {
+    constexpr int TPL = 1 << (LOGN - 4);
+    const int j = t + s * TPL;
+    if constexpr (IN) return j + (r << (LOGN - LR));
+    const int k = j & ((1 << LOGNS) - 1);
+    return ((j - k) << LR) + k + (r << LOGNS);
 }
-// Stage the roots W_n^m, m < n = 2^LOGN, from the NT-point table (NT >= n).
+// shared-memory slot of point e of line l
+template <int LOGN, bool COLS>
+__device__ __forceinline__ int reg_slot(int l, int e) {
+    using S = RegShape<LOGN>;
+    return COLS ? (e + (e >> 4)) * S::L + l : l * S::ROW + e + (e >> 4);
+}
+// passes P .. NP-1; FROM: the points of pass P come from the exchange buffer
+template <typename R, int LOGN, bool INV, bool REV, bool COLS, int P = 0, bool FROM = false>
+__device__ __forceinline__ void reg_fft(cplx<R> (&v)[16], int t, int l, cplx<R>* buf, const cplx<R>* twn) {
+    using PL = RegPlan<LOGN, REV>;
+    constexpr int LR = PL::lr(P), LOGNS = PL::logns(P), RR = 1 << LR, KB = 16 / RR;
+    if constexpr (FROM) {
+#pragma unroll
+        for (int s = 0; s < KB; ++s)
+#pragma unroll
+            for (int r = 0; r < RR; ++r) v[s * RR + r] = buf[reg_slot<LOGN, COLS>(l, reg_point<LOGN, LR, LOGNS, true>(t, s, r))];
+    }
+    reg_pass<R, LOGN, LR, LOGNS, INV>(v, t, twn);
+    if constexpr (P + 1 < PL::NP) {
+        if constexpr (FROM) __syncthreads();   // every thread has read the previous exchange
+#pragma unroll
+        for (int s = 0; s < KB; ++s)
+#pragma unroll
+            for (int q = 0; q < RR; ++q) buf[reg_slot<LOGN, COLS>(l, reg_point<LOGN, LR, LOGNS, false>(t, s, q))] = v[s * RR + q];
+        __syncthreads();
+        reg_fft<R, LOGN, INV, REV, COLS, P + 1, true>(v, t, l, buf, twn);
+    }
+}
+// the point in v[s RR + r] that the first pass expects / the last pass leaves
+template <int LOGN, bool REV>
+__device__ __forceinline__ int reg_in(int t, int e) {
+    constexpr int LR = RegPlan<LOGN, REV>::lr(0);
+    return reg_point<LOGN, LR, 0, true>(t, e >> LR, e & ((1 << LR) - 1));
+}
+template <int LOGN, bool REV>
+__device__ __forceinline__ int reg_out(int t, int e) {
+    using PL = RegPlan<LOGN, REV>;
+    constexpr int LR = PL::lr(PL::NP - 1), LOGNS = PL::logns(PL::NP - 1);
+    return reg_point<LOGN, LR, LOGNS, false>(t, e >> LR, e & ((1 << LR) - 1));
+}
+// Stage the roots W_n^m, m < n, from the NT-point table (NT >= n).
 template <typename R, int LOGN>
 __device__ __forceinline__ void stage_roots(cplx<R>* twn, const cplx<R>* __restrict__ tw, int NT) {
-    if constexpr (LOGN > 0) {
-        const int sh = (__ffs(NT) - 1) - LOGN;
-        for (int m = threadIdx.x; m < (1 << LOGN); m += blockDim.x) twn[m] = tw[m << sh];
-    }
+    const int sh = (__ffs(NT) - 1) - LOGN;
+    for (int m = threadIdx.x; m < (1 << LOGN); m += blockDim.x) twn[m] = tw[m << sh];
 }
-// the extra shared memory of a compile-time-length kernel
-template <typename R>
-inline size_t roots_smem(int logn) { return (logn >= 7 && logn <= 9) ? ((size_t)1 << logn) * sizeof(cplx<R>) : 0; }
 
 // ---- divergence ------------------------------------------------------------------
 // The divergence of the predicted velocity (the source of the pressure solve)
@@ -358,17 +385,14 @@ __device__ __forceinline__ cplx<R> c2r_pre(cplx<R> a, cplx<R> b, cplx<R> wv) {
 // The CTA stages its rows' half spectra with one coalesced load per bin,
 // pre-processes the bin pairs (u, M-u) (unit 0 of a row: bins 0 and M/2) in
 // registers, writes the packed M-point lines skewed, runs the inverse FFT
-// and stores the real pairs.
-template <typename R, int LOGN = 0>
+// and stores the real pairs.  (Row lengths outside the register form's.)
+template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) ifftx_kernel(Geo g, const cplx<R>* __restrict__ S, R* __restrict__ phi,
                                                     const cplx<R>* __restrict__ tw, int NT, int rows, R scale) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
     constexpr int UPT = FftCfg<R>::PTS / 2;
-    const int M = LOGN > 0 ? (1 << LOGN) : g.nx / 2, Mh = M + 1, lM = LOGN > 0 ? LOGN : __ffs(M) - 1, LS = xrow(M);
-    if (LOGN > 0) rows = 1 << (11 - LOGN);
-    cplx<R>* twn = buf + rows * LS;
-    stage_roots<R, LOGN>(twn, tw, NT);
+    const int M = g.nx / 2, lM = __ffs(M) - 1, LS = xrow(M);
     const long long nrows = (long long)g.ny * g.nz;
     const long long row0 = (long long)blockIdx.x * rows;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -377,11 +401,11 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) ifftx_kernel(Geo 
     for (int e = tid; e < (rows << lM); e += nthr) {
         const int r = e >> lM, kk = e & (M - 1);
         const long long row = row0 + r;
-        buf[r * LS + kk] = row < nrows ? S[row * Mh + kk] : cmk<R>(R(0), R(0));
+        buf[r * LS + kk] = row < nrows ? S[row * g.sp + kk] : cmk<R>(R(0), R(0));
     }
     for (int r = tid; r < rows; r += nthr) {
         const long long row = row0 + r;
-        buf[r * LS + M] = row < nrows ? S[row * Mh + M] : cmk<R>(R(0), R(0));
+        buf[r * LS + M] = row < nrows ? S[row * g.sp + M] : cmk<R>(R(0), R(0));
     }
     __syncthreads();
     const int lH = lM - 1, H = M >> 1;
@@ -413,7 +437,7 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) ifftx_kernel(Geo 
         }
     }
     __syncthreads();
-    run_fft<R, true, false, LOGN>(buf, lM, __ffs(rows) - 1, LS, 1, tw, NT, twn);
+    smem_fft<R, true, false>(buf, lM, __ffs(rows) - 1, LS, 1, tw, NT);
     for (int e = tid; e < (rows << lM); e += nthr) {
         const int r = e >> lM, n = e & (M - 1);
         const long long row = row0 + r;
@@ -424,50 +448,114 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) ifftx_kernel(Geo 
     }
 }
 
+// The register form for M = 2^LOGN bins: a thread loads the bins u and M-u of
+// its pairs from the spectrum, pre-processes both and writes them to the
+// exchange buffer; the passes read it from there and the last one's points
+// go to phi as real pairs.
+template <typename R, int LOGN>
+__global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
+    ifftx_reg_kernel(Geo g, const cplx<R>* __restrict__ S, R* __restrict__ phi, const cplx<R>* __restrict__ tw, int NT,
+                     R scale) {
+    using Sh = RegShape<LOGN>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
+    cplx<R>* twn = buf + Sh::L * Sh::ROW;
+    constexpr int M = Sh::N, H = M / 2, TPL = 1 << Sh::LOGT;
+    const long long nrows = (long long)g.ny * g.nz;
+    const int t = threadIdx.x & (TPL - 1), l = threadIdx.x >> Sh::LOGT;
+    const long long row = (long long)blockIdx.x * Sh::L + l;
+    const int tsh = (__ffs(NT) - 1) - (LOGN + 1);
+    stage_roots<R, LOGN>(twn, tw, NT);
+    const cplx<R>* Sr = S + (row < nrows ? row : nrows - 1) * g.sp;
+    cplx<R> a[8], b[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int u = t + s * TPL;   // pairs (u, M - u), u < M/2
+        a[s] = Sr[u];
+        b[s] = Sr[M - u];
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int u = t + s * TPL;
+        const cplx<R> w = tw[u << tsh];
+        cplx<R> z0 = c2r_pre(a[s], b[s], w), z1;
+        if (u == 0) {   // bin 0's partner is bin M; bin M/2 pairs with itself (twiddle -i)
+            const cplx<R> h = Sr[H];
+            z1 = c2r_pre(h, h, cmk<R>(R(0), R(-1)));
+        } else {
+            z1 = c2r_pre(b[s], a[s], cmk<R>(-w.x, w.y));   // W^(M-u) = -conj W^u
+        }
+        buf[reg_slot<LOGN, false>(l, u)] = z0;
+        buf[reg_slot<LOGN, false>(l, u == 0 ? H : M - u)] = z1;
+    }
+    __syncthreads();
+    cplx<R> v[16];
+    reg_fft<R, LOGN, true, false, false, 0, true>(v, t, l, buf, twn);
+    if (row >= nrows) return;
+    cplx<R>* out = reinterpret_cast<cplx<R>*>(phi + row * g.nx);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) out[reg_out<LOGN, false>(t, e)] = cmk<R>(v[e].x * scale, v[e].y * scale);
+}
+
 // ---- complex transform along y (MODE 0 forward, 1 inverse) ----------------------
 // CTA: tile of `tpx` consecutive kx columns at one kz, all ky.
-template <typename R, int MODE, int LOGN = 0>
+template <typename R, int MODE>
 __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) ffty_kernel(Geo g, cplx<R>* __restrict__ S, const cplx<R>* __restrict__ tw,
                                                    int NT, int tpx) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
-    if (LOGN > 0) tpx = 1 << (11 - LOGN);
-    cplx<R>* twn = buf + g.ny * tpx;
-    stage_roots<R, LOGN>(twn, tw, NT);
     const int Mh = g.nx / 2 + 1;
     const int k = blockIdx.y, p0 = blockIdx.x * tpx;
     const int tid = threadIdx.x, nthr = blockDim.x;
-    const long long base = (long long)k * g.ny * Mh;
+    const long long base = (long long)k * g.ny * g.sp;
     const int lt = __ffs(tpx) - 1;
 #pragma unroll 16
     for (int e = tid; e < g.ny * tpx; e += nthr) {
         const int jj = e >> lt, c = e & (tpx - 1), p = p0 + c;
-        buf[e] = p < Mh ? S[base + (long long)jj * Mh + p] : cmk<R>(R(0), R(0));
+        buf[e] = p < Mh ? S[base + (long long)jj * g.sp + p] : cmk<R>(R(0), R(0));
     }
     __syncthreads();
-    run_fft<R, MODE == 1, true, LOGN>(buf, __ffs(g.ny) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT, twn);
+    smem_fft<R, MODE == 1, true>(buf, __ffs(g.ny) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT);
     for (int e = tid; e < g.ny * tpx; e += nthr) {
         const int jj = e >> lt, c = e & (tpx - 1), p = p0 + c;
-        if (p < Mh) S[base + (long long)jj * Mh + p] = buf[e];
+        if (p < Mh) S[base + (long long)jj * g.sp + p] = buf[e];
     }
+}
+template <typename R, int MODE, int LOGN>
+__global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
+    ffty_reg_kernel(Geo g, cplx<R>* __restrict__ S, const cplx<R>* __restrict__ tw, int NT) {
+    using Sh = RegShape<LOGN>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
+    cplx<R>* twn = buf + Sh::L * Sh::ROW;
+    const int l = threadIdx.x & (Sh::L - 1), t = threadIdx.x >> Sh::LOGL;
+    const int p = blockIdx.x * Sh::L + l;
+    const bool in = p < g.nx / 2 + 1;
+    cplx<R>* col = S + (long long)blockIdx.y * g.ny * g.sp + p;
+    cplx<R> v[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+        v[e] = in ? col[(long long)reg_in<LOGN, false>(t, e) * g.sp] : cmk<R>(R(0), R(0));
+    stage_roots<R, LOGN>(twn, tw, NT);   // (the first pass has no twiddles; the first exchange's barrier orders it)
+    reg_fft<R, LOGN, MODE == 1, false, true>(v, t, l, buf, twn);
+    if (!in) return;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) col[(long long)reg_out<LOGN, false>(t, e) * g.sp] = v[e];
 }
 
 // ---- periodic z: forward, scale by nrm/lambda, inverse -------------------------
-template <typename R, int LOGN = 0>
+template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) fftz_solve_kernel(Geo g, cplx<R>* __restrict__ S, const cplx<R>* __restrict__ tw,
                                                          int NT, int tpx, const double* __restrict__ kx2,
                                                          const double* __restrict__ ky2, const double* __restrict__ kz2,
                                                          double nrm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
-    if (LOGN > 0) tpx = 1 << (11 - LOGN);
-    cplx<R>* twn = buf + g.nz * tpx;
-    stage_roots<R, LOGN>(twn, tw, NT);
     const int Mh = g.nx / 2 + 1;
     const int j = blockIdx.y, p0 = blockIdx.x * tpx;
     const int tid = threadIdx.x, nthr = blockDim.x;
-    const long long sk = (long long)g.ny * Mh;
-    const long long base = (long long)j * Mh;
+    const long long sk = (long long)g.ny * g.sp;
+    const long long base = (long long)j * g.sp;
     const int lt = __ffs(tpx) - 1;
 #pragma unroll 16
     for (int e = tid; e < g.nz * tpx; e += nthr) {
@@ -475,7 +563,7 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) fftz_solve_kernel
         buf[e] = p < Mh ? S[base + kz * sk + p] : cmk<R>(R(0), R(0));
     }
     __syncthreads();
-    run_fft<R, false, true, LOGN>(buf, __ffs(g.nz) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT, twn);
+    smem_fft<R, false, true>(buf, __ffs(g.nz) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT);
     for (int e = tid; e < g.nz * tpx; e += nthr) {
         const int kz = e >> lt, c = e & (tpx - 1), p = p0 + c;
         if (p < Mh) {
@@ -486,11 +574,45 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) fftz_solve_kernel
         }
     }
     __syncthreads();
-    run_fft<R, true, true, LOGN>(buf, __ffs(g.nz) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT, twn);
+    smem_fft<R, true, true>(buf, __ffs(g.nz) - 1, __ffs(tpx) - 1, 1, tpx, tw, NT);
     for (int e = tid; e < g.nz * tpx; e += nthr) {
         const int kz = e >> lt, c = e & (tpx - 1), p = p0 + c;
         if (p < Mh) S[base + kz * sk + p] = buf[e];
     }
+}
+template <typename R, int LOGN>
+__global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
+    fftz_solve_reg_kernel(Geo g, cplx<R>* __restrict__ S, const cplx<R>* __restrict__ tw, int NT,
+                          const double* __restrict__ kx2, const double* __restrict__ ky2,
+                          const double* __restrict__ kz2, double nrm) {
+    using Sh = RegShape<LOGN>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
+    cplx<R>* twn = buf + Sh::L * Sh::ROW;
+    const int l = threadIdx.x & (Sh::L - 1), t = threadIdx.x >> Sh::LOGL;
+    const int p = blockIdx.x * Sh::L + l, j = blockIdx.y;
+    const bool in = p < g.nx / 2 + 1;
+    const long long sk = (long long)g.ny * g.sp;
+    cplx<R>* col = S + (long long)j * g.sp + p;
+    cplx<R> v[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] = in ? col[reg_in<LOGN, false>(t, e) * sk] : cmk<R>(R(0), R(0));
+    stage_roots<R, LOGN>(twn, tw, NT);
+    reg_fft<R, LOGN, false, false, true>(v, t, l, buf, twn);
+    const double kxy = in ? kx2[p] + ky2[j] : 1.0;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        // the sum in the reference's order (kx2 + ky2) + kz2
+        const double lam = -(kxy + __ldg(kz2 + reg_out<LOGN, false>(t, e)));
+        const R il = lam == 0.0 ? R(0) : R(nrm / lam);
+        v[e] = cmk<R>(v[e].x * il, v[e].y * il);
+    }
+    // the inverse's first pass takes the points where the forward's last one left them
+    if constexpr (RegPlan<LOGN, false>::NP > 1) __syncthreads();   // every thread has read the forward's last exchange
+    reg_fft<R, LOGN, true, true, true>(v, t, l, buf, twn);
+    if (!in) return;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) col[reg_out<LOGN, true>(t, e) * sk] = v[e];
 }
 
 // ---- walls in z: the batched column solve ------------------------------------------
@@ -574,10 +696,11 @@ template <typename RD>
 __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restrict__ mtab, RD* __restrict__ ctab,
                                                             ColumnCoef c) {
     const int Mh = g.nx / 2 + 1;
-    const long long sk = (long long)g.ny * Mh;
-    const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col == 0 || col >= sk) return;
-    const int p = (int)(col % Mh), j = (int)(col / Mh);
+    const long long sk = (long long)g.ny * g.sp;
+    const long long id0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id0 == 0 || id0 >= (long long)g.ny * Mh) return;
+    const int p = (int)(id0 % Mh), j = (int)(id0 / Mh);
+    const long long col = (long long)j * g.sp + p;
     const double lam = c.kx2[p] + c.ky2[j];
     double cprev = 0.0;
     for (int k = 0; k < g.nz; ++k) {
@@ -604,7 +727,7 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, cplx<RD>*
     double* after = reinterpret_cast<double*>(ring + D * 32);
     const int Mh = g.nx / 2 + 1;
     const int lane = threadIdx.x;
-    const long long sk = (long long)g.ny * Mh;
+    const long long sk = (long long)g.ny * g.sp;
     const int nz = g.nz;
     if (blockIdx.x == 0) {
         // the mean mode (_mean_mode!, src/PressureSolvers.jl:780-805), real:
@@ -657,9 +780,10 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, cplx<RD>*
         s_hw[k] = c.hw[k];
     }
     __syncwarp();
-    const long long col = (long long)(blockIdx.x - 1) * 32 + lane;
-    if (col == 0 || col >= sk) return;
-    const int p = (int)(col % Mh), j = (int)(col / Mh);
+    const long long id0 = (long long)(blockIdx.x - 1) * 32 + lane;
+    if (id0 == 0 || id0 >= (long long)g.ny * Mh) return;
+    const int p = (int)(id0 % Mh), j = (int)(id0 / Mh);
+    const long long col = (long long)j * g.sp + p;
     const double lam = c.kx2[p] + c.ky2[j];
     // forward elimination: level k waits in slot k % D; the copy of level
     // k + D - 1 goes to the slot read one level earlier
@@ -765,17 +889,12 @@ __device__ __forceinline__ cplx<R> div_pair(const Geo& g, const R* __restrict__ 
                   (ue - uc1) * idx + (vn1 - vc1) * idy + (wn1 - wc1) * idz);
 }
 
-template <typename R, int LOGN = 0, int DIV = 0>   // DIV: 0 src; 1 plain, 2 W-weighted divergence (+4: stretched)
+template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) src_fftx_kernel(Geo g, const R* __restrict__ src, cplx<R>* __restrict__ S,
-                                                       const cplx<R>* __restrict__ tw, int NT, int rows,
-                                                       const R* __restrict__ us = nullptr, const R* __restrict__ vs = nullptr,
-                                                       const R* __restrict__ ws = nullptr) {
+                                                       const cplx<R>* __restrict__ tw, int NT, int rows) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
-    const int M = LOGN > 0 ? (1 << LOGN) : g.nx / 2, Mh = M + 1, lM = LOGN > 0 ? LOGN : __ffs(M) - 1, LS = xrow(M);
-    if (LOGN > 0) rows = 1 << (11 - LOGN);
-    cplx<R>* twn = buf + rows * LS;
-    stage_roots<R, LOGN>(twn, tw, NT);
+    const int M = g.nx / 2, lM = __ffs(M) - 1, LS = xrow(M);
     const long long nrows = (long long)g.ny * g.nz;
     const long long row0 = (long long)blockIdx.x * rows;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -784,22 +903,70 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) src_fftx_kernel(G
         const int r = e >> lM, n = e & (M - 1);
         const long long row = row0 + r;
         cplx<R> z = cmk<R>(R(0), R(0));
-        if (row < nrows) {
-            if constexpr (DIV == 0) z = cmk<R>(src[row * g.nx + 2 * n], src[row * g.nx + 2 * n + 1]);
-            else z = div_pair<R, (DIV & 3) == 2, (DIV & 4) == 0>(g, us, vs, ws, row, 2 * n);
-        }
+        if (row < nrows) z = cmk<R>(src[row * g.nx + 2 * n], src[row * g.nx + 2 * n + 1]);
         buf[r * LS + sk16<true>(n)] = z;
     }
     __syncthreads();
-    run_fft<R, false, false, LOGN>(buf, lM, __ffs(rows) - 1, LS, 1, tw, NT, twn);
+    smem_fft<R, false, false>(buf, lM, __ffs(rows) - 1, LS, 1, tw, NT);
     const int tstep = NT / g.nx;
     for (int e = tid; e < (rows << lM); e += nthr) {
         const int r = e >> lM, kk = e & (M - 1);
         const long long row = row0 + r;
-        if (row < nrows) S[row * Mh + kk] = r2c_bin(buf + r * LS, M, kk, tw[(kk * tstep) & (NT - 1)]);
+        if (row < nrows) S[row * g.sp + kk] = r2c_bin(buf + r * LS, M, kk, tw[(kk * tstep) & (NT - 1)]);
     }
     for (int r = tid; r < rows; r += nthr) {   // the Nyquist bin, twiddle exactly -1
         const long long row = row0 + r;
-        if (row < nrows) S[row * Mh + M] = r2c_bin(buf + r * LS, M, M, cmk<R>(R(-1), R(0)));
+        if (row < nrows) S[row * g.sp + M] = r2c_bin(buf + r * LS, M, M, cmk<R>(R(-1), R(0)));
+    }
+}
+
+// The register form for M = 2^LOGN: the points go from global memory (or, DIV:
+// 1 plain, 2 W-weighted divergence, +4 stretched, from the predicted velocity)
+// into the first pass, the last pass's points to the exchange buffer, and a
+// thread post-processes the bins k and M-k of a pair from one read of both.
+template <typename R, int LOGN, int DIV>
+__global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
+    src_fftx_reg_kernel(Geo g, const R* __restrict__ src, cplx<R>* __restrict__ S, const cplx<R>* __restrict__ tw, int NT,
+                        const R* __restrict__ us, const R* __restrict__ vs, const R* __restrict__ ws) {
+    using Sh = RegShape<LOGN>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
+    cplx<R>* twn = buf + Sh::L * Sh::ROW;
+    constexpr int M = Sh::N, H = M / 2, TPL = 1 << Sh::LOGT;
+    const long long nrows = (long long)g.ny * g.nz;
+    const int t = threadIdx.x & (TPL - 1), l = threadIdx.x >> Sh::LOGT;
+    const long long row = (long long)blockIdx.x * Sh::L + l;
+    const long long rl = row < nrows ? row : nrows - 1;   // a row past the end repeats the last one
+    cplx<R> v[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const int n = reg_in<LOGN, false>(t, e);
+        if constexpr (DIV == 0) v[e] = reinterpret_cast<const cplx<R>*>(src + rl * g.nx)[n];
+        else v[e] = div_pair<R, (DIV & 3) == 2, (DIV & 4) == 0>(g, us, vs, ws, rl, 2 * n);
+    }
+    stage_roots<R, LOGN>(twn, tw, NT);
+    reg_fft<R, LOGN, false, false, false>(v, t, l, buf, twn);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) buf[reg_slot<LOGN, false>(l, reg_out<LOGN, false>(t, e))] = v[e];
+    __syncthreads();
+    if (row >= nrows) return;
+    const int tsh = (__ffs(NT) - 1) - (LOGN + 1);
+    const cplx<R>* rb = buf + l * Sh::ROW;
+    cplx<R>* Sr = S + row * g.sp;
+    const R hf = R(0.5);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int u = t + s * TPL;
+        const cplx<R> a = rb[sk16<true>(u)], b = rb[sk16<true>(u == 0 ? 0 : M - u)];
+        const cplx<R> w = tw[u << tsh];
+        const R er = hf * (a.x + b.x), ei = hf * (a.y - b.y), orr = hf * (a.y + b.y), oi = -hf * (a.x - b.x);
+        const R pr = w.x * orr - w.y * oi, pi = w.x * oi + w.y * orr;
+        Sr[u] = cmk<R>(er + pr, ei + pi);
+        Sr[M - u] = cmk<R>(er - pr, pi - ei);   // conj of the even part minus the odd one (u = 0: the Nyquist bin)
+        if (u == 0) {                           // bin M/2 pairs with itself, twiddle -i
+            const cplx<R> h = rb[sk16<true>(H)];
+            Sr[H] = cmk<R>(h.x, -h.y);
+        }
     }
 }

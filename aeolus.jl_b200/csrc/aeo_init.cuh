@@ -74,7 +74,7 @@ __global__ void iso_modes_kernel(Geo g, cplx<R>* __restrict__ S, IsoParams p) {
             out = cmk<R>(R(amp * (pr * cr - pi * ci)), R(amp * (pr * ci + pi * cr)));
         }
     }
-    S[t] = out;
+    S[a + (long long)g.sp * (b + (long long)g.ny * c)] = out;
 }
 
 // inverse complex transform along z of the spectrum (the field generator's z pass)
@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) fftz_inv_kernel(G
     cplx<R>* buf = reinterpret_cast<cplx<R>*>(smem_raw);
     const int Mh = g.nx / 2 + 1;
     const int j = blockIdx.y, p0 = blockIdx.x * tpx;
-    const long long sk = (long long)g.ny * Mh;
-    const long long base = (long long)j * Mh;
+    const long long sk = (long long)g.ny * g.sp;
+    const long long base = (long long)j * g.sp;
     const int lt = __ffs(tpx) - 1;
 #pragma unroll 16
     for (int e = threadIdx.x; e < g.nz * tpx; e += blockDim.x) {

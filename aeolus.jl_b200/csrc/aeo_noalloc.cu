@@ -150,6 +150,7 @@ extern "C" aeo_status aeo_pressure_solve_column_noalloc(int32_t nx, int32_t ny, 
     Geo g{};
     g.nx = nx; g.ny = ny; g.nz = nz;
     g.nin = (long long)nx * ny * nz;
+    g.sp = Mh;   // rows back to back: the fixed scratch holds no padding
     const double dx = lx / nx, dy = ly / ny;
     int tmax = NT > Mh ? NT : Mh;
     if (ny > tmax) tmax = ny;

@@ -28,6 +28,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/aeolus_b200.h"
@@ -44,15 +45,19 @@
 #include "aeo_sweep_pair.cuh"
 #include "aeo_sweep_wpair.cuh"
 
-// A transform kernel at a compile-time length 2^LG (128, 256 or 512 points:
-// the lines fill the CTA's 2048 points) or its general form (LG = 0).
-#define AEO_FFT_LEN(L, CALL)                                  \
-    switch (L) {                                              \
-        case 7: { constexpr int LG = 7; CALL; } break;        \
-        case 8: { constexpr int LG = 8; CALL; } break;        \
-        case 9: { constexpr int LG = 9; CALL; } break;        \
-        default: { constexpr int LG = 0; CALL; } break;       \
+// reg(length) with the compile-time length 2^5 .. 2^9 of a register transform,
+// or smem() for the shared-memory form of the other lengths.
+template <class Reg, class Smem>
+static void fft_len(int lg, Reg reg, Smem smem) {
+    switch (lg) {
+        case 5: reg(std::integral_constant<int, 5>{}); break;
+        case 6: reg(std::integral_constant<int, 6>{}); break;
+        case 7: reg(std::integral_constant<int, 7>{}); break;
+        case 8: reg(std::integral_constant<int, 8>{}); break;
+        case 9: reg(std::integral_constant<int, 9>{}); break;
+        default: smem(); break;
     }
+}
 static inline int ilog2i(int n) { int l = 0; while ((1 << (l + 1)) <= n) ++l; return l; }
 #include "aeo_sweep_tile.cuh"
 
@@ -694,7 +699,10 @@ struct Core : CoreBase {
             if (aeo_status e = alloc(&nut, np)) return e;
         if (aeo_status e = alloc(&phi, g.nin)) return e;
         if (aeo_status e = alloc(&pres, g.nin)) return e;
-        const long long ns = (long long)Mh * Ny * Nz;
+        // rows of the spectrum start on a 128-byte line (FP64: every second one), so
+        // that eight columns of a transform along y or z are whole sectors of each row
+        g.sp = (Mh + 15) / 16 * 16;
+        const long long ns = (long long)g.sp * Ny * Nz;
         if (aeo_status e = alloc(&S, ns)) return e;
         if (c.solver == AEO_SOLVER_COLUMN) {
             // the elimination factors m and c' of every column in the working precision
@@ -1440,6 +1448,41 @@ struct Core : CoreBase {
         return AEO_OK;
     }
 
+    // a register transform of FP64 lines of 512 points needs more than the default shared memory
+    template <class K>
+    void reg_smem(K* kernel, size_t bytes) {
+        if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    }
+    template <int LG>
+    void launch_src_reg(const R* src) {
+        using Sh = RegShape<LG>;
+        const unsigned gx = (unsigned)((g.ny * (long long)g.nz + Sh::L - 1) / Sh::L);
+        const size_t sm = Sh::template smem<R>();
+        auto go = [&](auto* kernel) {
+            reg_smem(kernel, sm);
+            kernel<<<gx, Sh::THREADS, sm, st>>>(g, src, S, tw, NT, Q[0], Q[1], Q[2]);
+        };
+        if (src) go(src_fftx_reg_kernel<R, LG, 0>);
+        else if (anel) uni ? go(src_fftx_reg_kernel<R, LG, 2>) : go(src_fftx_reg_kernel<R, LG, 6>);
+        else uni ? go(src_fftx_reg_kernel<R, LG, 1>) : go(src_fftx_reg_kernel<R, LG, 5>);
+    }
+    template <int MODE>
+    aeo_status launch_ffty(int lgy) {
+        const int Mh = g.nx / 2 + 1;
+        fft_len(lgy, [&](auto lg) {
+            constexpr int LG = lg;
+            using Sh = RegShape<LG>;
+            reg_smem(ffty_reg_kernel<R, MODE, LG>, Sh::template smem<R>());
+            ffty_reg_kernel<R, MODE, LG><<<dim3((Mh + Sh::L - 1) / Sh::L, g.nz), Sh::THREADS, Sh::template smem<R>(), st>>>(
+                g, S, tw, NT);
+        }, [&] {
+            ffty_kernel<R, MODE><<<dim3((Mh + tpx_y - 1) / tpx_y, g.nz), FFT_THREADS(R),
+                                   (size_t)tpx_y * g.ny * sizeof(cplx<R>), st>>>(g, S, tw, NT, tpx_y);
+        });
+        CKL();
+        return AEO_OK;
+    }
+
     // The pressure solve from the source (src == nullptr: divergence of Q) into phi.
     aeo_status solve(const R* src) {
         if (pcg) {
@@ -1468,45 +1511,37 @@ struct Core : CoreBase {
         size_t smx = (size_t)rows_x * xrow(M) * sizeof(cplx<R>);
         unsigned gx = (unsigned)((g.ny * (long long)g.nz + rows_x - 1) / rows_x);
         const int lgx = ilog2i(M), lgy = ilog2i(g.ny), lgz = ilog2i(g.nz);
-        if (src) {
-            AEO_FFT_LEN(lgx, (src_fftx_kernel<R, LG><<<gx, FFT_THREADS(R), smx + roots_smem<R>(LG), st>>>(
-                                 g, src, S, tw, NT, rows_x)));
-        } else if (lgx >= 7 && lgx <= 9) {
-            // the divergence formed in the r2c's staging (it never goes to memory)
-            const int dv = (anel ? 2 : 1) | (uni ? 0 : 4);
-#define AEO_SRC_DIV(D) AEO_FFT_LEN(lgx, (src_fftx_kernel<R, LG, D><<<gx, FFT_THREADS(R), smx + roots_smem<R>(LG), st>>>( \
-                                             g, nullptr, S, tw, NT, rows_x, Q[0], Q[1], Q[2])))
-            switch (dv) {
-                case 1: AEO_SRC_DIV(1); break;
-                case 2: AEO_SRC_DIV(2); break;
-                case 5: AEO_SRC_DIV(5); break;
-                default: AEO_SRC_DIV(6); break;
+        // the source: the divergence formed in the r2c's loads (it never goes to
+        // memory), or src; the shared-memory form takes an array, so the divergence
+        // goes through phi (overwritten by the c2r at the end)
+        fft_len(lgx, [&](auto lg) { launch_src_reg<lg>(src); }, [&] {
+            const R* in = src;
+            if (!src) {
+                if (anel && uni) div_kernel<R, true, true><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
+                else if (anel) div_kernel<R, true, false><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
+                else if (uni) div_kernel<R, false, true><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
+                else div_kernel<R, false, false><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
+                in = phi;
             }
-#undef AEO_SRC_DIV
-        } else {
-            // the divergence into phi (overwritten by the c2r at the end), then its r2c
-            if (anel && uni) div_kernel<R, true, true><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
-            else if (anel) div_kernel<R, true, false><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
-            else if (uni) div_kernel<R, false, true><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
-            else div_kernel<R, false, false><<<gvec(), 256, 0, st>>>(g, Q[0], Q[1], Q[2], phi);
-            CKL();
-            AEO_FFT_LEN(lgx, (src_fftx_kernel<R, LG><<<gx, FFT_THREADS(R), smx + roots_smem<R>(LG), st>>>(
-                                 g, phi, S, tw, NT, rows_x)));
-        }
+            src_fftx_kernel<R><<<gx, FFT_THREADS(R), smx, st>>>(g, in, S, tw, NT, rows_x);
+        });
         CKL();
         mark(AEO_K_DIV_FFTX);
-        const int Mh = M + 1;
-        dim3 gy((Mh + tpx_y - 1) / tpx_y, g.nz);
-        size_t smy = (size_t)tpx_y * g.ny * sizeof(cplx<R>);
-        AEO_FFT_LEN(lgy, (ffty_kernel<R, 0, LG><<<gy, FFT_THREADS(R), smy + roots_smem<R>(LG), st>>>(g, S, tw, NT, tpx_y)));
-        CKL();
+        if (aeo_status e = launch_ffty<0>(lgy)) return e;
         mark(AEO_K_FFTY);
         if (cfg.solver == AEO_SOLVER_FFT) {
-            dim3 gz((Mh + tpx_z - 1) / tpx_z, g.ny);
-            size_t smz = (size_t)tpx_z * g.nz * sizeof(cplx<R>);
-            double nrm = 1.0 / ((double)g.nx * g.ny * g.nz);
-            AEO_FFT_LEN(lgz, (fftz_solve_kernel<R, LG><<<gz, FFT_THREADS(R), smz + roots_smem<R>(LG), st>>>(
-                                 g, S, tw, NT, tpx_z, kx2, ky2, kz2, nrm)));
+            const int Mh = M + 1;
+            const double nrm = 1.0 / ((double)g.nx * g.ny * g.nz);
+            fft_len(lgz, [&](auto lg) {
+                constexpr int LG = lg;
+                using Sh = RegShape<LG>;
+                reg_smem(fftz_solve_reg_kernel<R, LG>, Sh::template smem<R>());
+                fftz_solve_reg_kernel<R, LG><<<dim3((Mh + Sh::L - 1) / Sh::L, g.ny), Sh::THREADS, Sh::template smem<R>(), st>>>(
+                    g, S, tw, NT, kx2, ky2, kz2, nrm);
+            }, [&] {
+                fftz_solve_kernel<R><<<dim3((Mh + tpx_z - 1) / tpx_z, g.ny), FFT_THREADS(R),
+                                       (size_t)tpx_z * g.nz * sizeof(cplx<R>), st>>>(g, S, tw, NT, tpx_z, kx2, ky2, kz2, nrm);
+            });
         } else {
             size_t smt = thomas_smem(g, true);
             if (smt > 48 * 1024)
@@ -1514,17 +1549,21 @@ struct Core : CoreBase {
                                      (int)smt);
             // d' in place in S; the factors m and c' from the tables made at set-up
             R* ftab = reinterpret_cast<R*>(cps);
-            const long long ns = (long long)(g.nx / 2 + 1) * g.ny * g.nz;
+            const long long ns = (long long)g.sp * g.ny * g.nz;
             thomas_kernel<R, true, R, true><<<thomas_blocks(g), 32, smt, st>>>(g, S, S, ftab + ns, cc, ftab);
         }
         CKL();
         mark(AEO_K_ZSOLVE);
-        AEO_FFT_LEN(lgy, (ffty_kernel<R, 1, LG><<<gy, FFT_THREADS(R), smy + roots_smem<R>(LG), st>>>(g, S, tw, NT, tpx_y)));
-        CKL();
+        if (aeo_status e = launch_ffty<1>(lgy)) return e;
         mark(AEO_K_FFTY);
-        R scale = cfg.solver == AEO_SOLVER_FFT ? R(1) : R(1.0 / ((double)g.nx * g.ny));
-        AEO_FFT_LEN(lgx, (ifftx_kernel<R, LG><<<gx, FFT_THREADS(R), smx + roots_smem<R>(LG), st>>>(
-                             g, S, phi, tw, NT, rows_x, scale)));
+        const R scale = cfg.solver == AEO_SOLVER_FFT ? R(1) : R(1.0 / ((double)g.nx * g.ny));
+        fft_len(lgx, [&](auto lg) {
+            constexpr int LG = lg;
+            using Sh = RegShape<LG>;
+            reg_smem(ifftx_reg_kernel<R, LG>, Sh::template smem<R>());
+            ifftx_reg_kernel<R, LG><<<(unsigned)((g.ny * (long long)g.nz + Sh::L - 1) / Sh::L), Sh::THREADS,
+                                      Sh::template smem<R>(), st>>>(g, S, phi, tw, NT, scale);
+        }, [&] { ifftx_kernel<R><<<gx, FFT_THREADS(R), smx, st>>>(g, S, phi, tw, NT, rows_x, scale); });
         CKL();
         mark(AEO_K_IFFTX);
         return AEO_OK;
@@ -2152,7 +2191,7 @@ struct Core : CoreBase {
             return AEO_ERR_ARGUMENT;
         }
         const int Mh = g.nx / 2 + 1, M = g.nx / 2;
-        const long long ns = (long long)Mh * g.ny * g.nz;
+        const long long ns = (long long)Mh * g.ny * g.nz;   // modes (rows of pitch g.sp)
         dim3 gy((Mh + tpx_y - 1) / tpx_y, g.nz);
         size_t smy = (size_t)tpx_y * g.ny * sizeof(cplx<R>);
         dim3 gz((Mh + tpx_z - 1) / tpx_z, g.ny);

@@ -108,3 +108,58 @@ def test_cfl_and_guard_over_shared_levels(size, precision):
     from aeolus_b200._lib import NumericalFailure
     with pytest.raises(NumericalFailure):
         s.step_adaptive(c)
+
+
+# ---- the transforms: registers for 32 .. 512 points a line, shared memory otherwise ----------------------------
+def poisson(g, b):
+    """The FFT solver's answer in numpy (zero mean mode)."""
+    k = [4 / h ** 2 * np.sin(np.pi * np.arange(n) / n) ** 2 for h, n in ((g.dz, g.nz), (g.dy, g.ny), (g.dx, g.nx))]
+    lam = -(k[0][:, None, None] + k[1][None, :, None] + k[2][None, None, :])
+    lam[0, 0, 0] = 1.0
+    f = np.fft.fftn(b) / lam
+    f[0, 0, 0] = 0
+    return np.fft.ifftn(f).real
+
+
+@pytest.mark.parametrize("size", [(32, 16, 16), (64, 32, 32), (128, 64, 8), (256, 128, 4), (512, 8, 64), (1024, 4, 128),
+                                  (2048, 4, 4), (16, 256, 8), (8, 512, 4), (4, 1024, 8), (8, 4, 256), (4, 8, 512),
+                                  (4, 4, 1024), (64, 64, 64)])
+@pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("fp32_mixed", 2.0 ** -24)])
+def test_fft_pressure_solve_at_every_length(size, precision, eps):
+    """Tolerance: the two transforms' rounding, eps log2(N) |b| each in the 2-norm, grows by the largest 1/lambda of the
+    inverted operator; |b| max(1/lambda) / |x| makes that a relative error."""
+    g = regular_grid(size, (1.0, 0.7, 1.3))
+    b = np.random.default_rng(sum(size)).standard_normal((g.nz, g.ny, g.nx))
+    s = Sim(CoreSpec(grid=g, precision=precision))
+    x, want = s.pressure_solve(b), poisson(g, b)
+    low = max(h * h / 4 / np.sin(np.pi / n) ** 2 for h, n in ((g.dx, g.nx), (g.dy, g.ny), (g.dz, g.nz)))
+    assert rel(x, want) <= 2 * eps * np.log2(g.ncells) * low * np.linalg.norm(b) / np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("size", [(32, 8, 7), (64, 32, 5), (128, 16, 33), (256, 64, 3), (512, 4, 9), (16, 128, 6)])
+@pytest.mark.parametrize("core", ["boussinesq", "anelastic"])
+@pytest.mark.parametrize("stretched", [False, True])
+def test_column_projection_at_every_row_length(size, core, stretched):
+    """The divergence formed in the r2c's loads (plain, W-weighted, stretched), through the column solve: the
+    projected velocity and phi match the oracle's, and a source array through the same transforms too."""
+    from aeolus_b200 import stretched_grid, tanh_faces
+    from aeolus_b200.reference_state import anelastic_profiles, exponential_density
+    nz = size[2]
+    if stretched:
+        g = stretched_grid(size, (1000.0, 800.0, 600.0), tanh_faces(nz, 600.0, 0.8))
+    else:
+        g = regular_grid(size, (1000.0, 800.0, 600.0), bc_z="wall")
+    kw = dict(grid=g)
+    if core == "anelastic":
+        prof = anelastic_profiles(g, exponential_density(g), np.full(nz, 300.0))
+        kw.update(core=core, wc=prof["wc"], wf=prof["wf"], thf=prof["thf"])
+    o, s64, s32 = OracleSimulation(CoreSpec(**kw)), Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
+    for s in (o, s64, s32):
+        s.set_state(*random_state(g, 9))
+        s.project()
+    for n in ("u", "v", "w"):
+        want = o.get_field(n)[g.interior]
+        assert rel(s64.get_field(n)[g.interior], want) <= 1e-12, n
+        assert rel(s32.get_field(n)[g.interior], want) <= 1e-5, n
+    b = np.random.default_rng(1).standard_normal((nz, g.ny, g.nx))
+    assert rel(s64.pressure_solve(b), o.pressure_solve(b)) <= 1e-12
