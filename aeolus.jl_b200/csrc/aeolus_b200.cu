@@ -1650,11 +1650,6 @@ struct Core : CoreBase {
         return hs;
     }
 
-    aeo_status enqueue_pick(int s_state) {
-        R** in = P[s_state];
-        if (dyn())
-            if (aeo_status e = enqueue_dynamic(in)) return e;
-        if (uni) {
     // CTAs a level of the diagnostics: enough for eight of 256 threads an SM, at
     // least 4096 cells each
     int level_ctas() const {
@@ -1662,9 +1657,14 @@ struct Core : CoreBase {
         return (int)std::min(std::max(want, 1LL), std::min(most, (long long)AEO_LEVEL_CTAS));
     }
 
+    aeo_status enqueue_pick(int s_state) {
+        R** in = P[s_state];
+        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
+        if (dyn())
+            if (aeo_status e = enqueue_dynamic(in)) return e;
+        if (uni) {
             if (sgs) cfl_levels_kernel<R, true, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
             else cfl_levels_kernel<R, true, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
-        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
         } else {
             if (sgs) cfl_levels_kernel<R, false, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
             else cfl_levels_kernel<R, false, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], R(cfg.c_s), R(cfg.pr_t), d_cs2, dyn_d2, d_part, d_cs2f);
@@ -1861,6 +1861,8 @@ struct Core : CoreBase {
     // the post-step guard of set s: (finite, max |div|, max speed)
     aeo_status guard(int s, bool* finite, double* div, double* speed) {
         R** in = P[s];
+        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
+        CK(cudaMemsetAsync(d_part, 0, 3 * (size_t)g.nz * sizeof(double), st));
         if (anel) {
             if (uni) guard_levels_kernel<R, true, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
             else guard_levels_kernel<R, true, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
@@ -1868,8 +1870,6 @@ struct Core : CoreBase {
             if (uni) guard_levels_kernel<R, false, true><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
             else guard_levels_kernel<R, false, false><<<lg, 256, 0, st>>>(g, in[0], in[1], in[2], in[3], pres, d_part);
         }
-        const dim3 lg((unsigned)g.nz, (unsigned)level_ctas());
-        CK(cudaMemsetAsync(d_part, 0, 3 * (size_t)g.nz * sizeof(double), st));
         CKL();
         std::vector<double> h(3 * (size_t)g.nz);
         CK(cudaMemcpyAsync(h.data(), d_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
