@@ -532,11 +532,11 @@ __global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
     const int p = blockIdx.x * Sh::L + l;
     const bool in = p < g.nx / 2 + 1;
     cplx<R>* col = S + (long long)blockIdx.y * g.ny * g.sp + p;
+    stage_roots<R, LOGN>(twn, tw, NT);   // (the first pass has no twiddles; the first exchange's barrier orders it)
     cplx<R> v[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e)
         v[e] = in ? col[(long long)reg_in<LOGN, false>(t, e) * g.sp] : cmk<R>(R(0), R(0));
-    stage_roots<R, LOGN>(twn, tw, NT);   // (the first pass has no twiddles; the first exchange's barrier orders it)
     reg_fft<R, LOGN, MODE == 1, false, true>(v, t, l, buf, twn);
     if (!in) return;
 #pragma unroll
@@ -594,17 +594,17 @@ __global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
     const bool in = p < g.nx / 2 + 1;
     const long long sk = (long long)g.ny * g.sp;
     cplx<R>* col = S + (long long)j * g.sp + p;
+    stage_roots<R, LOGN>(twn, tw, NT);
     cplx<R> v[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) v[e] = in ? col[reg_in<LOGN, false>(t, e) * sk] : cmk<R>(R(0), R(0));
-    stage_roots<R, LOGN>(twn, tw, NT);
     reg_fft<R, LOGN, false, false, true>(v, t, l, buf, twn);
     const double kxy = in ? kx2[p] + ky2[j] : 1.0;
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
         // the sum in the reference's order (kx2 + ky2) + kz2
         const double lam = -(kxy + __ldg(kz2 + reg_out<LOGN, false>(t, e)));
-        const R il = lam == 0.0 ? R(0) : R(nrm / lam);
+        const R il = lam == 0.0 ? R(0) : R(nrm * wrcp(lam));   // (an IEEE division a point: a third of the kernel)
         v[e] = cmk<R>(v[e].x * il, v[e].y * il);
     }
     // the inverse's first pass takes the points where the forward's last one left them
@@ -857,37 +857,45 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, cplx<RD>*
     thomas_wait<0>();
 }
 
-// r2c of an interior source along x: pack pairs, FFT, post-process.
-// DIV: the source is the divergence of the predicted velocity (us, vs, ws:
-// interior arrays), formed while the rows are staged with div_kernel's
-// arithmetic (plain, or W-weighted for the sound-proof core), instead of
-// being read from src: the divergence never goes to memory.
+// r2c of an interior source along x: pack pairs, FFT, post-process.  The
+// register form can take the divergence of the predicted velocity (us, vs, ws:
+// interior arrays) for its source, formed as the rows are loaded with
+// div_kernel's arithmetic (plain, or W-weighted for the sound-proof core): the
+// divergence never goes to memory.
 template <typename R, bool ANEL, bool UNI>
-__device__ __forceinline__ cplx<R> div_pair(const Geo& g, const R* __restrict__ us, const R* __restrict__ vs,
-                                            const R* __restrict__ ws, long long row, int i0) {
-    const int j = (int)(row % g.ny), k = (int)(row / g.ny);
-    const long long q = row * g.nx + i0, pl = (long long)g.nx * g.ny;
-    const Met<R, UNI> m(g);
-    const R uc0 = __ldg(us + q), uc1 = __ldg(us + q + 1);
-    const R ue = __ldg(us + (i0 + 2 < g.nx ? q + 2 : q + 2 - g.nx));
-    const long long qn = j + 1 < g.ny ? q + g.nx : q - (long long)(g.ny - 1) * g.nx;
-    const R vc0 = __ldg(vs + q), vc1 = __ldg(vs + q + 1), vn0 = __ldg(vs + qn), vn1 = __ldg(vs + qn + 1);
-    const R wc0 = __ldg(ws + q), wc1 = __ldg(ws + q + 1);
-    R wn0 = R(0), wn1 = R(0);   // the top wall face
-    if (k + 1 < g.nz) { wn0 = __ldg(ws + q + pl); wn1 = __ldg(ws + q + pl + 1); }
-    else if (g.bc_z == 0) {
-        const long long qb = q - (long long)(g.nz - 1) * pl;
-        wn0 = __ldg(ws + qb); wn1 = __ldg(ws + qb + 1);
+struct DivRow {   // a row of the predicted velocity with its north and top neighbours
+    const cplx<R>*uc, *vc, *vn, *wc, *wn;   // in pairs of x-adjacent cells
+    bool top;                               // wn is the top wall face: zero
+    int M;
+    R idx, idy, idz, wcv, wfb, wft;
+    __device__ __forceinline__ DivRow(const Geo& g, const R* us, const R* vs, const R* ws, long long row) {
+        const int j = (int)(row % g.ny), k = (int)(row / g.ny);
+        const long long q = row * g.nx, pl = (long long)g.nx * g.ny;
+        auto at = [](const R* p) { return reinterpret_cast<const cplx<R>*>(p); };
+        uc = at(us + q);
+        vc = at(vs + q);
+        vn = at(vs + (j + 1 < g.ny ? q + g.nx : q - (long long)(g.ny - 1) * g.nx));
+        wc = at(ws + q);
+        top = k + 1 >= g.nz && g.bc_z != 0;
+        wn = at(ws + (k + 1 < g.nz ? q + pl : (top ? q : q - (long long)(g.nz - 1) * pl)));
+        M = g.nx / 2;
+        const Met<R, UNI> m(g);
+        idx = R(g.idx); idy = R(g.idy); idz = m.idz(k);
+        if (ANEL) { wcv = m.wc(k); wfb = m.wf(k); wft = m.wf(k + 1); }
     }
-    const R idx = R(g.idx), idy = R(g.idy), idz = m.idz(k);
-    if (ANEL) {
-        const R wcv = m.wc(k), wfb = m.wf(k), wft = m.wf(k + 1);
-        return cmk<R>(wcv * ((uc1 - uc0) * idx + (vn0 - vc0) * idy) + (wft * wn0 - wfb * wc0) * idz,
-                      wcv * ((ue - uc1) * idx + (vn1 - vc1) * idy) + (wft * wn1 - wfb * wc1) * idz);
+    // the divergences of the cells 2n and 2n + 1 (div_kernel's arithmetic)
+    __device__ __forceinline__ cplx<R> operator()(int n) const {
+        const cplx<R> u = uc[n], v = vc[n], vq = vn[n], w = wc[n];
+        const R ue = uc[n + 1 < M ? n + 1 : 0].x;
+        cplx<R> wq = wn[n];
+        if (top) wq = cmk<R>(R(0), R(0));
+        if (ANEL)
+            return cmk<R>(wcv * ((u.y - u.x) * idx + (vq.x - v.x) * idy) + (wft * wq.x - wfb * w.x) * idz,
+                          wcv * ((ue - u.y) * idx + (vq.y - v.y) * idy) + (wft * wq.y - wfb * w.y) * idz);
+        return cmk<R>((u.y - u.x) * idx + (vq.x - v.x) * idy + (wq.x - w.x) * idz,
+                      (ue - u.y) * idx + (vq.y - v.y) * idy + (wq.y - w.y) * idz);
     }
-    return cmk<R>((uc1 - uc0) * idx + (vn0 - vc0) * idy + (wn0 - wc0) * idz,
-                  (ue - uc1) * idx + (vn1 - vc1) * idy + (wn1 - wc1) * idz);
-}
+};
 
 template <typename R>
 __global__ void __launch_bounds__(FFT_THREADS(R), FFT_MINB(R)) src_fftx_kernel(Geo g, const R* __restrict__ src, cplx<R>* __restrict__ S,
@@ -937,14 +945,17 @@ __global__ void __launch_bounds__(RegShape<LOGN>::THREADS, RegShape<LOGN>::MINB)
     const int t = threadIdx.x & (TPL - 1), l = threadIdx.x >> Sh::LOGT;
     const long long row = (long long)blockIdx.x * Sh::L + l;
     const long long rl = row < nrows ? row : nrows - 1;   // a row past the end repeats the last one
-    cplx<R> v[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-        const int n = reg_in<LOGN, false>(t, e);
-        if constexpr (DIV == 0) v[e] = reinterpret_cast<const cplx<R>*>(src + rl * g.nx)[n];
-        else v[e] = div_pair<R, (DIV & 3) == 2, (DIV & 4) == 0>(g, us, vs, ws, rl, 2 * n);
-    }
     stage_roots<R, LOGN>(twn, tw, NT);
+    cplx<R> v[16];
+    if constexpr (DIV == 0) {
+        const cplx<R>* in = reinterpret_cast<const cplx<R>*>(src + rl * g.nx);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = in[reg_in<LOGN, false>(t, e)];
+    } else {
+        const DivRow<R, (DIV & 3) == 2, (DIV & 4) == 0> div(g, us, vs, ws, rl);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = div(reg_in<LOGN, false>(t, e));
+    }
     reg_fft<R, LOGN, false, false, false>(v, t, l, buf, twn);
     __syncthreads();
 #pragma unroll

@@ -59,22 +59,6 @@ struct Nb {
 };
 
 // ---- WENO reconstructions (src/AdvectionSchemes.jl:105-120, :240-255, :319-333)
-// The reciprocal of the nonlinear weights' denominators, which lie in the
-// normal range.  FP32: rcp.approx (1 ulp).  FP64: the hardware's approximation
-// (its upper 32 bits, 20 bits good) and one third-order step of Newton's
-// series, r (1 + e + e^2) with e = 1 - x r: the error e^3 is below 2^-53.  Four
-// operations and no branch, against the ten-odd of an IEEE division.
-__device__ __forceinline__ float wrcp(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ double wrcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
 __device__ __forceinline__ float wabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double wabs(double x) { return fabs(x); }
 template <class VT>
