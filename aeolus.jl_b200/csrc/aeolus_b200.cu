@@ -1549,14 +1549,12 @@ struct Core : CoreBase {
                                        (size_t)tpx_z * g.nz * sizeof(cplx<R>), st>>>(g, S, tw, NT, tpx_z, kx2, ky2, kz2, nrm);
             });
         } else {
-            size_t smt = thomas_smem(g, true);
-            if (smt > 48 * 1024)
-                cudaFuncSetAttribute(thomas_kernel<R, true, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smt);
-            // d' in place in S; the factors m and c' from the tables made at set-up
-            R* ftab = reinterpret_cast<R*>(cps);
+            const size_t smt = thomas_tw_smem(g);
+            reg_smem(thomas_tw_kernel<R>, smt);
+            // d in place in S; the factors from the tables made at set-up
+            const R* ftab = reinterpret_cast<const R*>(cps);
             const long long ns = (long long)g.sp * g.ny * g.nz;
-            thomas_kernel<R, true, R, true><<<thomas_blocks(g), 32, smt, st>>>(g, S, S, ftab + ns, cc, ftab);
+            thomas_tw_kernel<R><<<thomas_blocks(g), 64, smt, st>>>(g, S, cc, ftab, ftab + ns);
         }
         CKL();
         mark(AEO_K_ZSOLVE);
@@ -1802,8 +1800,10 @@ struct Core : CoreBase {
         if (aeo_status e = sgs_ready()) return e;
         set_scalar_kernel<<<1, 1, 0, st>>>(&d_sc->dt, dt);
         CKL();
-        if (n >= 2) {
-            // the pairs of steps as one launch of the multi-step graph
+        if (pcg && n >= 2) {
+            // the pairs of steps as one launch of the multi-step graph (the direct solvers'
+            // steps are launched one by one below: a node of a WHILE body costs about a
+            // microsecond more than a node of a graph of its own, 23-30 us a step)
             cudaGraphExec_t ge;
             if (aeo_status e = multi_graph_for(&ge)) return e;
             steps_set_kernel<<<1, 1, 0, st>>>(d_steps, n / 2);

@@ -163,3 +163,14 @@ def test_column_projection_at_every_row_length(size, core, stretched):
         assert rel(s32.get_field(n)[g.interior], want) <= 1e-5, n
     b = np.random.default_rng(1).standard_normal((nz, g.ny, g.nx))
     assert rel(s64.pressure_solve(b), o.pressure_solve(b)) <= 1e-12
+
+
+# ---- the Thomas solve from both ends: every remainder of its unrolled loops ------------------------------------
+@pytest.mark.parametrize("nz", [2, 3, 4, 5, 6, 7, 8, 9, 15, 16, 17, 31, 64, 93])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("fp32_mixed", 1e-4)])
+def test_column_solve_of_every_depth(nz, precision, tol):
+    g = regular_grid((16, 4, nz), (1.0, 1.0, 0.1 * nz), bc_z="wall")
+    b = np.random.default_rng(nz).standard_normal((nz, 4, 16))
+    b -= b.mean()
+    s, o = Sim(CoreSpec(grid=g, precision=precision)), OracleSimulation(CoreSpec(grid=g))
+    assert rel(s.pressure_solve(b), o.pressure_solve(b)) <= tol
