@@ -16,34 +16,34 @@ struct HaloSet {
     int nf;
 };
 
-__device__ __forceinline__ void shell_point(const Geo& g, long long t, int* i, int* j, int* k) {
+template <typename I>
+__device__ __forceinline__ void shell_point(const Geo& g, I t, int* i, int* j, int* k) {
     const int H = AEO_H;
-    const long long bx = g.nx + 2 * H, by = g.ny + 2 * H;
-    const long long nzs = 2LL * H * bx * by;          // the two z slabs
+    const I bx = g.nx + 2 * H, by = g.ny + 2 * H;
+    const I nzs = 2 * H * bx * by;                    // the two z slabs
     if (t < nzs) {
-        long long s = t;
-        *i = (int)(s % bx) - H; s /= bx;
-        *j = (int)(s % by) - H; s /= by;
-        int kz = (int)s;
-        *k = kz < H ? kz - H : g.nz + (kz - H);
+        const I row = t / bx, kz = row / by;
+        *i = (int)(t - row * bx) - H;
+        *j = (int)(row - kz * by) - H;
+        *k = (int)kz < H ? (int)kz - H : g.nz + ((int)kz - H);
         return;
     }
     t -= nzs;
-    const long long nys = 2LL * H * bx * g.nz;        // the two y slabs (interior k)
+    const I nys = 2 * H * bx * g.nz;                  // the two y slabs (interior k)
     if (t < nys) {
-        long long s = t;
-        *i = (int)(s % bx) - H; s /= bx;
-        int jy = (int)(s % (2 * H)); s /= (2 * H);
+        const I row = t / bx, kk = row / (2 * H);
+        *i = (int)(t - row * bx) - H;
+        const int jy = (int)(row - kk * (2 * H));
         *j = jy < H ? jy - H : g.ny + (jy - H);
-        *k = (int)s;
+        *k = (int)kk;
         return;
     }
     t -= nys;                                          // the two x slabs (interior j, k)
-    long long s = t;
-    int ix = (int)(s % (2 * H)); s /= (2 * H);
+    const I row = t / (2 * H), kk = row / g.ny;
+    const int ix = (int)(t - row * (2 * H));
     *i = ix < H ? ix - H : g.nx + (ix - H);
-    *j = (int)(s % g.ny); s /= g.ny;
-    *k = (int)s;
+    *j = (int)(row - kk * g.ny);
+    *k = (int)kk;
 }
 
 __host__ __device__ __forceinline__ long long shell_count(const Geo& g) {
@@ -51,16 +51,20 @@ __host__ __device__ __forceinline__ long long shell_count(const Geo& g) {
     return 2 * H * bx * by + 2 * H * bx * g.nz + 2 * H * (long long)g.ny * g.nz;
 }
 
-template <typename R>
+// A thread a point, every field's source first, then the stores: the loads do
+// not wait for the stores of the fields before them (the arrays could alias, as
+// far as the compiler knows), so one memory latency a point instead of one a
+// field.  I: the integer of the shell's index arithmetic; its divisions were most
+// of what the kernel issued in 64 bits.  (A warp a row, the source row found once,
+// was slower: 29 us a launch against 21 on 256 x 256 x 128 FP32, too few warps in
+// flight.)
+template <typename R, typename I>
 __global__ void __launch_bounds__(256) halo_fill_kernel(Geo g, HaloSet<R> hs) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= shell_count(g)) return;
+    const I t = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (I)shell_count(g)) return;
     int i, j, k;
-    shell_point(g, t, &i, &j, &k);
+    shell_point<I>(g, t, &i, &j, &k);
     int ii = wrapi(i, g.nx), jj = wrapi(j, g.ny);
-    // every field's source first, then the stores: the loads do not wait for
-    // the stores of the fields before them (the arrays could alias, as far as
-    // the compiler knows), so one memory latency a point instead of one a field
     R v[5];
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
@@ -438,7 +442,7 @@ __global__ void __launch_bounds__(256) open_halo_fill_kernel(Geo g, HaloSet<R> h
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= shell_count(g)) return;
     int i, j, k;
-    shell_point(g, t, &i, &j, &k);
+    shell_point<long long>(g, t, &i, &j, &k);
     const int pid[4] = {pid4.x, pid4.y, pid4.z, pid4.w};
     R v[4];
 #pragma unroll

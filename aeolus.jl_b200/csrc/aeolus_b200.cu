@@ -1337,8 +1337,10 @@ struct Core : CoreBase {
         HaloSet<R> hs{};
         for (int q = 0; q < nf; ++q) { hs.f[q] = f[q]; hs.loc[q] = loc[q]; }
         hs.nf = nf;
-        long long n = shell_count(g);
-        halo_fill_kernel<R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, hs);
+        const long long n = shell_count(g);
+        const unsigned nb = (unsigned)((n + 255) / 256);
+        if (n < (1LL << 31) - 256) halo_fill_kernel<R, unsigned><<<nb, 256, 0, st>>>(g, hs);
+        else halo_fill_kernel<R, long long><<<nb, 256, 0, st>>>(g, hs);
         CKL();
         return AEO_OK;
     }
@@ -1454,7 +1456,7 @@ struct Core : CoreBase {
         return AEO_OK;
     }
 
-    // a register transform of FP64 lines of 512 points needs more than the default shared memory
+    // more than the default shared memory: register transforms of FP64 lines of 512 points, deep columns
     template <class K>
     void reg_smem(K* kernel, size_t bytes) {
         if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
