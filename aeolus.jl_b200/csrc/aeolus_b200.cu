@@ -1810,11 +1810,10 @@ struct Core : CoreBase {
             if (aeo_status e = multi_graph_for(&ge)) return e;
             steps_set_kernel<<<1, 1, 0, st>>>(d_steps, n / 2);
             CKL();
-            if (pcg)
-                if (aeo_status e = aeo_mg_order_before(mg, st)) {
-                    fail(std::string("the MG-PCG pressure solve: ") + aeo_mg_last_error(mg));
-                    return e;
-                }
+            if (aeo_status e = aeo_mg_order_before(mg, st)) {
+                fail(std::string("the MG-PCG pressure solve: ") + aeo_mg_last_error(mg));
+                return e;
+            }
             CK(cudaGraphLaunch(ge, st));
             n -= 2 * (n / 2);   // the state is back in set cur
         }
