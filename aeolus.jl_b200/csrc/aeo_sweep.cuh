@@ -571,8 +571,10 @@ __device__ __noinline__ R sigma_operator(R g11, R g12, R g13, R g21, R g22, R g2
 // with g.sgs_model = 1, Vreman's nut = c sqrt(B_beta / alpha:alpha) from the
 // same gradient tensor, B_beta in the Cauchy-Binet form over the rows a_m =
 // d_m u (_vreman_point / _vreman_body!, src/operators/sgs_amd_vreman.jl:93-100,
-// :293-298; uniform grids).
-template <typename R, bool UNI, class AU, class AV, class AW>
+// :293-298; uniform grids).  MODEL 0: Smagorinsky at compile time -- the sigma
+// model's out-of-line call kept a stack frame and its registers in every
+// Smagorinsky sweep; -1: by g.sgs_model.
+template <typename R, bool UNI, int MODEL = -1, class AU, class AV, class AW>
 __device__ __forceinline__ auto smag_point(const Met<R, UNI>& m, const Geo& g, int k, R c_s, const AU& U, const AV& V,
                                            const AW& W) {
     using VT = decltype(U(0, 0, 0));   // R, or a pair of FP32 lanes
@@ -588,6 +590,7 @@ __device__ __forceinline__ auto smag_point(const Met<R, UNI>& m, const Geo& g, i
     VT dw_dx = ((W(1, 0, 0) + W(1, 0, 1)) - (W(-1, 0, 0) + W(-1, 0, 1))) * (R(0.25) * idx);
     VT dv_dz = ((V(0, 0, 1) + V(0, 1, 1)) - (V(0, 0, -1) + V(0, 1, -1))) * (R(0.25) * ido);
     VT dw_dy = ((W(0, 1, 0) + W(0, 1, 1)) - (W(0, -1, 0) + W(0, -1, 1))) * (R(0.25) * idy);
+    if constexpr (MODEL != 0) {
     if (g.sgs_model == 2)   // sigma model: (C_sigma Delta)^2 D_sigma (compute_sigma_nut!, sigma_closure.jl:208-222)
         return VT(VT(coef) * sigma_operator(VT(du_dx), VT(du_dy), VT(du_dz), VT(dv_dx), VT(dv_dy), VT(dv_dz),
                                             VT(dw_dx), VT(dw_dy), VT(dw_dz)));
@@ -604,6 +607,7 @@ __device__ __forceinline__ auto smag_point(const Met<R, UNI>& m, const Geo& g, i
         VT aa = du_dx * du_dx + du_dy * du_dy + du_dz * du_dz + dv_dx * dv_dx + dv_dy * dv_dy + dv_dz * dv_dz +
                 dw_dx * dw_dx + dw_dy * dw_dy + dw_dz * dw_dz;
         return sqrt_ratio_or_zero(Bb, aa, R(g.sgs_cv));
+    }
     }
     VT S12 = R(0.5) * (du_dy + dv_dx), S13 = R(0.5) * (du_dz + dw_dx), S23 = R(0.5) * (dv_dz + dw_dy);
     VT S2 = R(2) * (du_dx * du_dx + dv_dy * dv_dy + dw_dz * dw_dz) + R(4) * (S12 * S12 + S13 * S13 + S23 * S23);

@@ -127,8 +127,8 @@ struct NutAcc {
     __device__ __forceinline__ NutAcc shifted(int o) const { return NutAcc{{p[0] + o, p[1] + o, p[2] + o}}; }
 };
 
-// CLOS: the closure of the coefficient pass: 0 the static ones (smag_point),
-// 1 the anisotropic minimum-dissipation closure (its kappa_t planes KT_OFS
+// CLOS: the closure of the coefficient pass: 0 Smagorinsky, 4 the other static
+// ones (smag_point: Vreman, sigma), 1 the anisotropic minimum-dissipation closure (its kappa_t planes KT_OFS
 // elements past the nut planes), 2 dynamic Smagorinsky (cs2 per level or
 // cell), 3 the TKE closure (tke_point; its kappa_t planes as the AMD's)
 template <typename R, int ADV, bool SGS, bool ANEL, bool UNI, int CLOS = 0>
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(TileShape<R, ADV, SGS>::NT) sweep_tile_kernel(
                         np[cj * S::NPW + ci] = nk.nu;
                         np[cj * S::NPW + ci + S::KT_OFS] = nk.ka;
                     } else {
-                        np[cj * S::NPW + ci] = smag_point<R, UNI>(m, g, L, R(a.c_s), Uq, Vq, Wq);
+                        np[cj * S::NPW + ci] = smag_point<R, UNI, CLOS == 0 ? 0 : -1>(m, g, L, R(a.c_s), Uq, Vq, Wq);
                     }
                 }
             }

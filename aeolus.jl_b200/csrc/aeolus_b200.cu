@@ -1345,97 +1345,55 @@ struct Core : CoreBase {
         return AEO_OK;
     }
 
+    // the sweep's closure flag (CLOS of the kernels): uniform grids have all, a
+    // stretched column Smagorinsky
+    template <bool SG, bool AN, bool UN, class Go>
+    void with_closure(Go go) {
+        if constexpr (SG && UN) {
+            if (amd()) return go(std::integral_constant<int, 1>{});
+            if (dyncl()) return go(std::integral_constant<int, 2>{});
+            if constexpr (!AN)
+                if (tke()) return go(std::integral_constant<int, 3>{});
+            if (cfg.sgs_model != AEO_SGS_SMAGORINSKY) return go(std::integral_constant<int, 4>{});
+        }
+        go(std::integral_constant<int, 0>{});
+    }
+    template <class K, class... A>
+    void sweep_go(K* kernel, dim3 grid, dim3 block, size_t smem, A... args) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<grid, block, smem, st>>>(args...);
+    }
+
     template <int ADV, bool SG, bool AN, bool UN>
     void launch_sweep_t(int s_in, const SweepArgs<R>& a) {
-        if constexpr (ADV == 0 && sizeof(R) == sizeof(float)) {
-            if (pair) {
-                using PS = PairShape<SG>;
-                // persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
-                const int ntx = (g.nx + PS::TX - 1) / PS::TX, nty = (g.ny + PS::TY - 1) / PS::TY;
-                const int items = ntx * nty * g.nz;
-                const dim3 grid((unsigned)std::min(items, PS::CTAS_PER_SM * nsm));
-                if constexpr (SG && UN) {
-                    if (amd()) {
-                        SweepArgs<R> b = a;
-                        b.kofs = PS::KT_OFS;
-                        cudaFuncSetAttribute(sweep_pair_kernel<SG, AN, UN, 1>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS::SMEM_AMD);
-                        sweep_pair_kernel<SG, AN, UN, 1><<<grid, dim3(PS::TXT, PS::TY), PS::SMEM_AMD, st>>>(
-                            tmaps[s_in], b, ntx, items, d_flag);
-                        return;
-                    }
-                }
-                if constexpr (SG && !AN && UN) {
-                    if (tke()) {
-                        SweepArgs<R> b = a;
-                        b.kofs = PS::KT_OFS;
-                        cudaFuncSetAttribute(sweep_pair_kernel<SG, AN, UN, 3>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS::SMEM_AMD);
-                        sweep_pair_kernel<SG, AN, UN, 3><<<grid, dim3(PS::TXT, PS::TY), PS::SMEM_AMD, st>>>(
-                            tmaps[s_in], b, ntx, items, d_flag);
-                        return;
-                    }
-                }
-                if constexpr (SG && UN) {
-                    if (dyncl()) {
-                        cudaFuncSetAttribute(sweep_pair_kernel<SG, AN, UN, 2>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS::SMEM);
-                        sweep_pair_kernel<SG, AN, UN, 2><<<grid, dim3(PS::TXT, PS::TY), PS::SMEM, st>>>(
-                            tmaps[s_in], a, ntx, items, d_flag);
-                        return;
-                    }
-                }
-                cudaFuncSetAttribute(sweep_pair_kernel<SG, AN, UN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)PS::SMEM);
-                sweep_pair_kernel<SG, AN, UN><<<grid, dim3(PS::TXT, PS::TY), PS::SMEM, st>>>(tmaps[s_in], a, ntx,
-                                                                                           items, d_flag);
-                return;
-            }
-        }
-        if constexpr (ADV > 0 && !SG && !AN && UN && sizeof(R) == sizeof(float)) {
+        if constexpr (ADV > 0 && !SG && sizeof(R) == sizeof(float)) {
             // FP32 WENO without a closure: cell pairs, every face once
             using WS = WPairShape;
             const dim3 grid((g.nx + WS::TX - 1) / WS::TX, (g.ny + WS::TY - 1) / WS::TY, (g.nz + wchunk - 1) / wchunk);
-            cudaFuncSetAttribute(sweep_wpair_kernel<ADV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS::SMEM);
-            sweep_wpair_kernel<ADV><<<grid, dim3(WS::TXT, WS::TY), WS::SMEM, st>>>(tmaps[s_in], a, wchunk, d_flag);
-            return;
-        }
-        using TS = TileShape<R, ADV, SG>;
-        dim3 grid((g.nx + TS::TX - 1) / TS::TX, (g.ny + TS::TY - 1) / TS::TY, (g.nz + kchunk - 1) / kchunk);
-        if constexpr (SG && UN) {
-            if (amd()) {
+            sweep_go(sweep_wpair_kernel<ADV>, grid, dim3(WS::TXT, WS::TY), WS::SMEM, tmaps[s_in], a, wchunk, d_flag);
+        } else {
+            with_closure<SG, AN, UN>([&](auto cl) {
+                constexpr int CLOS = cl;
+                constexpr bool kap = CLOS == 1 || CLOS == 3;
                 SweepArgs<R> b = a;
-                b.kofs = TS::KT_OFS;
-                cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 1>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM_AMD);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 1><<<grid, TS::NT, TS::SMEM_AMD, st>>>(
-                    tmaps[s_in], b, kchunk, d_flag);
-                return;
-            }
+                using PS = PairShape<R, SG>;
+                using TS = TileShape<R, ADV, SG>;
+                if constexpr (ADV == 0 && (!kap || PS::KAPPA)) {
+                    // centred, persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
+                    const int ntx = (g.nx + PS::TX - 1) / PS::TX, nty = (g.ny + PS::TY - 1) / PS::TY;
+                    const int items = ntx * nty * g.nz;
+                    const dim3 grid((unsigned)std::min(items, PS::CTAS_PER_SM * nsm));
+                    if (kap) b.kofs = PS::KT_OFS;
+                    sweep_go(sweep_pair_kernel<R, SG, AN, UN, CLOS>, grid, dim3(PS::TXT, PS::TY),
+                             kap ? PS::SMEM_AMD : PS::SMEM, tmaps[s_in], b, ntx, items, d_flag);
+                } else {
+                    const dim3 grid((g.nx + TS::TX - 1) / TS::TX, (g.ny + TS::TY - 1) / TS::TY, (g.nz + kchunk - 1) / kchunk);
+                    if (kap) b.kofs = TS::KT_OFS;
+                    sweep_go(sweep_tile_kernel<R, ADV, SG, AN, UN, CLOS>, grid, dim3(TS::NT), kap ? TS::SMEM_AMD : TS::SMEM,
+                             tmaps[s_in], b, kchunk, d_flag);
+                }
+            });
         }
-        if constexpr (SG && !AN && UN) {
-            if (tke()) {
-                SweepArgs<R> b = a;
-                b.kofs = TS::KT_OFS;
-                cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 3>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM_AMD);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 3><<<grid, TS::NT, TS::SMEM_AMD, st>>>(
-                    tmaps[s_in], b, kchunk, d_flag);
-                return;
-            }
-        }
-        if constexpr (SG && UN) {
-            if (dyncl()) {
-                cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN, 2>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM);
-                sweep_tile_kernel<R, ADV, SG, AN, UN, 2><<<grid, TS::NT, TS::SMEM, st>>>(
-                    tmaps[s_in], a, kchunk, d_flag);
-                return;
-            }
-        }
-        const size_t sm = TS::SMEM;
-        cudaFuncSetAttribute(sweep_tile_kernel<R, ADV, SG, AN, UN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        sweep_tile_kernel<R, ADV, SG, AN, UN><<<grid, TS::NT, sm, st>>>(tmaps[s_in], a, kchunk, d_flag);
     }
 
     aeo_status launch_sweep(int s_in, const SweepArgs<R>& a) {

@@ -192,3 +192,57 @@ def test_a_run_of_steps_is_its_single_steps(steps):
                 s.step_rk3(1e-3, n)
             out.append([s.get_field(n) for n in ("u", "v", "w", "theta", "p")])
         assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+# ---- the centred sweeps: persistent CTAs over (tile, level) items, 64 (FP32) or 32 (FP64) columns by 8 rows -----
+@pytest.mark.parametrize("size,wall", [((8, 4, 5), True), ((32, 8, 4), False), ((64, 16, 13), True), ((128, 4, 33), True),
+                                       ((32, 32, 64), False)])
+@pytest.mark.parametrize("sgs", [None, "smagorinsky", "vreman", "sigma", "dynamic", "amd"])
+def test_centred_steps_at_tile_and_range_edges(size, wall, sgs):
+    g = regular_grid(size, (2 * np.pi,) * 3, bc_z="wall" if wall else "periodic")
+    kw = dict(grid=g, nu=1e-3, theta0=300.0 if wall else 0.0)
+    if sgs:
+        kw.update(sgs=sgs, c_s=0.5 if sgs == "dynamic" else 0.17)
+    state = random_state(g, 7, 0.5)
+    state[3] += kw["theta0"]
+    o = OracleSimulation(CoreSpec(**kw))
+    s64, s32 = Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
+    for s in (o, s64, s32):
+        s.set_state(*state)
+        s.project()
+        s.step_rk3(1e-3, 2)
+    for n in ("u", "v", "w", "theta"):
+        want = o.get_field(n)[g.interior]
+        assert rel(s64.get_field(n)[g.interior], want) <= 1e-11, n
+        # the dynamic coefficient is a quotient of differences, its FP32 form the pair tests'
+        assert rel(s32.get_field(n)[g.interior], want) <= (1e-4 if sgs == "dynamic" else 1e-5), n
+
+
+@pytest.mark.parametrize("size", [(16, 8, 5), (64, 16, 33)])
+@pytest.mark.parametrize("core", ["boussinesq", "anelastic"])
+@pytest.mark.parametrize("stretched", [False, True])
+@pytest.mark.parametrize("c_s", [0.0, 0.17])
+def test_centred_steps_of_every_column_form(size, core, stretched, c_s):
+    from aeolus_b200 import stretched_grid, tanh_faces
+    from aeolus_b200.reference_state import anelastic_profiles, exponential_density
+    nz = size[2]
+    if stretched:
+        g = stretched_grid(size, (1000.0, 800.0, 600.0), tanh_faces(nz, 600.0, 0.8))
+    else:
+        g = regular_grid(size, (1000.0, 800.0, 600.0), bc_z="wall")
+    kw = dict(grid=g, nu=0.1, c_s=c_s, theta0=300.0, g=9.81)
+    if core == "anelastic":
+        prof = anelastic_profiles(g, exponential_density(g), np.full(nz, 300.0))
+        kw.update(core=core, wc=prof["wc"], wf=prof["wf"], thf=prof["thf"])
+    state = random_state(g, 8)
+    state[3] += 300.0
+    o, s64, s32 = OracleSimulation(CoreSpec(**kw)), Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
+    for s in (o, s64, s32):
+        s.set_state(*state)
+        s.project()
+        s.step_rk3(0.1, 2)
+    for n in ("u", "v", "w", "theta"):
+        want = o.get_field(n)[g.interior]
+        assert rel(s64.get_field(n)[g.interior], want) <= 1e-11, n
+        assert rel(s32.get_field(n)[g.interior], want) <= 1e-5, n
+
