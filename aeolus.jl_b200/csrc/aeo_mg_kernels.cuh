@@ -68,7 +68,6 @@ template <typename R> struct Level {
     R ix2, iy2, iz2;
     R* phi;
     R* b;
-    R* r;                               // residual (every level but the coarsest)
     Coef<R> c;
     double* bmean;                      // mean of b to subtract before use (device scalar)
 };
@@ -603,10 +602,64 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_rbgs_kernel(Level<R> L, Bc bc,
     }
 }
 
-// r = b - A phi on a level (_compute_residual!, src/Multigrid.jl:281-285):
-// one thread per cell, a 3-D grid; the arithmetic of aphi.
+// Coarse b = mean of the eight fine residuals r = b - A phi (_compute_residual!,
+// _restrict!, src/Multigrid.jl:281-285, :380-406), the residuals in the
+// arithmetic of aphi and summed in the reference's order, one thread per coarse
+// cell: no residual array goes to memory and comes back (as two kernels the pair
+// was bound by its loads' latency and moved 8 B a fine cell more; finest level of
+// 256 x 256 x 96 FP32: 58 us, now 32).  CF: the level's coefficient form, stab its table.
 template <typename R, int CF>
-__global__ void __launch_bounds__(RB_X * RB_Y) mg_residual_kernel(Level<R> F, Bc bc, const int* done) {
+__device__ __forceinline__ R restrict_cell(const Level<R>& F, Bc bc, const R* stab, int I, int J, int K) {
+    const int nx = F.nx, ny = F.ny, nz = F.nz, pl = nx * ny;
+    const R* f = F.phi;
+    // the neighbours outside the 2 x 2 x 2 block: steps from its low corner (periodic wrap, or the
+    // mirror: the cell itself)
+    const int i0 = 2 * I, j0 = 2 * J, k0 = 2 * K;
+    const int q0 = i0 + nx * (j0 + ny * k0);
+    const int dxm = i0 > 0 ? -1 : (bc.x == 0 ? nx - 1 : 0), dxp = i0 + 2 < nx ? 2 : (bc.x == 0 ? 2 - nx : 1);
+    const int dym = j0 > 0 ? -nx : (bc.y == 0 ? (ny - 1) * nx : 0), dyp = j0 + 2 < ny ? 2 * nx : (bc.y == 0 ? (2 - ny) * nx : nx);
+    const int dzm = k0 > 0 ? -pl : (bc.z == 0 ? (nz - 1) * pl : 0), dzp = k0 + 2 < nz ? 2 * pl : (bc.z == 0 ? (2 - nz) * pl : pl);
+    R c[2][2][2];
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) c[z][y][x] = f[q0 + x + y * nx + z * pl];
+    R s = R(0);
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int q = q0 + x + y * nx + z * pl;
+                const R cc = c[z][y][x];
+                const R fxm = x ? c[z][y][0] : f[q0 + y * nx + z * pl + dxm], fxp = x ? f[q0 + y * nx + z * pl + dxp] : c[z][y][1];
+                const R fym = y ? c[z][0][x] : f[q0 + x + z * pl + dym], fyp = y ? f[q0 + x + z * pl + dyp] : c[z][1][x];
+                const R fzm = z ? c[0][y][x] : f[q0 + x + y * nx + dzm], fzp = z ? f[q0 + x + y * nx + dzp] : c[1][y][x];
+                R a;
+                if (CF == CF_CONST) {
+                    a = (fxp - R(2) * cc + fxm) * F.ix2 + (fyp - R(2) * cc + fym) * F.iy2 + (fzp - R(2) * cc + fzm) * F.iz2;
+                } else {
+                    const int j = j0 + y, k = k0 + z;
+                    const int gx = q + j + ny * k, gy = q + nx * k;
+                    const R axm = face_coef<R, CF>(F.c.cx, F.c.kx, stab, gx), axp = face_coef<R, CF>(F.c.cx, F.c.kx, stab, gx + 1);
+                    const R aym = face_coef<R, CF>(F.c.cy, F.c.ky, stab, gy), ayp = face_coef<R, CF>(F.c.cy, F.c.ky, stab, gy + nx);
+                    const R azm = face_coef<R, CF>(F.c.cz, F.c.kz, stab, q), azp = face_coef<R, CF>(F.c.cz, F.c.kz, stab, q + pl);
+                    a = (axp * (fxp - cc) - axm * (cc - fxm)) * F.ix2 + (ayp * (fyp - cc) - aym * (cc - fym)) * F.iy2 +
+                        (azp * (fzp - cc) - azm * (cc - fzm)) * F.iz2;
+                }
+                s += F.b[q] - a;
+            }
+    return s * R(0.125);
+}
+
+// The last block stores the coarse mean that the coarse level subtracts before
+// use.
+template <typename R, int CF>
+__global__ void __launch_bounds__(RB_X * RB_Y) mg_restrict_kernel(Level<R> F, Level<R> Cl, Bc bc, double* part,
+                                                                 unsigned* counter, const int* done) {
     pdl_wait();
     __shared__ R stab[CF == CF_CODES ? 256 : 1];
     if (*done) return;
@@ -614,50 +667,10 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_residual_kernel(Level<R> F, Bc
         for (int q = tid(); q < 256; q += nthreads()) stab[q] = F.c.tab[q];
         __syncthreads();
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    const int nx = F.nx, ny = F.ny, nz = F.nz, pl = nx * ny;
-    if (i >= nx || j >= ny) return;
-    const int q = i + nx * (j + ny * k);
-    const Nbr n = nbr_of(q, i, j, k, nx, ny, nz, pl, bc);
-    const R* __restrict__ f = F.phi;
-    const R c = f[q];
-    R a;
-    if (CF == CF_CONST) {
-        a = (f[n.xp] - R(2) * c + f[n.xm]) * F.ix2 + (f[n.yp] - R(2) * c + f[n.ym]) * F.iy2 +
-            (f[n.zp] - R(2) * c + f[n.zm]) * F.iz2;
-    } else {
-        const int fx = q + j + ny * k, fy = q + nx * k;
-        const R fxm = face_coef<R, CF>(F.c.cx, F.c.kx, stab, fx), fxp = face_coef<R, CF>(F.c.cx, F.c.kx, stab, fx + 1);
-        const R fym = face_coef<R, CF>(F.c.cy, F.c.ky, stab, fy), fyp = face_coef<R, CF>(F.c.cy, F.c.ky, stab, fy + nx);
-        const R fzm = face_coef<R, CF>(F.c.cz, F.c.kz, stab, q), fzp = face_coef<R, CF>(F.c.cz, F.c.kz, stab, q + pl);
-        a = (fxp * (f[n.xp] - c) - fxm * (c - f[n.xm])) * F.ix2 + (fyp * (f[n.yp] - c) - fym * (c - f[n.ym])) * F.iy2 +
-            (fzp * (f[n.zp] - c) - fzm * (c - f[n.zm])) * F.iz2;
-    }
-    F.r[q] = F.b[q] - a;
-}
-
-// Coarse b = mean of the eight fine residuals (src/Multigrid.jl:380-406),
-// summed in the reference's order; one thread per coarse cell on a 3-D
-// grid.  The last block stores the coarse mean that the coarse level
-// subtracts before use.
-template <typename R>
-__global__ void mg_restrict_kernel(Level<R> F, Level<R> Cl, double* part, unsigned* counter, const int* done) {
-    pdl_wait();
-    if (*done) return;
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y, K = blockIdx.z;
     double v[1] = {0.0};
     if (I < Cl.nx && J < Cl.ny) {
-        const int sy = F.nx, sz = F.nx * F.ny;
-        const R* r = F.r + (2 * I) + sy * (2 * J) + sz * (2 * K);
-        R s = r[0];
-        s += r[1];
-        s += r[sy];
-        s += r[sy + 1];
-        s += r[sz];
-        s += r[sz + 1];
-        s += r[sz + sy];
-        s += r[sz + sy + 1];
-        const R bcv = s * R(0.125);
+        const R bcv = restrict_cell<R, CF>(F, bc, stab, I, J, K);
         Cl.b[Cl.nx * (J + Cl.ny * K) + I] = bcv;
         v[0] = double(bcv);
     }

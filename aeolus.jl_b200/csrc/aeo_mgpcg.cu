@@ -361,7 +361,6 @@ struct Mg : MgBase {
             V.iz2 = R(1) / (R(dz) * R(dz));
             if (aeo_status s = dalloc(&V.phi, V.n)) return s;
             if (aeo_status s = dalloc(&V.b, V.n)) return s;
-            V.r = nullptr;
             V.bmean = bmeans + nl;
             V.c = Coef<R>();
             if (coeff) {
@@ -412,7 +411,6 @@ struct Mg : MgBase {
                 restrict_coeff(nx, ny, nz, hx, hy, hz, cnx, cny, cnz, Cx, Cy, Cz);
                 hx.swap(Cx); hy.swap(Cy); hz.swap(Cz);
             }
-            if (aeo_status s = dalloc(&V.r, V.n)) return s;
             nx = cnx; ny = cny; nz = cnz;
             dx *= 2; dy *= 2; dz *= 2;
         }
@@ -510,7 +508,7 @@ struct Mg : MgBase {
 
     int vcycle_launches() const {
         int c = 1;   // coarsest
-        for (int l = 0; l < nl - 1; ++l) c += 2 * cfg.nu1 + 2 * cfg.nu2 + 3;
+        for (int l = 0; l < nl - 1; ++l) c += 2 * cfg.nu1 + 2 * cfg.nu2 + 2;
         return c;
     }
 
@@ -564,9 +562,7 @@ struct Mg : MgBase {
                 for (int c = 0; c < 2; ++c)
                     if (aeo_status q = launch_rbgs(s, F, c, done)) return q;
             Level<R>& Cl = L[l + 1];
-            if (aeo_status q = launch_residual(s, F, done)) return q;
-            AEO_PDL_LAUNCH((mg_restrict_kernel<R>), restrict_grid(Cl), blk, 0, s, F, Cl, part, &S->counter, done);
-            CKL();
+            if (aeo_status q = launch_restrict(s, F, Cl, done)) return q;
         }
         if (aeo_status q = launch_coarsest(s, L[nl - 1], nullptr, done)) return q;
         for (int l = nl - 2; l >= 0; --l) {
@@ -598,11 +594,12 @@ struct Mg : MgBase {
         CKL();
         return AEO_OK;
     }
-    aeo_status launch_residual(cudaStream_t s, const Level<R>& F, const int* done) {
-        const dim3 g = cell_grid(F), blk(RB_X, RB_Y);
-        if (F.c.kx) AEO_PDL_LAUNCH((mg_residual_kernel<R, CF_CODES>), g, blk, 0, s, F, bc, done);
-        else if (F.c.cx) AEO_PDL_LAUNCH((mg_residual_kernel<R, CF_VALUES>), g, blk, 0, s, F, bc, done);
-        else AEO_PDL_LAUNCH((mg_residual_kernel<R, CF_CONST>), g, blk, 0, s, F, bc, done);
+    // the coarse right-hand side of level F's residual
+    aeo_status launch_restrict(cudaStream_t s, const Level<R>& F, const Level<R>& Cl, const int* done) {
+        const dim3 g = restrict_grid(Cl), blk(RB_X, RB_Y);
+        if (F.c.kx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CODES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
+        else if (F.c.cx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_VALUES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
+        else AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CONST>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
         CKL();
         return AEO_OK;
     }
@@ -1046,11 +1043,7 @@ struct Mg : MgBase {
             case 4: return launch_coarsest(st, L[nl - 1], nl == 1 ? r : nullptr, dzero);
             case 5: {
                 if (nl < 2) { fail("profile: one level, no restriction"); return AEO_ERR_ARGUMENT; }
-                if (aeo_status q = launch_residual(st, L[0], dzero)) return q;
-                AEO_PDL_LAUNCH((mg_restrict_kernel<R>), restrict_grid(L[1]), dim3(RB_X, RB_Y), 0, st, L[0], L[1], part, &S->counter,
-                                                                                      dzero);
-                CKL();
-                return AEO_OK;
+                return launch_restrict(st, L[0], L[1], dzero);
             }
             case 6: {
                 if (nl < 2) { fail("profile: one level, no smoothing sweep"); return AEO_ERR_ARGUMENT; }
