@@ -21,6 +21,12 @@ constexpr int COARSE_MAX_CELLS = 16384;
 // kernel wrote, for that kernel's completion and memory (a no-op when the
 // launch had no such attribute).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next programmatic launch start while this kernel still runs: it prepares what does
+// not change during a solve (coefficients, indices) and then waits in pdl_wait.  Only for a
+// kernel whose successor reads what changes with plain loads after that wait: one that
+// takes the read-only path (phi of large levels, the CG vectors) may find lines that
+// were fetched while this kernel was writing them.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 constexpr int RB_X = 32, RB_Y = 8;     // block of the 3-D stencil grids
 
@@ -259,9 +265,10 @@ __global__ void pcg_mean_kernel(const double* __restrict__ a, int n, PcgState* S
     }
 }
 
-// r = b - mb (zero guess), x = 0; (|b - mb|^2, sum r); a zero rhs ends the solve
+// r = b - mb (zero guess), x = 0; (|b - mb|^2, sum r); a zero rhs ends the solve;
+// the condition of the loop (0: no loop follows)
 __global__ void pcg_init_kernel(const double* __restrict__ b, double* __restrict__ r, double* __restrict__ x, int n,
-                                PcgState* S, double* part) {
+                                PcgState* S, double* part, cudaGraphConditionalHandle loop) {
     const double mb = S->mb;
     double v[2] = {0.0, 0.0};
     GRID_STRIDE(q, n) {
@@ -273,7 +280,8 @@ __global__ void pcg_init_kernel(const double* __restrict__ b, double* __restrict
     }
     double t[2];
     if (reduce_last<2>(v, part, &S->counter, t) && tid() == 0) {
-        S->bnorm = sqrt(t[0]);
+        S->bnorm = S->rnorm = sqrt(t[0]);
+        S->rprev = INFINITY;
         S->mr = S->project ? t[1] / S->n : 0.0;
         S->iters = 0;
         S->curvature = nan("");
@@ -289,6 +297,7 @@ __global__ void pcg_init_kernel(const double* __restrict__ b, double* __restrict
             S->status = MG_MAXIT;
             S->done = 0;
         }
+        if (loop) cudaGraphSetConditional(loop, S->done == 0 && S->maxit > 0);
     }
 }
 
@@ -351,11 +360,15 @@ __global__ void __launch_bounds__(RB_X * RB_Y) pcg_apply_kernel(const double* __
     }
 }
 
-// x += alpha p, r -= alpha Ap; (r.r, sum r); the convergence test
+// x += alpha p, r -= alpha Ap; (r.r, sum r); the convergence test and the loop's condition
 __global__ void pcg_update_kernel(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-                                  const double* __restrict__ Ap, int n, PcgState* S, double* part) {
+                                  const double* __restrict__ Ap, int n, PcgState* S, double* part,
+                                  cudaGraphConditionalHandle loop) {
     pdl_wait();
-    if (S->done) return;
+    if (S->done) {
+        if (blockIdx.x == 0 && tid() == 0) cudaGraphSetConditional(loop, 0);
+        return;
+    }
     const double alpha = S->alpha;
     double v[2] = {0.0, 0.0};
     GRID_STRIDE(q, n) {
@@ -374,6 +387,7 @@ __global__ void pcg_update_kernel(double* __restrict__ x, double* __restrict__ r
             S->status = MG_CONVERGED;
             S->done = 1;
         }
+        cudaGraphSetConditional(loop, S->done == 0 && S->iters < S->maxit);
     }
 }
 
@@ -381,10 +395,9 @@ __global__ void pcg_update_kernel(double* __restrict__ x, double* __restrict__ r
 // m = sum z / n, (r.z) -= m sum r, and beta (Polak-Ribiere when flexible)
 template <typename Z>
 __global__ void pcg_rz_kernel(const double* __restrict__ r, const Z* __restrict__ z, const double* __restrict__ Ap,
-                              int n, PcgState* S, double* part, int first) {
+                              int n, PcgState* S, double* part) {
     pdl_wait();
-    if (S->done) return;
-    const bool flex = S->flexible && !first;
+    const bool first = S->iters == 0, flex = S->flexible && !first;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     GRID_STRIDE(q, n) {
         double rv = r[q], zv = double(z[q]);
@@ -427,9 +440,9 @@ __global__ void pcg_rz_kernel(const double* __restrict__ r, const Z* __restrict_
 
 // p = (z - m) + beta p  (p = z - m on the first pass)
 template <typename Z>
-__global__ void pcg_dir_kernel(double* __restrict__ p, const Z* __restrict__ z, int n, const PcgState* S, int first) {
+__global__ void pcg_dir_kernel(double* __restrict__ p, const Z* __restrict__ z, int n, const PcgState* S) {
     pdl_wait();
-    if (S->done) return;
+    const bool first = S->iters == 0;
     const double m = S->m, beta = S->beta;
     GRID_STRIDE(q, n) p[q] = first ? double(z[q]) - m : (double(z[q]) - m) + beta * p[q];
 }
@@ -437,17 +450,14 @@ __global__ void pcg_dir_kernel(double* __restrict__ p, const Z* __restrict__ z, 
 // z = r / diag(A), the Jacobi preconditioner (1/diag precomputed; 0 on a
 // fully blocked cell)
 __global__ void pcg_jacobi_kernel(double* __restrict__ z, const double* __restrict__ r,
-                                  const double* __restrict__ invd, int n, const PcgState* S) {
+                                  const double* __restrict__ invd, int n) {
     pdl_wait();
-    if (S->done) return;
     GRID_STRIDE(q, n) z[q] = r[q] * invd[q];
 }
 
-// the loop condition of the WHILE node: mode 0 CG, mode 1 multigrid cycles
-__global__ void pcg_cond_kernel(PcgState* S, cudaGraphConditionalHandle h, int mode) {
-    unsigned go = (S->done == 0 && S->iters < S->maxit) ? 1u : 0u;
-    if (mode == 0 && S->done == 0 && S->iters >= S->maxit) S->status = MG_MAXIT;
-    cudaGraphSetConditional(h, go);
+// the loop condition of the standalone cycles
+__global__ void mg_cond_kernel(PcgState* S, cudaGraphConditionalHandle h) {
+    cudaGraphSetConditional(h, S->done == 0 && S->iters < S->maxit);
 }
 
 // The preconditioner of the next application (the IF node's value): the
@@ -489,33 +499,49 @@ __global__ void shift_kernel(double* __restrict__ x, int n, const PcgState* S) {
 // ------------------------------------------------------- multigrid kernels
 // 3-D grids: x lanes over half-rows (RB) or cells, y over rows j, z over planes k.
 
+template <typename R> struct Vec2;
+template <> struct Vec2<float> { using T = float2; };
+template <> struct Vec2<double> { using T = double2; };
+
 // The first half-sweep of a level whose phi starts at zero: every neighbour
 // is zero, so colour-0 cells take (b - 0)/diag, colour-1 cells stay 0.
 // Fused with the zeroing and with the mean projection of the level's
 // right-hand side (level 0 takes it from the FP64 residual r - mean r).
-// One thread per pair of cells (2ih, 2ih+1).
-template <typename R>
-__global__ void mg_first_kernel(Level<R> L, Bc bc, const double* __restrict__ r0, const double* mr0, const int* done) {
-    pdl_wait();
-    if (*done) return;
+// One thread per pair of cells (2ih, 2ih+1), whose coefficients are fetched
+// before the wait for the kernel ahead.
+template <typename R, int CF>
+__global__ void __launch_bounds__(RB_X * RB_Y) mg_first_kernel(Level<R> L, Bc bc, const double* __restrict__ r0,
+                                                              const double* mr0, int early) {
+    __shared__ R stab[CF == CF_CODES ? 256 : 1];
+    if (early) pdl_trigger();
+    if (CF == CF_CODES) {
+        for (int q = tid(); q < 256; q += nthreads()) stab[q] = __ldg(L.c.tab + q);
+        __syncthreads();
+    }
     const int ih = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (ih >= (L.nx >> 1) || j >= L.ny) return;
+    const bool in = ih < (L.nx >> 1) && j < L.ny;
+    const int s = (j + k) & 1, q0 = L.nx * (j + L.ny * k) + 2 * ih;   // s: the pair's cell of colour 0
+    R diag = -R(2) * (L.ix2 + L.iy2 + L.iz2);
+    bool open = true;
+    if (CF != CF_CONST && in) {
+        const int q = q0 + s, fx = q + j + L.ny * k, fy = q + L.nx * k;
+        const R fxp = face_coef<R, CF>(L.c.cx, L.c.kx, stab, fx + 1), fxm = face_coef<R, CF>(L.c.cx, L.c.kx, stab, fx);
+        const R fyp = face_coef<R, CF>(L.c.cy, L.c.ky, stab, fy + L.nx), fym = face_coef<R, CF>(L.c.cy, L.c.ky, stab, fy);
+        const R fzp = face_coef<R, CF>(L.c.cz, L.c.kz, stab, q + L.nx * L.ny), fzm = face_coef<R, CF>(L.c.cz, L.c.kz, stab, q);
+        diag = -((fxp + fxm) * L.ix2 + (fyp + fym) * L.iy2 + (fzp + fzm) * L.iz2);
+        open = !(fabs(diag) < Eps<R>::v());
+    }
+    pdl_wait();
+    if (!in) return;
     const double m0 = r0 ? *mr0 : 0.0;
     const R m = r0 ? R(0) : R(*L.bmean);
+    R bv[2];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        const int i = 2 * ih + s;
-        const int q = L.nx * (j + L.ny * k) + i;
-        R bv = r0 ? R(r0[q] - m0) : L.b[q] - m;
-        L.b[q] = bv;
-        R out = R(0);
-        if (((i + j + k) & 1) == 0) {
-            Idx d = make_idx(i, j, k, L.nx, L.ny, L.nz, bc);
-            R diag;
-            if (gs_diag<R>(d, L, &diag)) out = (bv - R(0)) / diag;
-        }
-        L.phi[q] = out;
-    }
+    for (int c = 0; c < 2; ++c) bv[c] = r0 ? R(r0[q0 + c] - m0) : L.b[q0 + c] - m;
+    const R out = open ? (s ? bv[1] : bv[0]) / diag : R(0);
+    using V2 = typename Vec2<R>::T;
+    *reinterpret_cast<V2*>(L.b + q0) = V2{bv[0], bv[1]};
+    *reinterpret_cast<V2*>(L.phi + q0) = s ? V2{R(0), out} : V2{out, R(0)};
 }
 
 // One colour pass of red-black Gauss-Seidel over an even-nx level.  A
@@ -529,32 +555,31 @@ __global__ void mg_first_kernel(Level<R> L, Bc bc, const double* __restrict__ r0
 // table, padded to 256 entries, staged in shared memory); K = 1 on levels too
 // small to fill the GPU with K-level columns.
 
-template <typename R> struct Vec2;
-template <> struct Vec2<float> { using T = float2; };
-template <> struct Vec2<double> { using T = double2; };
-
 template <typename R, int CF, int RB_K>
-__global__ void __launch_bounds__(RB_X * RB_Y) mg_rbgs_kernel(Level<R> L, Bc bc, int colour, const int* done) {
-    pdl_wait();
+__global__ void __launch_bounds__(RB_X * RB_Y) mg_rbgs_kernel(Level<R> L, Bc bc, int colour, int early) {
     __shared__ R stab[CF == CF_CODES ? 256 : 1];
-    if (*done) return;
+    if (RB_K == 1 && early) pdl_trigger();
+    if (RB_K > 1) pdl_wait();
     if (CF == CF_CODES) {
-        for (int q = tid(); q < 256; q += nthreads()) stab[q] = L.c.tab[q];
+        for (int q = tid(); q < 256; q += nthreads()) stab[q] = __ldg(L.c.tab + q);
         __syncthreads();
     }
     using V2 = typename Vec2<R>::T;
     const int ih = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k0 = blockIdx.z * RB_K;
     const int nx = L.nx, ny = L.ny, nz = L.nz, pl = nx * ny;
-    if (ih >= (nx >> 1) || j >= ny) return;
+    if (ih >= (nx >> 1) || j >= ny) {
+        if (RB_K == 1) pdl_wait();
+        return;
+    }
     const int i0 = 2 * ih, row0 = i0 + nx * j;
     // in-plane neighbours outside the pair (-1 / 0: the Neumann mirror, the cell itself)
     const int xl = i0 > 0 ? row0 - 1 : (bc.x == 0 ? row0 + nx - 1 : -1);
     const int xr = i0 + 2 < nx ? row0 + 2 : (bc.x == 0 ? row0 + 2 - nx : -1);
     const int dym = j > 0 ? -nx : (bc.y == 0 ? (ny - 1) * nx : 0);
     const int dyp = j < ny - 1 ? nx : (bc.y == 0 ? -(ny - 1) * nx : 0);
-    const R* __restrict__ f = L.phi;
-    // the coefficient codes / values and b through restrict pointers: no store
+    const R* f = L.phi;
+    // the coefficient codes / values through restrict pointers: no store
     // of this kernel (phi's colour) touches them, so the loads of the levels
     // ahead need not wait for the stores of the levels before (the byte codes
     // could alias phi as far as the compiler knows)
@@ -564,11 +589,32 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_rbgs_kernel(Level<R> L, Bc bc,
     const R* __restrict__ ccx = L.c.cx;
     const R* __restrict__ ccy = L.c.cy;
     const R* __restrict__ ccz = L.c.cz;
-    const R* __restrict__ bb = L.b;
-    // phi through the non-coherent path as well: a colour pass reads only the
-    // other colour's cells and the cells this thread itself writes (before it
-    // writes them), so no value read here changes during the pass
-    auto pair_at = [&](int k) { return __ldg(reinterpret_cast<const V2*>(f + (size_t)k * pl + row0)); };
+    const R* bb = L.b;
+    // phi through the non-coherent path as well where a thread marches: a colour
+    // pass reads only the other colour's cells and the cells this thread itself
+    // writes (before it writes them), so no value read here changes during the
+    // pass.  A one-level pass may start while the kernel ahead still writes phi and
+    // takes plain loads after the wait.
+    auto ld = [&](const R* a) { return RB_K == 1 ? *a : __ldg(a); };
+    auto pair_at = [&](int k) {
+        const V2* a = reinterpret_cast<const V2*>(f + (size_t)k * pl + row0);
+        return RB_K == 1 ? *a : __ldg(a);
+    };
+    R fxp = R(0), fxm = R(0), fyp = R(0), fym = R(0), fzp = R(0), fzm = R(0);
+    auto coefs = [&](int q, int k) {
+        if (CF == CF_CONST) return;
+        const int fx = q + j + ny * k, fy = q + nx * k;   // (nx+1)(j + ny k) + i, nx(j + (ny+1) k) + i
+        fxm = face_coef<R, CF>(ccx, ckx, stab, fx);
+        fxp = face_coef<R, CF>(ccx, ckx, stab, fx + 1);
+        fym = face_coef<R, CF>(ccy, cky, stab, fy);
+        fyp = face_coef<R, CF>(ccy, cky, stab, fy + nx);
+        fzm = face_coef<R, CF>(ccz, ckz, stab, q);
+        fzp = face_coef<R, CF>(ccz, ckz, stab, q + pl);
+    };
+    if (RB_K == 1) {
+        coefs(k0 * pl + row0 + ((j + k0 + colour) & 1), k0);
+        pdl_wait();
+    }
     V2 pc = pair_at(k0);
     V2 pm = k0 > 0 ? pair_at(k0 - 1) : (bc.z == 0 ? pair_at(nz - 1) : pc);
 #pragma unroll
@@ -579,23 +625,14 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_rbgs_kernel(Level<R> L, Bc bc,
         const int a = (j + k + colour) & 1;   // the pair's cell of this colour
         const int q = k * pl + row0 + a;
         const R c = a ? pc.y : pc.x;
-        const R nxm = a ? pc.x : (xl >= 0 ? __ldg(f + k * pl + xl) : c);
-        const R nxp = a ? (xr >= 0 ? __ldg(f + k * pl + xr) : c) : pc.y;
-        const R nym = dym ? __ldg(f + q + dym) : c;
-        const R nyp = dyp ? __ldg(f + q + dyp) : c;
+        const R nxm = a ? pc.x : (xl >= 0 ? ld(f + k * pl + xl) : c);
+        const R nxp = a ? (xr >= 0 ? ld(f + k * pl + xr) : c) : pc.y;
+        const R nym = dym ? ld(f + q + dym) : c;
+        const R nyp = dyp ? ld(f + q + dyp) : c;
         const R nzm = a ? pm.y : pm.x, nzp = a ? pp.y : pp.x;
-        R fxp = R(0), fxm = R(0), fyp = R(0), fym = R(0), fzp = R(0), fzm = R(0);
-        if (CF != CF_CONST) {
-            const int fx = q + j + ny * k, fy = q + nx * k;   // (nx+1)(j + ny k) + i, nx(j + (ny+1) k) + i
-            fxm = face_coef<R, CF>(ccx, ckx, stab, fx);
-            fxp = face_coef<R, CF>(ccx, ckx, stab, fx + 1);
-            fym = face_coef<R, CF>(ccy, cky, stab, fy);
-            fyp = face_coef<R, CF>(ccy, cky, stab, fy + nx);
-            fzm = face_coef<R, CF>(ccz, ckz, stab, q);
-            fzp = face_coef<R, CF>(ccz, ckz, stab, q + pl);
-        }
+        if (RB_K > 1) coefs(q, k);
         R v;
-        if (gs_vals<R, CF>(nxp, nxm, nyp, nym, nzp, nzm, fxp, fxm, fyp, fym, fzp, fzm, __ldg(bb + q), L.ix2, L.iy2, L.iz2, &v))
+        if (gs_vals<R, CF>(nxp, nxm, nyp, nym, nzp, nzm, fxp, fxm, fyp, fym, fzp, fzm, ld(bb + q), L.ix2, L.iy2, L.iz2, &v))
             L.phi[q] = v;
         pm = pc;
         pc = pp;
@@ -659,14 +696,14 @@ __device__ __forceinline__ R restrict_cell(const Level<R>& F, Bc bc, const R* st
 // use.
 template <typename R, int CF>
 __global__ void __launch_bounds__(RB_X * RB_Y) mg_restrict_kernel(Level<R> F, Level<R> Cl, Bc bc, double* part,
-                                                                 unsigned* counter, const int* done) {
-    pdl_wait();
+                                                                 unsigned* counter, int early) {
     __shared__ R stab[CF == CF_CODES ? 256 : 1];
-    if (*done) return;
+    if (early) pdl_trigger();
     if (CF == CF_CODES) {
-        for (int q = tid(); q < 256; q += nthreads()) stab[q] = F.c.tab[q];
+        for (int q = tid(); q < 256; q += nthreads()) stab[q] = __ldg(F.c.tab + q);
         __syncthreads();
     }
+    pdl_wait();
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y, K = blockIdx.z;
     double v[1] = {0.0};
     if (I < Cl.nx && J < Cl.ny) {
@@ -681,9 +718,9 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_restrict_kernel(Level<R> F, Le
 // phi_fine += trilinear (3/4, 1/4) interpolation of phi_coarse
 // (src/Multigrid.jl:412-455), the eight terms in the reference's order.
 template <typename R>
-__global__ void mg_prolong_kernel(Level<R> F, Level<R> Cl, Bc bc, const int* done) {
+__global__ void mg_prolong_kernel(Level<R> F, Level<R> Cl, Bc bc, int early) {
+    if (early) pdl_trigger();
     pdl_wait();
-    if (*done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
     if (i >= F.nx || j >= F.ny) return;
     const int Ih = i >> 1, Jh = j >> 1, Kh = k >> 1;
@@ -723,9 +760,8 @@ template <typename R>
 __global__ void __launch_bounds__(COARSE_THREADS) mg_coarsest_kernel(Level<R> L, R* spare, Bc bc, int sweeps,
                                                                     int staged, int inplace,
                                                                     const double* __restrict__ r0, const double* mr0,
-                                                                    const int* done, R* mat) {
+                                                                    R* mat) {
     pdl_wait();
-    if (*done) return;
     const int unit = mat ? (int)blockIdx.x : -1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nx = L.nx, ny = L.ny, nz = L.nz, n = L.n;
@@ -832,9 +868,9 @@ __global__ void __launch_bounds__(COARSE_THREADS) mg_coarsest_kernel(Level<R> L,
 // dependent passes on one.  One warp per row, FP64 accumulation, fixed order.
 template <typename R>
 __global__ void mg_coarse_matvec_kernel(Level<R> L, const R* __restrict__ mat, const double* __restrict__ r0,
-                                        const double* mr0, const int* done) {
+                                        const double* mr0, int early) {
+    if (early) pdl_trigger();
     pdl_wait();
-    if (*done) return;
     const int n = L.n;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= n) return;
@@ -860,9 +896,8 @@ constexpr int COL_NZ = 8;
 template <typename R, int MAXT>
 __global__ void __launch_bounds__(MAXT) mg_coarsest_col_kernel(Level<R> L, Bc bc, int sweeps,
                                                                         const double* __restrict__ r0,
-                                                                        const double* mr0, const int* done) {
+                                                                        const double* mr0) {
     pdl_wait();
-    if (*done) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nx = L.nx, ny = L.ny, nz = L.nz, n = L.n, ncol = nx * ny;
     const int ncx = (nx + 1) * ny * nz, ncy = nx * (ny + 1) * nz, ncz = nx * ny * (nz + 1);

@@ -233,7 +233,6 @@ struct Mg : MgBase {
     PcgState* S = nullptr;
     PcgState* hS = nullptr;        // pinned host copy
     cudaEvent_t ev_own = nullptr;  // orders this handle's stream before a launch on another
-    int* dzero = nullptr;          // a device flag that stays 0 (kernels run outside a solve)
     int coarse_staged = 0;
     int coarse_inplace = 1;        // 0 when a periodic axis of the coarsest level has an odd length
     size_t coarse_smem = 0;
@@ -445,12 +444,9 @@ struct Mg : MgBase {
         // the matrix is modest: one block per unit right-hand side
         if (coarse_staged && (size_t)C.n * C.n * sizeof(R) <= (size_t(512) << 20) && cfg.coarse_sweeps > 0) {
             if (aeo_status s = dalloc(&coarse_mat, (size_t)C.n * C.n)) return s;
-            int* dz = nullptr;
-            if (aeo_status s = dalloc(&dz, 1)) return s;
-            CK(cudaMemset(dz, 0, sizeof(int)));
             mg_coarsest_kernel<R><<<C.n, COARSE_THREADS, coarse_smem, st>>>(L[nl - 1], coarse_spare, bc,
                                                                             cfg.coarse_sweeps, 1, coarse_inplace,
-                                                                            nullptr, nullptr, dz, coarse_mat);
+                                                                            nullptr, nullptr, coarse_mat);
             CKL();
             CK(cudaStreamSynchronize(st));
         }
@@ -472,8 +468,6 @@ struct Mg : MgBase {
         }
         if (aeo_status s = dalloc(&part, part_cap)) return s;
         if (aeo_status s = dalloc(&S, 1)) return s;
-        if (aeo_status s = dalloc(&dzero, 1)) return s;
-        CK(cudaMemset(dzero, 0, sizeof(int)));
         CK(cudaMallocHost(&hS, sizeof(PcgState)));
         PcgState h0{};
         h0.tol = cfg.tol;
@@ -512,25 +506,24 @@ struct Mg : MgBase {
         return c;
     }
 
-    aeo_status launch_coarsest(cudaStream_t s, Level<R>& C, const double* r0, const int* done) {
+    aeo_status launch_coarsest(cudaStream_t s, Level<R>& C, const double* r0) {
         if (coarse_mat) {
-            AEO_PDL_LAUNCH((mg_coarse_matvec_kernel<R>), (C.n + 7) / 8, 256, 0, s, C, coarse_mat, r0, &S->mr, done);
+            AEO_PDL_LAUNCH((mg_coarse_matvec_kernel<R>), (C.n + 7) / 8, 256, 0, s, C, coarse_mat, r0, &S->mr, nl > 1);
             CKL();
             return AEO_OK;
         }
         if (coarse_col) {
             if (coarse_col_threads <= 256)
                 AEO_PDL_LAUNCH((mg_coarsest_col_kernel<R, 256>), 1, coarse_col_threads, coarse_col_smem, s, C, bc, cfg.coarse_sweeps,
-                                                                                             r0, &S->mr, done);
+                                                                                             r0, &S->mr);
             else
                 AEO_PDL_LAUNCH((mg_coarsest_col_kernel<R, COARSE_THREADS>), 1, coarse_col_threads, coarse_col_smem, s, 
-                    C, bc, cfg.coarse_sweeps, r0, &S->mr, done);
+                    C, bc, cfg.coarse_sweeps, r0, &S->mr);
             CKL();
             return AEO_OK;
         }
         mg_coarsest_kernel<R><<<1, COARSE_THREADS, coarse_smem, s>>>(C, coarse_spare, bc, cfg.coarse_sweeps,
-                                                                     coarse_staged, coarse_inplace, r0, &S->mr, done,
-                                                                     nullptr);
+                                                                     coarse_staged, coarse_inplace, r0, &S->mr, nullptr);
         CKL();
         return AEO_OK;
     }
@@ -538,7 +531,7 @@ struct Mg : MgBase {
     // One V-cycle from phi = 0 with level-0 right-hand side r0 - mean
     // (mg_vcycle!, src/Multigrid.jl:706-739); from_zero = false: level 0
     // keeps its phi and b (the standalone cycles).
-    aeo_status launch_vcycle(cudaStream_t s, const double* r0, bool from_zero, const int* done) {
+    aeo_status launch_vcycle(cudaStream_t s, const double* r0, bool from_zero) {
         const double* mr = &S->mr;
         const dim3 blk(RB_X, RB_Y);
         if (nl == 1) {
@@ -546,86 +539,98 @@ struct Mg : MgBase {
                 fail("standalone multigrid cycles need at least two levels");
                 return AEO_ERR_ARGUMENT;
             }
-            return launch_coarsest(s, L[0], r0, done);
+            return launch_coarsest(s, L[0], r0);
         }
         for (int l = 0; l < nl - 1; ++l) {
             Level<R>& F = L[l];
             const dim3 hg = half_grid(F);
             int sw0 = 0;
             if (l > 0 || from_zero) {
-                AEO_PDL_LAUNCH((mg_first_kernel<R>), hg, blk, 0, s, F, bc, l == 0 ? r0 : nullptr, mr, done);
+                const double* rl = l == 0 ? r0 : nullptr;
+                if (F.c.kx) AEO_PDL_LAUNCH((mg_first_kernel<R, CF_CODES>), hg, blk, 0, s, F, bc, rl, mr, early(F));
+                else if (F.c.cx) AEO_PDL_LAUNCH((mg_first_kernel<R, CF_VALUES>), hg, blk, 0, s, F, bc, rl, mr, early(F));
+                else AEO_PDL_LAUNCH((mg_first_kernel<R, CF_CONST>), hg, blk, 0, s, F, bc, rl, mr, early(F));
                 CKL();
-                if (aeo_status q = launch_rbgs(s, F, 1, done)) return q;
+                if (aeo_status q = launch_rbgs(s, F, 1)) return q;
                 sw0 = 1;
             }
             for (int sw = sw0; sw < cfg.nu1; ++sw)
                 for (int c = 0; c < 2; ++c)
-                    if (aeo_status q = launch_rbgs(s, F, c, done)) return q;
+                    if (aeo_status q = launch_rbgs(s, F, c)) return q;
             Level<R>& Cl = L[l + 1];
-            if (aeo_status q = launch_restrict(s, F, Cl, done)) return q;
+            if (aeo_status q = launch_restrict(s, F, Cl)) return q;
         }
-        if (aeo_status q = launch_coarsest(s, L[nl - 1], nullptr, done)) return q;
+        if (aeo_status q = launch_coarsest(s, L[nl - 1], nullptr)) return q;
         for (int l = nl - 2; l >= 0; --l) {
             Level<R>& F = L[l];
-            AEO_PDL_LAUNCH((mg_prolong_kernel<R>), cell_grid(F), blk, 0, s, F, L[l + 1], bc, done);
+            AEO_PDL_LAUNCH((mg_prolong_kernel<R>), cell_grid(F), blk, 0, s, F, L[l + 1], bc, early(F));
             CKL();
             for (int sw = 0; sw < cfg.nu2; ++sw)
                 for (int c = 0; c < 2; ++c)
-                    if (aeo_status q = launch_rbgs(s, F, c, done)) return q;
+                    if (aeo_status q = launch_rbgs(s, F, c)) return q;
         }
         return AEO_OK;
     }
 
-    // one colour pass / the residual of level F in its coefficient form
-    // columns of 8 levels a thread where that still leaves 8 blocks an SM
-    aeo_status launch_rbgs(cudaStream_t s, const Level<R>& F, int colour, const int* done) {
+    // whether a colour pass of F takes columns of 8 levels a thread: where that still
+    // leaves 8 blocks an SM
+    static bool columns(const Level<R>& F) {
+        const size_t bx = (size_t)((F.nx / 2 + RB_X - 1) / RB_X), by = (size_t)((F.ny + RB_Y - 1) / RB_Y);
+        return bx * by * ((F.nz + 7) / 8) >= 8 * 148;
+    }
+    // whether F's kernels let their successor start early (pdl_trigger): the finest
+    // level's are followed by CG kernels, and the marching passes read phi through the
+    // read-only path
+    int early(const Level<R>& F) const { return &F != &L[0] && !columns(F); }
+    // one colour pass of level F in its coefficient form
+    aeo_status launch_rbgs(cudaStream_t s, const Level<R>& F, int colour) {
         const unsigned bx = (unsigned)((F.nx / 2 + RB_X - 1) / RB_X), by = (unsigned)((F.ny + RB_Y - 1) / RB_Y);
-        const bool col = (size_t)bx * by * ((F.nz + 7) / 8) >= 8 * 148;
+        const bool col = columns(F);
         const dim3 hg(bx, by, (unsigned)(col ? (F.nz + 7) / 8 : F.nz)), blk(RB_X, RB_Y);
         if (col) {
-            if (F.c.kx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CODES, 8>), hg, blk, 0, s, F, bc, colour, done);
-            else if (F.c.cx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_VALUES, 8>), hg, blk, 0, s, F, bc, colour, done);
-            else AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CONST, 8>), hg, blk, 0, s, F, bc, colour, done);
+            if (F.c.kx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CODES, 8>), hg, blk, 0, s, F, bc, colour, early(F));
+            else if (F.c.cx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_VALUES, 8>), hg, blk, 0, s, F, bc, colour, early(F));
+            else AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CONST, 8>), hg, blk, 0, s, F, bc, colour, early(F));
         } else {
-            if (F.c.kx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CODES, 1>), hg, blk, 0, s, F, bc, colour, done);
-            else if (F.c.cx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_VALUES, 1>), hg, blk, 0, s, F, bc, colour, done);
-            else AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CONST, 1>), hg, blk, 0, s, F, bc, colour, done);
+            if (F.c.kx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CODES, 1>), hg, blk, 0, s, F, bc, colour, early(F));
+            else if (F.c.cx) AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_VALUES, 1>), hg, blk, 0, s, F, bc, colour, early(F));
+            else AEO_PDL_LAUNCH((mg_rbgs_kernel<R, CF_CONST, 1>), hg, blk, 0, s, F, bc, colour, early(F));
         }
         CKL();
         return AEO_OK;
     }
     // the coarse right-hand side of level F's residual
-    aeo_status launch_restrict(cudaStream_t s, const Level<R>& F, const Level<R>& Cl, const int* done) {
+    aeo_status launch_restrict(cudaStream_t s, const Level<R>& F, const Level<R>& Cl) {
         const dim3 g = restrict_grid(Cl), blk(RB_X, RB_Y);
-        if (F.c.kx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CODES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
-        else if (F.c.cx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_VALUES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
-        else AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CONST>), g, blk, 0, s, F, Cl, bc, part, &S->counter, done);
+        if (F.c.kx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CODES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, early(F));
+        else if (F.c.cx) AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_VALUES>), g, blk, 0, s, F, Cl, bc, part, &S->counter, early(F));
+        else AEO_PDL_LAUNCH((mg_restrict_kernel<R, CF_CONST>), g, blk, 0, s, F, Cl, bc, part, &S->counter, early(F));
         CKL();
         return AEO_OK;
     }
 
     // z: level-0 phi after the cycle, the network's output, or r itself for plain CG
-    aeo_status launch_rz_dir(cudaStream_t s, int first, int pc = -1) {
+    aeo_status launch_rz_dir(cudaStream_t s, int pc = -1) {
         if (pc < 0) pc = cfg.precond;
         if (pc == AEO_PC_LEARNED) {
             const float* zf = aeo_unet_output(net);
-            AEO_PDL_LAUNCH((pcg_rz_kernel<float>), RED_BLOCKS, TPB, 0, s, r, zf, Ap, n, S, part, first);
+            AEO_PDL_LAUNCH((pcg_rz_kernel<float>), RED_BLOCKS, TPB, 0, s, r, zf, Ap, n, S, part);
             CKL();
-            AEO_PDL_LAUNCH((pcg_dir_kernel<float>), RED_BLOCKS, TPB, 0, s, p, zf, n, S, first);
+            AEO_PDL_LAUNCH((pcg_dir_kernel<float>), RED_BLOCKS, TPB, 0, s, p, zf, n, S);
         } else if (pc == AEO_PC_VCYCLE) {
-            AEO_PDL_LAUNCH((pcg_rz_kernel<R>), RED_BLOCKS, TPB, 0, s, r, L[0].phi, Ap, n, S, part, first);
+            AEO_PDL_LAUNCH((pcg_rz_kernel<R>), RED_BLOCKS, TPB, 0, s, r, L[0].phi, Ap, n, S, part);
             CKL();
-            AEO_PDL_LAUNCH((pcg_dir_kernel<R>), RED_BLOCKS, TPB, 0, s, p, L[0].phi, n, S, first);
+            AEO_PDL_LAUNCH((pcg_dir_kernel<R>), RED_BLOCKS, TPB, 0, s, p, L[0].phi, n, S);
         } else if (pc == AEO_PC_JACOBI) {
-            AEO_PDL_LAUNCH((pcg_jacobi_kernel), RED_BLOCKS, TPB, 0, s, zj, r, invd, n, S);
+            AEO_PDL_LAUNCH((pcg_jacobi_kernel), RED_BLOCKS, TPB, 0, s, zj, r, invd, n);
             CKL();
-            AEO_PDL_LAUNCH((pcg_rz_kernel<double>), RED_BLOCKS, TPB, 0, s, r, zj, Ap, n, S, part, first);
+            AEO_PDL_LAUNCH((pcg_rz_kernel<double>), RED_BLOCKS, TPB, 0, s, r, zj, Ap, n, S, part);
             CKL();
-            AEO_PDL_LAUNCH((pcg_dir_kernel<double>), RED_BLOCKS, TPB, 0, s, p, zj, n, S, first);
+            AEO_PDL_LAUNCH((pcg_dir_kernel<double>), RED_BLOCKS, TPB, 0, s, p, zj, n, S);
         } else {
-            AEO_PDL_LAUNCH((pcg_rz_kernel<double>), RED_BLOCKS, TPB, 0, s, r, r, Ap, n, S, part, first);
+            AEO_PDL_LAUNCH((pcg_rz_kernel<double>), RED_BLOCKS, TPB, 0, s, r, r, Ap, n, S, part);
             CKL();
-            AEO_PDL_LAUNCH((pcg_dir_kernel<double>), RED_BLOCKS, TPB, 0, s, p, r, n, S, first);
+            AEO_PDL_LAUNCH((pcg_dir_kernel<double>), RED_BLOCKS, TPB, 0, s, p, r, n, S);
         }
         CKL();
         return AEO_OK;
@@ -719,11 +724,11 @@ struct Mg : MgBase {
                     fail("learned preconditioner: forward pass could not be captured");
                     return q;
                 }
-                return launch_rz_dir(s0, 0, AEO_PC_LEARNED);
+                return launch_rz_dir(s0, AEO_PC_LEARNED);
             },
             [&](cudaStream_t s1) -> aeo_status {
-                if (aeo_status q = launch_vcycle(s1, r, true, &S->done)) return q;
-                return launch_rz_dir(s1, 0, AEO_PC_VCYCLE);
+                if (aeo_status q = launch_vcycle(s1, r, true)) return q;
+                return launch_rz_dir(s1, AEO_PC_VCYCLE);
             });
     }
 
@@ -747,9 +752,13 @@ struct Mg : MgBase {
         return AEO_OK;
     }
 
-    // The solve graph: prologue, WHILE(one CG iteration), the mean shift.
-    // The loop condition is set by pcg_cond_kernel before the loop and at
-    // the end of every iteration.
+    // The solve graph: the start, WHILE(one CG iteration), the mean shift.  An
+    // iteration begins with the preconditioner and ends with the update of x and r,
+    // which sets the loop's condition: nothing is launched after the update that
+    // converged, and no kernel of the cycle asks whether the solve is done.  (With the
+    // update ahead of the preconditioner and a kernel for the condition, every solve
+    // ended in a cycle of empty kernels, and each kernel of the cycle began with a load
+    // that the others waited for.)
     aeo_status build_solve(bool harvest = false) {
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         aeo_status s = capture_solve(st, harvest);
@@ -764,48 +773,35 @@ struct Mg : MgBase {
         if (aeo_status q = make_handle_on(s0, &hdl, 0)) return q;
         pcg_mean_kernel<<<RED_BLOCKS, TPB, 0, s0>>>(b, n, S, part, 0);
         CKL();
-        pcg_init_kernel<<<RED_BLOCKS, TPB, 0, s0>>>(b, r, x, n, S, part);
+        pcg_init_kernel<<<RED_BLOCKS, TPB, 0, s0>>>(b, r, x, n, S, part, hdl);
         CKL();
         if (harvest) {
             pcg_harvest_kernel<<<RED_BLOCKS, TPB, 0, s0>>>(x, r, hist_x, hist_r, n, hist_cap, S);
             CKL();
         }
-        if (cfg.precond == AEO_PC_VCYCLE)
-            if (aeo_status q = launch_vcycle(s0, r, true, &S->done)) return q;
-        if (cfg.precond == AEO_PC_LEARNED)
-            if (aeo_status q = aeo_unet_forward_on(net, r, s0)) return q;
-        if (aeo_status q = launch_rz_dir(s0, 1)) return q;
-        pcg_cond_kernel<<<1, 1, 0, s0>>>(S, hdl, 0);
-        CKL();
-        if (!harvest)
-            prologue_launches = 5 + (cfg.precond == AEO_PC_VCYCLE ? vcycle_launches() : 0) +
-                                (cfg.precond == AEO_PC_JACOBI ? 1 : 0);
+        if (!harvest) prologue_launches = 2;
         if (aeo_status q = capture_cond(s0, hdl, cudaGraphCondTypeWhile, 1, &st_body,
                 [&](cudaStream_t sb) -> aeo_status {
-                    int c0 = 0;
+                    int c0 = 4;   // rz, dir, apply, update
+                    if (cfg.precond == AEO_PC_LEARNED) {
+                        if (aeo_status q2 = launch_learned_pc(sb, &c0)) return q2;
+                    } else {
+                        if (cfg.precond == AEO_PC_VCYCLE) {
+                            if (aeo_status q2 = launch_vcycle(sb, r, true)) return q2;
+                            c0 += vcycle_launches();
+                        }
+                        if (aeo_status q2 = launch_rz_dir(sb)) return q2;
+                        c0 += cfg.precond == AEO_PC_JACOBI ? 1 : 0;
+                    }
                     if (aeo_status q2 = launch_apply(sb, p, Ap, 0)) return q2;
-                    AEO_PDL_LAUNCH((pcg_update_kernel), RED_BLOCKS, TPB, 0, sb, x, r, p, Ap, n, S, part);
+                    AEO_PDL_LAUNCH((pcg_update_kernel), RED_BLOCKS, TPB, 0, sb, x, r, p, Ap, n, S, part, hdl);
                     CKL();
-                    c0 += 2;
                     if (harvest) {
                         pcg_harvest_kernel<<<RED_BLOCKS, TPB, 0, sb>>>(x, r, hist_x, hist_r, n, hist_cap, S);
                         CKL();
                         c0 += 1;
                     }
-                    if (cfg.precond == AEO_PC_LEARNED) {
-                        if (aeo_status q2 = launch_learned_pc(sb, &c0)) return q2;
-                        c0 += 2;
-                    } else {
-                        if (cfg.precond == AEO_PC_VCYCLE) {
-                            if (aeo_status q2 = launch_vcycle(sb, r, true, &S->done)) return q2;
-                            c0 += vcycle_launches();
-                        }
-                        if (aeo_status q2 = launch_rz_dir(sb, 0)) return q2;
-                        c0 += cfg.precond == AEO_PC_JACOBI ? 3 : 2;
-                    }
-                    pcg_cond_kernel<<<1, 1, 0, sb>>>(S, hdl, 0);
-                    CKL();
-                    body_launches = c0 + 1;
+                    body_launches = c0;
                     return AEO_OK;
                 },
                 [](cudaStream_t) -> aeo_status { return AEO_OK; }))
@@ -898,13 +894,13 @@ struct Mg : MgBase {
             CKL();
             mg_bnorm_kernel<R><<<RED_BLOCKS, TPB, 0, st>>>(L[0], S, part);
             CKL();
-            pcg_cond_kernel<<<1, 1, 0, st>>>(S, hdl, 1);
+            mg_cond_kernel<<<1, 1, 0, st>>>(S, hdl);
             CKL();
             if (aeo_status q = capture_while(hdl, [&](cudaStream_t sb) -> aeo_status {
-                    if (aeo_status q2 = launch_vcycle(sb, nullptr, false, &S->done)) return q2;
+                    if (aeo_status q2 = launch_vcycle(sb, nullptr, false)) return q2;
                     mg_resnorm_kernel<R><<<row_blocks(cfg.ny * cfg.nz), dim3(RB_X, RB_Y), 0, sb>>>(L[0], bc, S, part);
                     CKL();
-                    pcg_cond_kernel<<<1, 1, 0, sb>>>(S, hdl, 1);
+                    mg_cond_kernel<<<1, 1, 0, sb>>>(S, hdl);
                     CKL();
                     return AEO_OK;
                 }))
@@ -955,9 +951,9 @@ struct Mg : MgBase {
             CK(cudaMemcpyAsync(b, rin, sizeof(double) * n, cudaMemcpyHostToDevice, st));
             pcg_mean_kernel<<<RED_BLOCKS, TPB, 0, st>>>(b, n, S, part, 0);
             CKL();
-            pcg_init_kernel<<<RED_BLOCKS, TPB, 0, st>>>(b, r, x, n, S, part);
+            pcg_init_kernel<<<RED_BLOCKS, TPB, 0, st>>>(b, r, x, n, S, part, 0);
             CKL();
-            if (aeo_status s = launch_vcycle(st, r, true, dzero)) return s;
+            if (aeo_status s = launch_vcycle(st, r, true)) return s;
             std::vector<R> hz((size_t)n);
             CK(cudaMemcpyAsync(hz.data(), L[0].phi, sizeof(R) * n, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
@@ -1036,19 +1032,19 @@ struct Mg : MgBase {
             case 1: {
                 Level<R>& F = L[0];
                 if (F.nx % 2) { fail("profile: odd finest nx"); return AEO_ERR_ARGUMENT; }
-                return launch_rbgs(st, F, 0, dzero);
+                return launch_rbgs(st, F, 0);
             }
             case 2: return launch_apply(st, p, Ap, 1);
-            case 3: return launch_vcycle(st, r, true, dzero);
-            case 4: return launch_coarsest(st, L[nl - 1], nl == 1 ? r : nullptr, dzero);
+            case 3: return launch_vcycle(st, r, true);
+            case 4: return launch_coarsest(st, L[nl - 1], nl == 1 ? r : nullptr);
             case 5: {
                 if (nl < 2) { fail("profile: one level, no restriction"); return AEO_ERR_ARGUMENT; }
-                return launch_restrict(st, L[0], L[1], dzero);
+                return launch_restrict(st, L[0], L[1]);
             }
             case 6: {
                 if (nl < 2) { fail("profile: one level, no smoothing sweep"); return AEO_ERR_ARGUMENT; }
-                if (aeo_status q = launch_rbgs(st, L[0], 0, dzero)) return q;
-                return launch_rbgs(st, L[0], 1, dzero);
+                if (aeo_status q = launch_rbgs(st, L[0], 0)) return q;
+                return launch_rbgs(st, L[0], 1);
             }
             default: fail("profile: unknown part"); return AEO_ERR_ARGUMENT;
             }

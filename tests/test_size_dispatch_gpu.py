@@ -246,3 +246,57 @@ def test_centred_steps_of_every_column_form(size, core, stretched, c_s):
         assert rel(s64.get_field(n)[g.interior], want) <= 1e-11, n
         assert rel(s32.get_field(n)[g.interior], want) <= 1e-5, n
 
+
+
+# ---- the multigrid cycle and the CG loop -----------------------------------------------------------------------
+def cut_coeffs(n, seed):
+    nx, ny, nz = n
+    rng = np.random.default_rng(seed)
+    c = [rng.choice([0.0, 0.3, 0.7, 1.0], s, p=[0.1, 0.1, 0.1, 0.7]) for s in ((nz, ny, nx + 1), (nz, ny + 1, nx), (nz + 1, ny, nx))]
+    c[0][:, :, -1], c[1][:, -1] = c[0][:, :, 0], c[1][:, 0]
+    c[2][0] = c[2][-1] = 0.0
+    return c
+
+
+@pytest.mark.parametrize("n", [(4, 4, 4), (32, 16, 8), (66, 6, 4), (64, 8, 12), (120, 88, 40), (256, 128, 64)])
+@pytest.mark.parametrize("form", ["constant", "codes", "values"])
+def test_cycle_over_every_level_size(n, form):
+    """One cycle against the oracle's: levels of one pass per plane and of marching columns, coefficient forms."""
+    from aeolus_b200.multigrid import MGPreconditionedCG
+    from oracle.mgpcg import OracleMGPCG
+    c = None if form == "constant" else cut_coeffs(n, sum(n))
+    if form == "values":
+        c = [a * (1 + 0.1 * np.sin(np.arange(a.size).reshape(a.shape))) for a in c]
+        c[0][:, :, -1], c[1][:, -1] = c[0][:, :, 0], c[1][:, 0]
+    b = np.random.default_rng(3).standard_normal(n[::-1])
+    h = (1.0, 1.3, 0.7)
+    want = OracleMGPCG(n, h, coeffs=c).precondition(b)
+    assert rel(MGPreconditionedCG(n, h, coeffs=c).precondition(b), want) <= 1e-11
+    assert rel(MGPreconditionedCG(n, h, coeffs=c, precision="fp32_mixed").precondition(b), want) <= 1e-4
+
+
+@pytest.mark.parametrize("precond", ["vcycle", "jacobi", "identity"])
+@pytest.mark.parametrize("n", [(16, 8, 8), (40, 24, 12), (9, 7, 5)])
+def test_cg_loop_counts_and_ends(n, precond):
+    """The loop ends after the update that converged or at maxit, with the oracle's count, the residual it reports
+    and the same iterates as the harvesting graph; a zero right-hand side and a huge tolerance end it before."""
+    from aeolus_b200.multigrid import MGPreconditionedCG
+    c = cut_coeffs(n, 11) if n[0] != 9 else None
+    b = MGPreconditionedCG(n, (1.0,) * 3, coeffs=c).apply(np.random.default_rng(4).standard_normal(n[::-1]))
+    make = lambda **k: MGPreconditionedCG(n, (1.0,) * 3, coeffs=c, precond=precond, **k)
+    for maxit in (1, 2, 5):
+        s = make(tol=1e-30, maxit=maxit)
+        x, st = s.solve(b)
+        assert st["iterations"] == maxit and st["status"] == "maxit", st
+        y, sh, pairs = s.solve_harvest(b, cap=8)
+        assert np.array_equal(x, y) and sh["iterations"] == maxit and len(pairs) == maxit + 1
+        r = b - b.mean() - s.apply(x)
+        assert abs(np.linalg.norm(r) - st["residual"]) <= 1e-10 * st["bnorm"]
+    s = make(tol=1e-6, maxit=400)
+    for _ in range(2):
+        x, st = s.solve(b)
+        assert st["status"] == "converged" and st["residual"] <= 1e-6 * st["bnorm"]
+    x, st = s.solve(np.zeros_like(b))
+    assert st["status"] == "zero_rhs" and st["iterations"] == 0 and not x.any()
+    x, st = make(tol=2.0, maxit=5).solve(b)
+    assert st["status"] == "converged" and st["iterations"] == 0 and not x.any()
