@@ -15,6 +15,7 @@
 // pooling; nearest upsampling.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -228,10 +229,11 @@ struct aeo_unet {
                                 (int)un::RingShape<32, 32, 1>::smem));
         CK(cudaFuncSetAttribute(un::conv_ring_kernel<32, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)un::RingShape<32, 16, 1>::smem));
-        CK(cudaFuncSetAttribute(un::conv_wgrad_ring_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)un::WgShape<16>::smem));
-        CK(cudaFuncSetAttribute(un::conv_wgrad_ring_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)un::WgShape<32>::smem));
+        auto wg_attr = [](auto* k, size_t sm) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); };
+        CK(wg_attr(un::conv_wgrad_ring_kernel<16, 16>, un::WgShape<16, 16>::smem));
+        CK(wg_attr(un::conv_wgrad_ring_kernel<16, 32>, un::WgShape<16, 32>::smem));
+        CK(wg_attr(un::conv_wgrad_ring_kernel<32, 32>, un::WgShape<32, 32>::smem));
+        CK(wg_attr(un::conv_wgrad_ring_kernel<32, 16>, un::WgShape<32, 16>::smem));
         CK(cudaFuncSetAttribute(un::conv_wgrad_kernel<16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w1616));
         CK(cudaFuncSetAttribute(un::conv_wgrad_kernel<16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w1632));
         CK(cudaFuncSetAttribute(un::conv_wgrad_kernel<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w3232));
@@ -312,6 +314,13 @@ struct aeo_unet {
         return AEO_OK;
     }
 
+    template <int CIN, int COUT>
+    void wgrad_ring(const Tiles& Tl, const un::WgradArgs& a) {
+        using W = un::WgShape<CIN, COUT>;
+        const int g = std::min(Tl.ntiles, sms * W::CTAS);
+        un::conv_wgrad_ring_kernel<CIN, COUT><<<g, un::RING_THREADS, W::smem, st>>>(a);
+    }
+
     aeo_status wgrad(int l, const bf16* xin, const bf16* g) {
         const int ci = LAYERS[l].cin, co = LAYERS[l].cout;
         const Tiles& Tl = T[LAYERS[l].level];
@@ -322,10 +331,11 @@ struct aeo_unet {
         a.dW = dW(l);
         a.db = db(l);
         a.err = derr;
-        if (ci == 16 && Tl.mode == 0 && Tl.ny >= 3) {   // x-segment tiles: the pipelined ring kernel, one CTA an SM
-            const int g1 = Tl.ntiles < sms ? Tl.ntiles : sms;
-            if (co == 16) un::conv_wgrad_ring_kernel<16><<<g1, un::RING_THREADS, un::WgShape<16>::smem, st>>>(a);
-            else un::conv_wgrad_ring_kernel<32><<<g1, un::RING_THREADS, un::WgShape<32>::smem, st>>>(a);
+        if (Tl.mode == 0 && Tl.ny >= 3) {   // x-segment tiles: the pipelined ring kernel
+            if (ci == 16 && co == 16) wgrad_ring<16, 16>(Tl, a);
+            else if (ci == 16 && co == 32) wgrad_ring<16, 32>(Tl, a);
+            else if (ci == 32 && co == 32) wgrad_ring<32, 32>(Tl, a);
+            else wgrad_ring<32, 16>(Tl, a);
             CKL();
             return AEO_OK;
         }

@@ -699,32 +699,44 @@ __global__ void __launch_bounds__(CONV_THREADS) conv_wgrad_kernel(WgradArgs a) {
     if (warp == 0) tc::tmem_dealloc(tmem, NCOL);
 }
 
-// The weight gradient on x-segment tiles as a pipeline (CIN = 16): the input
-// rows in the forward kernel's ring (PF = 1, R = 6 entries), the tile's
-// output-gradient rows beside it (two buffers), and the (tap, channel) rows of
-// each M-tile materialised into one of two shared buffers by warps 0-3 while
-// warp 4 multiplies the other: the 8 MMAs (K = 128 cells) of M-tile q run
-// while the rows of M-tile q+1 are gathered.  Named barriers 1, 2 "M buffer
-// ready" (arrived at by warps 0-3, waited on by warp 4, by the parity of q),
-// 5 the loader warps among themselves; the M buffers come back through the
-// MMA commits (mbarriers).  Accumulated in TMEM over the CTA's tiles, added
-// to dW at the end.
-template <int COUT>
+// The weight gradient on x-segment tiles as a pipeline with no gather.  The input
+// rows lie in a ring of y-row entries as in the forward kernel, an entry's planes
+// in the order (channel chunk, dz), so that the three entries of a tile are
+// 9 CIN/8 planes at one stride -- and an MN-major operand is just that: 16 planes
+// of 8 channels at a uniform stride are an M-tile of 128 (tap, channel) rows, its
+// K the tile's cells from any starting row, so the tap's dx is an offset of the
+// start address.  For each dx the first 16 floor(planes / 16) planes go in whole
+// M-tiles; a plane left over is an M-tile of its own whose "planes" are 16 bytes
+// apart (the first three are its dx = -1, 0, +1, the rest is never read back).
+// The ring's first two slots are kept twice (behind its end), so that three
+// consecutive entries never wrap.  Warp 4 issues a tile's MMAs (8 K-steps an
+// M-tile) straight from the ring while warps 0-3 load the next tile and sum the
+// bias gradient; accumulated in TMEM over the CTA's tiles, added to dW at the end.
+// Gathering every M-tile's rows into a shared buffer first (16 KB written and
+// read again for 8 MMAs) took 1.82 ms a full-resolution 16 -> 16 layer of
+// 256 x 256 x 96, this 0.36 ms; the MMAs themselves, bound by their A operand's
+// 4 KB each, 0.22 ms.
+template <int CIN, int COUT>
 struct WgShape {
-    static constexpr int CIN = 16, NCH = 2, NCO = COUT / 8, PF = 1;
-    static constexpr int NMT = wg_mtiles<16>();
-    static constexpr size_t ring_rows = (size_t)RingShape<16, COUT, 1>::R * RingShape<16, COUT, 1>::slot_rows;
+    static constexpr int NCH = CIN / 8, NCO = COUT / 8, PF = 1;
+    static constexpr int R = RingShape<CIN, COUT, PF>::R, PITCH = TM + 2;
+    static constexpr int EPL = 3 * NCH;                          // planes of an entry
+    static constexpr int NPL = 3 * EPL, FULL = NPL / 16, TAIL = NPL % 16;
+    static constexpr int NMT = 3 * FULL + TAIL;
+    static constexpr size_t entry_rows = (size_t)EPL * PITCH;    // 16-byte rows
+    static constexpr size_t ring_rows = (size_t)(R + 2) * entry_rows + 16;   // + what a left-over plane's M-tile reads past the end
     static constexpr size_t g_rows = (size_t)NCO * TM;           // one tile's gradient rows
-    static constexpr size_t m_rows = (size_t)16 * TM;            // one M buffer
-    static constexpr size_t smem = (ring_rows + 2 * g_rows + 2 * m_rows) * 16;
-    static constexpr uint32_t tmem_cols = wg_tmem_cols<16, COUT>();
+    static constexpr size_t smem = (ring_rows + 2 * g_rows) * 16;
+    static constexpr uint32_t cols = (uint32_t)(NMT * COUT);
+    static constexpr uint32_t tmem_cols = cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512));
+    static constexpr int CTAS = smem <= 113 * 1024 ? 2 : 1;      // an SM (TMEM: at most 2 x 256 columns)
+    static_assert(cols <= 512 && (CTAS == 1 || tmem_cols <= 256), "TMEM columns");
 };
 
-template <int COUT>
+template <int CIN, int COUT>
 __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs a) {
-    using W = WgShape<COUT>;
-    using RS = RingShape<16, COUT, 1>;
-    constexpr int NCH = W::NCH, NCO = W::NCO, NMT = W::NMT, R = RS::R, PITCH = RS::PITCH;
+    using W = WgShape<CIN, COUT>;
+    constexpr int NCH = W::NCH, NCO = W::NCO, NMT = W::NMT, R = W::R, PITCH = W::PITCH, EPL = W::EPL, PF = W::PF;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t mbM[2], rdy[2];
     __shared__ uint32_t tslot;
@@ -732,7 +744,6 @@ __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs
     const Tiles& T = a.T;
     uint4* sR = reinterpret_cast<uint4*>(smem);
     uint4* sG = sR + W::ring_rows;                 // 2 x NCO planes x 128 rows
-    uint4* sM = sG + 2 * W::g_rows;                // 2 x 16 planes x 128 rows
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = (int)((long long)T.ntiles * blockIdx.x / gridDim.x);
     const int cnt = (int)((long long)T.ntiles * (blockIdx.x + 1) / gridDim.x) - t0;
@@ -748,36 +759,45 @@ __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = tslot;
-    const int nq = cnt * NMT;
     bool failed = false;
 
     if (warp == 4) {
-        // ---- the MMA warp: M-tile q of tile i = q / NMT into TMEM columns (q % NMT) * COUT
+        // ---- the MMA warp: M-tile mt of every tile into TMEM columns mt * COUT
         const uint32_t idesc = tc::idesc_bf16(COUT, true, true);
+        const uint64_t planes = tc::sdesc(tc::smem_u32(sR), 128u, (uint32_t)PITCH * 16u);   // M chunks a plane apart
+        const uint64_t shifts = tc::sdesc(tc::smem_u32(sR), 128u, 16u);                     // ... a row apart
+        const uint64_t grad = tc::sdesc(tc::smem_u32(sG), 128u, (uint32_t)TM * 16u);
+        int qm = -1;
 #pragma unroll 1
-        for (int q = 0; q < nq; ++q) {
-            const int i = q / NMT, mt = q - i * NMT;
-            if (!tc::mbar_wait(&rdy[q & 1], (uint32_t)((q >> 1) & 1), WAIT_LIMIT)) {
+        for (int i = 0; i < cnt; ++i) {
+            const int tau = t0 + i;
+            qm += (i == 0 || tau % T.ny == 0) ? 3 : 1;
+            if (!tc::mbar_wait(&rdy[i & 1], (uint32_t)((i >> 1) & 1), WAIT_LIMIT)) {
                 if (lane == 0) mma_failed = 1;
                 __syncwarp();
                 continue;
             }
             tc::fence_after();
             if (lane == 0) {
-                const uint32_t mBase = tc::smem_u32(sM + (size_t)(q & 1) * W::m_rows);
-                const uint32_t gBase = tc::smem_u32(sG + (size_t)(i & 1) * W::g_rows);
+                const uint32_t row0 = (uint32_t)((qm - 2) % R) * (uint32_t)W::entry_rows;
+                const uint64_t gd = grad + (uint64_t)((i & 1) * (uint32_t)W::g_rows);
 #pragma unroll
-                for (int kk = 0; kk < TM / 16; ++kk) {
-                    const uint64_t ad = tc::sdesc(mBase + kk * 256u, 128u, (uint32_t)TM * 16u);
-                    const uint64_t bd = tc::sdesc(gBase + kk * 256u, 128u, (uint32_t)TM * 16u);
-                    tc::mma_bf16(tmem + (uint32_t)(mt * COUT), ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                for (int mt = 0; mt < NMT; ++mt) {
+                    const bool whole = mt < 3 * W::FULL;
+                    const int dx = whole ? mt / (W::FULL > 0 ? W::FULL : 1) : 0;
+                    const int pl = whole ? 16 * (mt - dx * W::FULL) : 16 * W::FULL + (mt - 3 * W::FULL);
+                    const uint64_t ad = (whole ? planes : shifts) + (uint64_t)(row0 + (uint32_t)(pl * PITCH + dx));
+#pragma unroll
+                    for (int kk = 0; kk < TM / 16; ++kk)
+                        tc::mma_bf16(tmem + (uint32_t)(mt * COUT), ad + (uint64_t)(kk * 16), gd + (uint64_t)(kk * 16), idesc,
+                                     (i > 0 || kk > 0) ? 1u : 0u);
                 }
-                tc::commit(&mbM[q & 1]);
+                tc::commit(&mbM[i & 1]);
             }
             __syncwarp();
         }
     } else {
-        // ---- warps 0-3: loads, gradient sums, the M rows
+        // ---- warps 0-3: loads and the bias gradient's sums
         const int tid = threadIdx.x;
         const uint4* inp = reinterpret_cast<const uint4*>(a.x);
         const uint4* gp = reinterpret_cast<const uint4*>(a.g);
@@ -792,7 +812,7 @@ __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs
                 jj = jj < 0 ? jj + T.ny : (jj >= T.ny ? jj - T.ny : jj);
                 ++ql;
                 const int slot = ql % R;
-                constexpr int TOTAL = 3 * NCH * PITCH;
+                constexpr int TOTAL = EPL * PITCH;
                 for (int idx = tid; idx < TOTAL; idx += 128) {
                     const int c = idx % NCH, rest = idx / NCH;
                     const int x = rest % PITCH, d = rest / PITCH;
@@ -801,7 +821,9 @@ __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs
                     int gx = x0 - 1 + x;
                     gx = gx < 0 ? gx + T.nx : (gx >= T.nx ? gx - T.nx : gx);
                     const uint4* src = inp + ((size_t)((zin ? gz : 0) * T.ny + jj) * T.nx + gx) * NCH + c;
-                    cp_async16(sR + ((size_t)((c * R + slot) * 3 + d)) * PITCH + x, src, zin);
+                    uint4* dst = sR + (size_t)slot * W::entry_rows + (size_t)(c * 3 + d) * PITCH + x;
+                    cp_async16(dst, src, zin);
+                    if (slot < 2) cp_async16(dst + (size_t)R * W::entry_rows, src, zin);   // the copy behind the ring's end
                 }
             }
             // the tile's gradient rows, N chunk c of cell m at sG[c * 128 + m]
@@ -815,76 +837,47 @@ __global__ void __launch_bounds__(RING_THREADS) conv_wgrad_ring_kernel(WgradArgs
         if (cnt > 0) load_tile(0);
         cp_async_commit();
         float dbacc = 0.0f;
-        int qm = -1;
+        const int co = tid % COUT, m0 = tid / COUT;      // this thread's output channel and first cell
 #pragma unroll 1
         for (int i = 0; i < cnt; ++i) {
-            const int tau = t0 + i;
-            qm += (i == 0 || tau % T.ny == 0) ? 3 : 1;
             cp_async_wait<0>();                        // tile i's rows and gradient landed
-            nb_sync_n(5, 128);                         // every loader's copies, before anyone reads them
-            if (tid < COUT) {
-                const int c = tid / 8, e = tid % 8;
-                const bf16* g8 = reinterpret_cast<const bf16*>(sG + (size_t)(i & 1) * W::g_rows + (size_t)c * TM);
-                for (int m = 0; m < TM; ++m) dbacc += __bfloat162float(g8[m * 8 + e]);
+            tc::fence_async_smem();
+            tc::mbar_arrive(&rdy[i & 1]);
+            nb_sync_n(5, 128);                         // every loader's copies, before anyone sums them
+            {
+                const bf16* g8 = reinterpret_cast<const bf16*>(sG + (size_t)(i & 1) * W::g_rows + (size_t)(co / 8) * TM) + co % 8;
+#pragma unroll
+                for (int m = 0; m < TM / (128 / COUT); ++m) dbacc += __bfloat162float(g8[(m0 + m * (128 / COUT)) * 8]);
             }
-#pragma unroll 1
-            for (int mt = 0; mt < NMT; ++mt) {
-                const int q = i * NMT + mt, b = q & 1;
-                if (q >= 2)                            // the MMAs of M-tile q-2 read this buffer
-                    if (!tc::mbar_wait(&mbM[b], (uint32_t)(((q - 2) >> 1) & 1), WAIT_LIMIT)) failed = true;
-                // warp w gathers M chunks 4w .. 4w+3 (one (tap, channel-chunk) row each),
-                // its lanes along the cells
-                uint4* dM = sM + (size_t)b * W::m_rows;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int gl = warp * 4 + u, G = mt * 16 + gl;
-                    uint4* dst = dM + (size_t)gl * TM;
-                    if (G < 27 * NCH) {
-                        const int t = G / NCH, c = G - t * NCH;
-                        const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-                        const uint4* src = sR + ((size_t)((c * R + (qm - 2 + dy) % R) * 3 + dz)) * PITCH + dx;
-#pragma unroll
-                        for (int m = lane; m < TM; m += 32) dst[m] = src[m];
-                    } else {
-#pragma unroll
-                        for (int m = lane; m < TM; m += 32) dst[m] = make_uint4(0u, 0u, 0u, 0u);
-                    }
-                }
-                tc::fence_async_smem();
-                tc::mbar_arrive(&rdy[b]);              // M-tile q ready
-            }
-            // every loader is done with tile i-1's ring slots and (its MMAs having
-            // completed, M-tile i*NMT-1 was waited for above) its gradient rows
-            nb_sync_n(5, 128);
-            if (i + 1 < cnt) load_tile(i + 1);
+            // tile i-1's MMAs done: its ring slots and gradient buffer are free
+            if (i > 0 && !failed)
+                if (!tc::mbar_wait(&mbM[(i - 1) & 1], (uint32_t)(((i - 1) >> 1) & 1), WAIT_LIMIT)) failed = true;
+            if (i + PF < cnt && !failed) load_tile(i + PF);
             cp_async_commit();
         }
         cp_async_wait<0>();
-        // the last two M-tiles' MMAs (the accumulators complete), bounded
-        for (int q = nq - 2 < 0 ? 0 : nq - 2; q < nq; ++q)
-            if (!tc::mbar_wait(&mbM[q & 1], (uint32_t)((q >> 1) & 1), WAIT_LIMIT)) failed = true;
-        if (tid < COUT && cnt > 0) atomicAdd(&a.db[tid], dbacc);
+        // the last tile's MMAs (the accumulators complete), bounded
+        if (cnt > 0 && !tc::mbar_wait(&mbM[(cnt - 1) & 1], (uint32_t)(((cnt - 1) >> 1) & 1), WAIT_LIMIT)) failed = true;
+        if (cnt > 0) atomicAdd(&a.db[co], dbacc);
         if (failed) {
-            if (tid == 0) atomicExch(a.err, 1);
+            if (lane == 0) atomicExch(a.err, 1);
         } else if (cnt > 0) {
             tc::fence_after();
-            const int m = warp * 32 + lane;
+            const int m = warp * 32 + lane, gl = m / 8;
+#pragma unroll 1
             for (int mt = 0; mt < NMT; ++mt) {
-                float v[COUT];
-                float h[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * COUT), h);
+                const bool whole = mt < 3 * W::FULL;
+                const int dx = whole ? mt / (W::FULL > 0 ? W::FULL : 1) : gl;
+                const int pl = whole ? 16 * (mt - dx * W::FULL) + gl : 16 * W::FULL + (mt - 3 * W::FULL);
+                const int dy = pl / EPL, c = (pl - dy * EPL) / 3, dz = pl % 3;
+                const int t = dz * 9 + dy * 3 + dx, ci = c * 8 + m % 8;
 #pragma unroll
-                for (int r = 0; r < 16; ++r) v[r] = h[r];
-                if constexpr (COUT == 32) {
-                    tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * COUT + 16), h);
+                for (int h0 = 0; h0 < COUT; h0 += 16) {
+                    float h[16];
+                    tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * COUT + h0), h);
+                    if (dx < 3)
 #pragma unroll
-                    for (int r = 0; r < 16; ++r) v[16 + r] = h[r];
-                }
-                const int G = mt * 16 + m / 8;
-                if (G < 27 * NCH) {
-                    const int t = G / NCH, ci = (G % NCH) * 8 + m % 8;
-#pragma unroll
-                    for (int co = 0; co < COUT; ++co) atomicAdd(&a.dW[((size_t)t * COUT + co) * 16 + ci], v[co]);
+                        for (int r = 0; r < 16; ++r) atomicAdd(&a.dW[((size_t)t * COUT + h0 + r) * CIN + ci], h[r]);
                 }
             }
         }

@@ -300,3 +300,11 @@ def test_cg_loop_counts_and_ends(n, precond):
     assert st["status"] == "zero_rhs" and st["iterations"] == 0 and not x.any()
     x, st = make(tol=2.0, maxit=5).solve(b)
     assert st["status"] == "converged" and st["iterations"] == 0 and not x.any()
+
+
+# ---- the U-Net: weight gradients of x-segment tiles at every channel count, host arrays through pinned lanes ----
+@pytest.mark.parametrize("shape", [(512, 24, 8), (256, 16, 12), (512, 8, 16)])
+def test_unet_gradients_where_every_level_takes_x_segments(shape):
+    import test_unet_gpu
+    test_unet_gpu.test_gradients_match_the_oracle(shape)
+
