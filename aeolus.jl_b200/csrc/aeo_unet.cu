@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/aeolus_b200_unet.h"
+#include "aeo_hostcopy.h"
 #include "aeo_unet_kernels.cuh"
 
 namespace {
@@ -113,6 +114,9 @@ struct aeo_unet {
     double* rbuf = nullptr;             // device residual / target for host-array calls
     double* ebuf = nullptr;
     int* derr = nullptr;
+    std::shared_ptr<HostStage> stage;   // the pageable host arrays' way to the device
+    cudaStream_t st_up = nullptr;       // the target's upload, beside the forward pass
+    cudaEvent_t ev_free = nullptr, ev_up = nullptr;
 
     template <typename T_>
     aeo_status dalloc(T_** p, size_t count) {
@@ -125,12 +129,22 @@ struct aeo_unet {
 
     ~aeo_unet() {
         if (st) cudaStreamSynchronize(st);
+        if (st_up) cudaStreamSynchronize(st_up);
         for (void* a : allocs) cudaFree(a);
+        if (ev_free) cudaEventDestroy(ev_free);
+        if (ev_up) cudaEventDestroy(ev_up);
+        if (st_up) cudaStreamDestroy(st_up);
         if (st) cudaStreamDestroy(st);
     }
 
     aeo_status init(uint64_t seed) {
         CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        CK(cudaStreamCreateWithFlags(&st_up, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&ev_free, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ev_up, cudaEventDisableTiming));
+        cudaError_t se = cudaSuccess;
+        stage = HostStage::get(&se);
+        CK(se);
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         for (int l = 0; l < 3; ++l) {
             const int f = 1 << l;
@@ -533,12 +547,13 @@ aeo_status aeo_unet_apply(aeo_unet* h, const double* r, double* z) {
     UN_ENTER(h);
     if (!r || !z) { h->err = "r and z must not be NULL"; return AEO_ERR_ARGUMENT; }
     std::string& err = h->err;
-    CK(cudaMemcpyAsync(h->rbuf, r, sizeof(double) * h->n[0], cudaMemcpyHostToDevice, h->st));
+    const size_t bytes = sizeof(double) * (size_t)h->n[0];
+    CK(h->stage->upload(h->rbuf, r, bytes, h->device, h->st));
     if (aeo_status s = h->forward_(h->rbuf)) return s;
-    std::vector<float> zf((size_t)h->n[0]);
-    CK(cudaMemcpyAsync(zf.data(), h->z, sizeof(float) * h->n[0], cudaMemcpyDeviceToHost, h->st));
+    un::widen_kernel<<<grid_for(h->n[0]), 256, 0, h->st>>>(h->z, h->ebuf, h->n[0]);
+    CKL();
     if (aeo_status s = h->check_err()) return s;
-    for (long long q = 0; q < h->n[0]; ++q) z[q] = zf[q];
+    CK(h->stage->download(z, h->ebuf, bytes, h->device, h->st));
     return AEO_OK;
 }
 
@@ -547,9 +562,15 @@ aeo_status aeo_unet_gradients(aeo_unet* h, const double* r, const double* e, dou
     if (!r || !e) { h->err = "r and e must not be NULL"; return AEO_ERR_ARGUMENT; }
     std::string& err = h->err;
     CK(cudaMemsetAsync(h->G, 0, sizeof(float) * h->off[NLAYERS], h->st));
-    CK(cudaMemcpyAsync(h->rbuf, r, sizeof(double) * h->n[0], cudaMemcpyHostToDevice, h->st));
-    CK(cudaMemcpyAsync(h->ebuf, e, sizeof(double) * h->n[0], cudaMemcpyHostToDevice, h->st));
+    const size_t bytes = sizeof(double) * (size_t)h->n[0];
+    // the target goes up beside the forward pass, which does not read it
+    CK(cudaEventRecord(h->ev_free, h->st));
+    CK(cudaStreamWaitEvent(h->st_up, h->ev_free, 0));
+    CK(h->stage->upload(h->rbuf, r, bytes, h->device, h->st));
     if (aeo_status s = h->forward_(h->rbuf)) return s;
+    CK(h->stage->upload(h->ebuf, e, bytes, h->device, h->st_up));
+    CK(cudaEventRecord(h->ev_up, h->st_up));
+    CK(cudaStreamWaitEvent(h->st, h->ev_up, 0));
     if (aeo_status s = h->backward(h->ebuf)) return s;
     double hl[5];
     CK(cudaMemcpyAsync(hl, h->acc + 4, sizeof(hl), cudaMemcpyDeviceToHost, h->st));

@@ -1072,6 +1072,11 @@ __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ g, float*
     }
 }
 
+// the output field as the host array takes it
+__global__ void widen_kernel(const float* __restrict__ a, double* __restrict__ b, long long n) {
+    GS(q, n) b[q] = (double)a[q];
+}
+
 // s = sqrt(n_fluid) / |r|, from a reduction of r^2 over fluid cells
 __global__ void rscale_kernel(const double* __restrict__ r, const float* __restrict__ mask, double* acc, long long n) {
     double s = 0.0, c = 0.0;

@@ -308,3 +308,37 @@ def test_unet_gradients_where_every_level_takes_x_segments(shape):
     import test_unet_gpu
     test_unet_gpu.test_gradients_match_the_oracle(shape)
 
+
+
+@pytest.mark.parametrize("shape", [(128, 16, 8), (128, 64, 32), (128, 48, 44), (256, 64, 56)])
+def test_host_arrays_pageable_pinned_and_from_threads(shape):
+    """Below and above the size that takes the pinned lanes, whole and ragged chunks: the same bits as from pinned
+    arrays, and from several handles at once."""
+    import threading
+    import torch
+    from aeolus_b200.unet import UNet
+    rng = np.random.default_rng(1)
+    n = shape[::-1]
+    mask = (rng.random(n) > 0.1).astype(np.float32)
+    rs = [rng.standard_normal(n) * mask for _ in range(3)]
+    e = rng.standard_normal(n) * mask
+    nets = [UNet(shape, seed=5) for _ in range(3)]
+    want = []
+    for net, r in zip(nets, rs):
+        net.set_mask(mask)
+        pin = torch.from_numpy(r).pin_memory().numpy()
+        want.append(np.array(net.apply(pin)))
+    loss = nets[0].gradients(torch.from_numpy(rs[0]).pin_memory().numpy(), torch.from_numpy(e).pin_memory().numpy())
+    assert abs(nets[0].gradients(rs[0], e) - loss) <= 1e-12 * abs(loss)
+    got = [None] * 3
+
+    def work(q):
+        for _ in range(3):
+            got[q] = np.array(nets[q].apply(rs[q]))
+
+    th = [threading.Thread(target=work, args=(q,)) for q in range(3)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
