@@ -36,7 +36,6 @@
 #include "aeo_mg_internal.h"
 #include "aeo_common.cuh"
 #include "aeo_cutcell.cuh"
-#include "aeo_positive.cuh"
 #include "aeo_fft.cuh"
 #include "aeo_init.cuh"
 #include "aeo_misc.cuh"
@@ -44,6 +43,7 @@
 #include "aeo_tke.cuh"
 #include "aeo_sweep_pair.cuh"
 #include "aeo_sweep_wpair.cuh"
+#include "aeo_positive.cuh"
 
 // reg(length) with the compile-time length 2^5 .. 2^9 of a register transform,
 // or smem() for the shared-memory form of the other lengths.
@@ -346,6 +346,19 @@ struct Core : CoreBase {
         g.tke_cl = c_l;
         return AEO_OK;
     }
+    // the limited tendency of a[3] in the flow a[0 .. 2]: chunks of levels such that the tiles
+    // fill the SMs several times over, at least eight levels each (a chunk computes one z
+    // face more than it has levels)
+    template <int SCH>
+    void launch_positive(const PosGeo& pg, const R* const* a, const double* dtp, R* tend, int accumulate) {
+        using T = PosTile<R>;
+        const unsigned tx = (unsigned)((g.nx + T::TX - 1) / T::TX), ty = (unsigned)((g.ny + T::TY - 1) / T::TY);
+        const int want = (int)((16LL * nsm + (long long)tx * ty - 1) / ((long long)tx * ty));
+        const int nc = std::max(1, std::min(want, g.nz / 8)), zc = (g.nz + nc - 1) / nc;
+        const dim3 grid(tx, ty, (unsigned)((g.nz + zc - 1) / zc));
+        pos_flux_ratio_kernel<R, SCH><<<grid, T::THREADS, 0, st>>>(pg, a[0], a[1], a[2], a[3], dtp, zc, pos_fx, pos_fy, pos_fz, pos_r);
+        pos_apply_kernel<R><<<grid, T::THREADS, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz, pos_r, zc, tend, accumulate);
+    }
     // advance_sgs! of the TKE closure for the state in `in` (halos filled)
     aeo_status enqueue_tke_commit(R* const* in) {
         const unsigned nb = (unsigned)std::min<long long>((g.nin + 255) / 256, 148LL * 16);
@@ -359,13 +372,8 @@ struct Core : CoreBase {
         pg.hx = AEO_HX; pg.hy = AEO_H; pg.hz = AEO_H;
         pg.sx = 1; pg.sy = g.sy; pg.sz = g.sz;
         pg.idx = g.idx; pg.idy = g.idy; pg.idz = g.idz;
-        const dim3 gf((unsigned)((g.nx + 1 + 127) / 128), (unsigned)(g.ny + 1), (unsigned)(g.nz + 1));
-        pos_flux_kernel<R, AEO_ADV_WENO_Z5><<<gf, 128, 0, st>>>(pg, in[0], in[1], in[2], d_tke, pos_fx, pos_fy, pos_fz);
-        CKL();
-        const dim3 gc((unsigned)((g.nx + 127) / 128), (unsigned)g.ny, (unsigned)g.nz);
-        pos_ratio_kernel<R><<<gc, 128, 0, st>>>(pg, in[0], in[1], in[2], d_tke, pos_fx, pos_fy, pos_fz, &d_sc->dt, pos_r);
-        CKL();
-        pos_apply_kernel<R><<<gc, 128, 0, st>>>(pg, in[0], in[1], in[2], d_tke, pos_fx, pos_fy, pos_fz, pos_r, d_tkt, 0);
+        const R* pa[4] = {in[0], in[1], in[2], d_tke};
+        launch_positive<AEO_ADV_WENO_Z5>(pg, pa, &d_sc->dt, d_tkt, 0);
         CKL();
         tke_update_kernel<R><<<(unsigned)((g.nin + 127) / 128), 128, 0, st>>>(g, tkeA, d_tke, d_tk2, in[3], in[0], in[1],
                                                                               in[2], &d_sc->dt, d_tkt);
@@ -2110,16 +2118,8 @@ struct Core : CoreBase {
         pg.sy = g.nx + 2LL * cfg.hx;
         pg.sz = pg.sy * (g.ny + 2LL * cfg.hy);
         pg.idx = g.idx; pg.idy = g.idy; pg.idz = g.idz;
-        const dim3 gf((unsigned)((g.nx + 1 + 127) / 128), (unsigned)(g.ny + 1), (unsigned)(g.nz + 1));
-        if (scheme == AEO_ADV_WENO_Z5)
-            pos_flux_kernel<R, AEO_ADV_WENO_Z5><<<gf, 128, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz);
-        else
-            pos_flux_kernel<R, AEO_ADV_WENO_JS5><<<gf, 128, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz);
-        CKL();
-        const dim3 gc((unsigned)((g.nx + 127) / 128), (unsigned)g.ny, (unsigned)g.nz);
-        pos_ratio_kernel<R><<<gc, 128, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz, &d_sc->pos_dt, pos_r);
-        CKL();
-        pos_apply_kernel<R><<<gc, 128, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz, pos_r, t, accumulate);
+        if (scheme == AEO_ADV_WENO_Z5) launch_positive<AEO_ADV_WENO_Z5>(pg, a, &d_sc->pos_dt, t, accumulate);
+        else launch_positive<AEO_ADV_WENO_JS5>(pg, a, &d_sc->pos_dt, t, accumulate);
         CKL();
         if (host) {
             convert_back_kernel<R><<<hb, 256, 0, st>>>(host_n, t, d_stage);

@@ -302,6 +302,27 @@ def test_cg_loop_counts_and_ends(n, precond):
     assert st["status"] == "converged" and st["iterations"] == 0 and not x.any()
 
 
+# ---- the positivity-preserving advection: tiles of 64 (FP32) or 32 columns by 8 rows, chunks of levels ----------
+@pytest.mark.parametrize("size", [(8, 4, 3), (16, 8, 9), (64, 8, 8), (32, 16, 33), (128, 32, 40), (64, 4, 70),
+                                  (256, 4, 24)])
+@pytest.mark.parametrize("scheme", ["weno_z5", "weno_js5"])
+def test_positive_tendency_over_ragged_tiles(size, scheme):
+    g = regular_grid(size, (1.0, 0.8, 0.6), bc_z="wall")
+    u, v, w, phi = random_state(g, 5)
+    phi = np.where(np.abs(phi) < 0.3, 0.0, np.abs(phi))
+    base = np.random.default_rng(6).standard_normal(g.storage_shape)
+    dt = 0.05 * min(g.dx, g.dy, g.dz)
+    o = OracleSimulation(CoreSpec(grid=g))
+    for precision, tol in (("fp64", 1e-11), ("fp32_mixed", 1e-5)):
+        s = Sim(CoreSpec(grid=g, precision=precision))
+        for acc in (False, True):
+            want = o.advect_positive(u, v, w, phi, dt, scheme=scheme, tend=base, accumulate=acc)
+            got = s.advect_positive(u, v, w, phi, dt, scheme=scheme, tend=base, accumulate=acc)
+            assert rel(got[g.interior], want[g.interior]) <= tol
+            if not acc and precision == "fp64":
+                assert (phi + dt * got)[g.interior].min() >= -1e-14
+
+
 # ---- the U-Net: weight gradients of x-segment tiles at every channel count, host arrays through pinned lanes ----
 @pytest.mark.parametrize("shape", [(512, 24, 8), (256, 16, 12), (512, 8, 16)])
 def test_unet_gradients_where_every_level_takes_x_segments(shape):
