@@ -679,9 +679,27 @@ inline size_t thomas_smem(const Geo& g) {
 }
 
 // the mean mode (_mean_mode!, src/PressureSolvers.jl:780-805), real: a warp
-// loads the column into shared memory, lane 0 runs the sums and the double
-// integration in the reference's order, the warp writes the gauged profile back
-// (the serial loops read shared memory only); sm holds 5 nz + 1 doubles
+// loads the column into shared memory, each lane takes a run of its levels, and the
+// sums and the double integration are the runs' sums and scans over the lanes; sm
+// holds 5 nz + 1 doubles.  (On one lane the three chains of nz FP64 additions
+// outlasted the other columns of a small grid: 128 x 64 x 93 FP32 20 us a launch,
+// now 18.5; larger grids' other columns take longer.)
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// the sum of the lanes before this one
+__device__ __forceinline__ double lane_scan(double v, int lane) {
+    double s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += t;
+    }
+    s = __shfl_up_sync(0xffffffffu, s, 1);
+    return lane ? s : 0.0;
+}
 template <typename R>
 __device__ __forceinline__ void thomas_mean(cplx<R>* S, long long sk, int nz, int lane, double* sm, const ColumnCoef& c) {
     double* sv = sm;             // [nz] the column's real parts
@@ -696,24 +714,26 @@ __device__ __forceinline__ void thomas_mean(cplx<R>* S, long long sk, int nz, in
     }
     for (int k = lane; k <= nz; k += 32) io[k] = c.iota[k];
     __syncwarp();
-    if (lane == 0) {
-        double mb = 0.0;
-        for (int k = 0; k < nz; ++k) mb += sv[k] * me[k];
-        mb /= c.meas_sum;
-        double F = 0.0, acc = 0.0, prev = sv[0] - mb;
-        ph[0] = 0.0;
-        for (int k = 1; k < nz; ++k) {
-            F += prev * me[k - 1];
-            acc += F * io[k];
-            prev = sv[k] - mb;
-            ph[k] = acc;
-        }
-        double mp = 0.0;
-        for (int k = 0; k < nz; ++k) mp += ph[k] * ga[k];
-        sv[0] = mp / c.gauge_sum;
+    const int run = (nz + 31) / 32, k0 = min(lane * run, nz), k1 = min(k0 + run, nz);
+    double v = 0.0;
+    for (int k = k0; k < k1; ++k) v += sv[k] * me[k];
+    const double mb = lane_sum(v) / c.meas_sum;
+    v = 0.0;
+    for (int k = k0; k < k1; ++k) v += (sv[k] - mb) * me[k];
+    double F = lane_scan(v, lane), acc = 0.0;   // F: the flux below level k
+    for (int k = k0; k < k1; ++k) {
+        if (k > 0) acc += F * io[k];
+        ph[k] = acc;
+        F += (sv[k] - mb) * me[k];
     }
+    acc = lane_scan(acc, lane);
+    v = 0.0;
+    for (int k = k0; k < k1; ++k) {
+        ph[k] += acc;
+        v += ph[k] * ga[k];
+    }
+    const double sh = lane_sum(v) / c.gauge_sum;
     __syncwarp();
-    const double sh = sv[0];
     for (int k = lane; k < nz; k += 32) S[k * sk] = cmk<R>(R(ph[k] - sh), R(0));
 }
 
@@ -756,8 +776,9 @@ __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restric
 // (the twisted factorisation; 1 - c c' > 0, the pivots of a diagonally dominant
 // column), and each warp substitutes back through its own half.  The solve is
 // bound by the latency of the FP64 recurrence at 1.7 warps a scheduler, and this
-// halves the chain and doubles the warps (one warp over the whole column:
-// 256 x 256 x 128 FP32 36 us a launch).  Levels stream through a cp.async ring
+// halves the chain and doubles the warps (128 x 64 x 93 FP32 23 -> 20 us a launch,
+// 256 x 256 x 128 FP64 42 -> 39); in FP32 at 256 x 256 x 128 (37 us) the levels'
+// four passes and the factors' two through L2 are the bound.  Levels stream through a cp.async ring
 // THOMAS_PF ahead, d in place over S, as in thomas_kernel.
 constexpr size_t THOMAS_TW_RING = (size_t)THOMAS_PF * 32 * 3 * sizeof(double);   // a warp's levels and factors
 inline size_t thomas_tw_smem(const Geo& g) {

@@ -323,6 +323,26 @@ def test_positive_tendency_over_ragged_tiles(size, scheme):
                 assert (phi + dt * got)[g.interior].min() >= -1e-14
 
 
+# ---- the halo written with the correction (nz >= 4) or by the shell's fill, where rows and columns have several images
+@pytest.mark.parametrize("size,bc_z", [((4, 4, 4), "periodic"), ((4, 4, 4), "wall"), ((8, 4, 8), "periodic"),
+                                       ((4, 8, 5), "wall"), ((16, 4, 3), "wall"), ((8, 8, 2), "wall"), ((64, 32, 7), "wall")])
+@pytest.mark.parametrize("scheme", ["centred", "weno_z5"])
+def test_halo_images_at_the_smallest_extents(size, bc_z, scheme):
+    g = regular_grid(size, (1.0, 1.0, 1.0), bc_z=bc_z)
+    kw = dict(grid=g, advection=scheme, nu=1e-3)
+    state = random_state(g, 12, 0.5)
+    o = OracleSimulation(CoreSpec(**kw))
+    s64, s32 = Sim(CoreSpec(**kw)), Sim(CoreSpec(precision="fp32_mixed", **kw))
+    for s in (o, s64, s32):
+        s.set_state(*state)
+        s.project()
+        s.step_rk3(2e-3, 3)
+    for n in ("u", "v", "w", "theta"):
+        want = o.get_field(n)[g.interior]
+        assert rel(s64.get_field(n)[g.interior], want) <= 1e-11, n
+        assert rel(s32.get_field(n)[g.interior], want) <= 1e-5, n
+
+
 # ---- the U-Net: weight gradients of x-segment tiles at every channel count, host arrays through pinned lanes ----
 @pytest.mark.parametrize("shape", [(512, 24, 8), (256, 16, 12), (512, 8, 16)])
 def test_unet_gradients_where_every_level_takes_x_segments(shape):
