@@ -304,7 +304,9 @@ __global__ void pcg_init_kernel(const double* __restrict__ b, double* __restrict
 // Ap = A p with p.Ap; the last block forms alpha or flags a breakdown.
 // Block (32, 8): lanes along x, warps over rows, rows looped on a fixed grid.
 // The coefficient form is a template parameter (codes: the table, padded to
-// 256 entries, staged in shared memory); the arithmetic of aphi in FP64.
+// 256 entries, staged in shared memory); the arithmetic of aphi in FP64.  Even nx:
+// two x-adjacent cells a thread and 16-byte accesses, 11 loads for the pair where
+// two cells take 26 (256 x 256 x 96 FP32 cycle: 50 -> 44 us).
 template <typename C, int CF>
 __global__ void __launch_bounds__(RB_X * RB_Y) pcg_apply_kernel(const double* __restrict__ p, double* __restrict__ Ap,
                                                                Coef<C> cf, int nx, int ny, int nz, Bc bc, double ix2,
@@ -319,29 +321,69 @@ __global__ void __launch_bounds__(RB_X * RB_Y) pcg_apply_kernel(const double* __
     }
     double v[1] = {0.0};
     const int nrows = ny * nz, pl = nx * ny;
+    // p and the coefficients are read-only here: the non-coherent path
+    auto fx_ = [&](int f) { return CF == CF_CODES ? stab[__ldg(cf.kx + f)] : double(__ldg(cf.cx + f)); };
+    // A p at a cell from p there and around it and its y and z coefficients
+    auto point = [&](double c, double pxm, double pxp, double pym, double pyp, double pzm, double pzp, double fxm,
+                     double fxp, double fym, double fyp, double fzm, double fzp) {
+        if (CF == CF_CONST)
+            return (pxp - 2.0 * c + pxm) * ix2 + (pyp - 2.0 * c + pym) * iy2 + (pzp - 2.0 * c + pzm) * iz2;
+        return (fxp * (pxp - c) - fxm * (c - pxm)) * ix2 + (fyp * (pyp - c) - fym * (c - pym)) * iy2 +
+               (fzp * (pzp - c) - fzm * (c - pzm)) * iz2;
+    };
     for (int row = blockIdx.x * blockDim.y + threadIdx.y; row < nrows; row += gridDim.x * blockDim.y) {
         const int j = row % ny, k = row / ny;
+        if ((nx & 1) == 0) {
+            // x pairs: every row, and so every pair, starts on 16 bytes (two codes on two)
+            for (int i = 2 * threadIdx.x; i < nx; i += 2 * blockDim.x) {
+                const int q = i + nx * row;
+                const Nbr n = nbr_of(q, i, j, k, nx, ny, nz, pl, bc);
+                auto ld = [&](int e) { return __ldg(reinterpret_cast<const double2*>(p + e)); };
+                const double2 c = ld(q), ym = ld(n.ym), yp = ld(n.yp), zm = ld(n.zm), zp = ld(n.zp);
+                const double xl = i > 0 || bc.x == 0 ? __ldg(p + n.xm) : c.x;
+                const double xr = i + 2 < nx ? __ldg(p + q + 2) : (bc.x == 0 ? __ldg(p + q + 2 - nx) : c.y);
+                double f0 = 0, f1 = 0, f2 = 0;
+                double2 gm{}, gp{}, hm{}, hp{};
+                if (CF != CF_CONST) {
+                    const int fx = q + j + ny * k, fy = q + nx * k;
+                    auto two = [&](const unsigned char* kc, const C* cv, int f) {
+                        if (CF == CF_CODES) {
+                            const uchar2 u = __ldg(reinterpret_cast<const uchar2*>(kc + f));
+                            return make_double2(stab[u.x], stab[u.y]);
+                        }
+                        return make_double2(double(__ldg(cv + f)), double(__ldg(cv + f + 1)));
+                    };
+                    f0 = fx_(fx);
+                    f1 = fx_(fx + 1);
+                    f2 = fx_(fx + 2);
+                    gm = two(cf.ky, cf.cy, fy);
+                    gp = two(cf.ky, cf.cy, fy + nx);
+                    hm = two(cf.kz, cf.cz, q);
+                    hp = two(cf.kz, cf.cz, q + pl);
+                }
+                double2 a;
+                a.x = point(c.x, xl, c.y, ym.x, yp.x, zm.x, zp.x, f0, f1, gm.x, gp.x, hm.x, hp.x);
+                a.y = point(c.y, c.x, xr, ym.y, yp.y, zm.y, zp.y, f1, f2, gm.y, gp.y, hm.y, hp.y);
+                *reinterpret_cast<double2*>(Ap + q) = a;
+                v[0] += c.x * a.x + c.y * a.y;
+            }
+            continue;
+        }
         for (int i = threadIdx.x; i < nx; i += blockDim.x) {
             const int q = i + nx * row;
             const Nbr n = nbr_of(q, i, j, k, nx, ny, nz, pl, bc);
-            // p and the coefficients are read-only here: the non-coherent path
             const double c = __ldg(p + q);
-            const double pxp = __ldg(p + n.xp), pxm = __ldg(p + n.xm), pyp = __ldg(p + n.yp), pym = __ldg(p + n.ym);
-            const double pzp = __ldg(p + n.zp), pzm = __ldg(p + n.zm);
-            double a;
-            if (CF == CF_CONST) {
-                a = (pxp - 2.0 * c + pxm) * ix2 + (pyp - 2.0 * c + pym) * iy2 + (pzp - 2.0 * c + pzm) * iz2;
-            } else {
-                const int fx = q + j + ny * k, fy = q + nx * k;
-                const double fxm = CF == CF_CODES ? stab[__ldg(cf.kx + fx)] : double(__ldg(cf.cx + fx));
-                const double fxp = CF == CF_CODES ? stab[__ldg(cf.kx + fx + 1)] : double(__ldg(cf.cx + fx + 1));
-                const double fym = CF == CF_CODES ? stab[__ldg(cf.ky + fy)] : double(__ldg(cf.cy + fy));
-                const double fyp = CF == CF_CODES ? stab[__ldg(cf.ky + fy + nx)] : double(__ldg(cf.cy + fy + nx));
-                const double fzm = CF == CF_CODES ? stab[__ldg(cf.kz + q)] : double(__ldg(cf.cz + q));
-                const double fzp = CF == CF_CODES ? stab[__ldg(cf.kz + q + pl)] : double(__ldg(cf.cz + q + pl));
-                a = (fxp * (pxp - c) - fxm * (c - pxm)) * ix2 + (fyp * (pyp - c) - fym * (c - pym)) * iy2 +
-                    (fzp * (pzp - c) - fzm * (c - pzm)) * iz2;
+            const int fx = q + j + ny * k, fy = q + nx * k;
+            auto fy_ = [&](int f) { return CF == CF_CODES ? stab[__ldg(cf.ky + f)] : double(__ldg(cf.cy + f)); };
+            auto fz_ = [&](int f) { return CF == CF_CODES ? stab[__ldg(cf.kz + f)] : double(__ldg(cf.cz + f)); };
+            double f[6] = {};
+            if (CF != CF_CONST) {
+                f[0] = fx_(fx); f[1] = fx_(fx + 1);
+                f[2] = fy_(fy); f[3] = fy_(fy + nx);
+                f[4] = fz_(q); f[5] = fz_(q + pl);
             }
+            const double a = point(c, __ldg(p + n.xm), __ldg(p + n.xp), __ldg(p + n.ym), __ldg(p + n.yp), __ldg(p + n.zm),
+                                   __ldg(p + n.zp), f[0], f[1], f[2], f[3], f[4], f[5]);
             Ap[q] = a;
             v[0] += c * a;
         }
@@ -716,31 +758,57 @@ __global__ void __launch_bounds__(RB_X * RB_Y) mg_restrict_kernel(Level<R> F, Le
 }
 
 // phi_fine += trilinear (3/4, 1/4) interpolation of phi_coarse
-// (src/Multigrid.jl:412-455), the eight terms in the reference's order.
+// (src/Multigrid.jl:412-455), the eight terms of a cell in the reference's order.
+// A thread takes the eight fine cells of a coarse cell: 27 coarse values for them
+// instead of eight for each, and phi in x pairs (a cycle of 256 x 256 x 96 FP32
+// 327 -> 311 us against a thread a cell).
 template <typename R>
-__global__ void mg_prolong_kernel(Level<R> F, Level<R> Cl, Bc bc, int early) {
+__global__ void __launch_bounds__(RB_X * RB_Y) mg_prolong_kernel(Level<R> F, Level<R> Cl, Bc bc, int early) {
     if (early) pdl_trigger();
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
-    if (i >= F.nx || j >= F.ny) return;
-    const int Ih = i >> 1, Jh = j >> 1, Kh = k >> 1;
-    const int Ix = (i & 1) ? wp(Ih, Cl.nx, bc.x) : wm(Ih, Cl.nx, bc.x);
-    const int Jy = (j & 1) ? wp(Jh, Cl.ny, bc.y) : wm(Jh, Cl.ny, bc.y);
-    const int Kz = (k & 1) ? wp(Kh, Cl.nz, bc.z) : wm(Kh, Cl.nz, bc.z);
+    const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y, K = blockIdx.z;
+    if (I >= Cl.nx || J >= Cl.ny) return;
+    const int xs[3] = {wm(I, Cl.nx, bc.x), I, wp(I, Cl.nx, bc.x)};
+    const int ys[3] = {Cl.nx * wm(J, Cl.ny, bc.y), Cl.nx * J, Cl.nx * wp(J, Cl.ny, bc.y)};
+    const int pl = Cl.nx * Cl.ny, zs[3] = {pl * wm(K, Cl.nz, bc.z), pl * K, pl * wp(K, Cl.nz, bc.z)};
+    using V2 = typename Vec2<R>::T;
+    V2* out = reinterpret_cast<V2*>(F.phi + 2 * I + F.nx * (2 * J + F.ny * 2 * K));
+    const int oy = F.nx / 2, oz = oy * F.ny;   // in pairs
+    V2 f[2][2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) f[c][b] = out[b * oy + c * oz];
+    R P[3][3][3];
+#pragma unroll
+    for (int z = 0; z < 3; ++z)
+#pragma unroll
+        for (int y = 0; y < 3; ++y)
+#pragma unroll
+            for (int x = 0; x < 3; ++x) P[z][y][x] = Cl.phi[xs[x] + ys[y] + zs[z]];
     const R n_ = R(3) / R(4), f_ = R(1) / R(4);
-    const int sy = Cl.nx, sz = Cl.nx * Cl.ny;
-    const R* P = Cl.phi;
-    R acc = R(0);
-    acc += (n_ * n_ * n_) * P[Ih + Jh * sy + Kh * sz];
-    acc += (f_ * n_ * n_) * P[Ix + Jh * sy + Kh * sz];
-    acc += (n_ * f_ * n_) * P[Ih + Jy * sy + Kh * sz];
-    acc += (f_ * f_ * n_) * P[Ix + Jy * sy + Kh * sz];
-    acc += (n_ * n_ * f_) * P[Ih + Jh * sy + Kz * sz];
-    acc += (f_ * n_ * f_) * P[Ix + Jh * sy + Kz * sz];
-    acc += (n_ * f_ * f_) * P[Ih + Jy * sy + Kz * sz];
-    acc += (f_ * f_ * f_) * P[Ix + Jy * sy + Kz * sz];
-    const int q = F.nx * (j + F.ny * k) + i;
-    F.phi[q] += acc;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            R acc[2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                R t = R(0);
+                t += (n_ * n_ * n_) * P[1][1][1];
+                t += (f_ * n_ * n_) * P[1][1][2 * a];
+                t += (n_ * f_ * n_) * P[1][2 * b][1];
+                t += (f_ * f_ * n_) * P[1][2 * b][2 * a];
+                t += (n_ * n_ * f_) * P[2 * c][1][1];
+                t += (f_ * n_ * f_) * P[2 * c][1][2 * a];
+                t += (n_ * f_ * f_) * P[2 * c][2 * b][1];
+                t += (f_ * f_ * f_) * P[2 * c][2 * b][2 * a];
+                acc[a] = t;
+            }
+            f[c][b].x += acc[0];
+            f[c][b].y += acc[1];
+            out[b * oy + c * oz] = f[c][b];
+        }
 }
 
 // The coarsest level: phi = 0, b -= mean, then `sweeps` RB-GS sweeps, all in

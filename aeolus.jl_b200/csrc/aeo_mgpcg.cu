@@ -563,7 +563,7 @@ struct Mg : MgBase {
         if (aeo_status q = launch_coarsest(s, L[nl - 1], nullptr)) return q;
         for (int l = nl - 2; l >= 0; --l) {
             Level<R>& F = L[l];
-            AEO_PDL_LAUNCH((mg_prolong_kernel<R>), cell_grid(F), blk, 0, s, F, L[l + 1], bc, early(F));
+            AEO_PDL_LAUNCH((mg_prolong_kernel<R>), cell_grid(L[l + 1]), blk, 0, s, F, L[l + 1], bc, early(F));
             CKL();
             for (int sw = 0; sw < cfg.nu2; ++sw)
                 for (int c = 0; c < 2; ++c)
