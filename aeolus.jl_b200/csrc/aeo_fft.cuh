@@ -743,7 +743,10 @@ __device__ __forceinline__ void thomas_mean(cplx<R>* S, long long sk, int nz, in
 // its neighbour on the far side, in precision RD at the spectrum's layout (mtab,
 // ctab).  They depend on the column's coefficients and its eigenvalue
 // kx^2 + ky^2 only, so the solves of a run stream them instead of recomputing
-// the division chain.
+// the division chain.  The elimination runs on g_k = 1 + c_k, whose recurrence adds
+// positive terms only: the pivot is -(far + lambda h + near g), where the textbook
+// form takes two numbers close to each other apart on the longest waves.  At the
+// meeting's two levels ctab holds g.
 template <typename RD>
 __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restrict__ mtab, RD* __restrict__ ctab,
                                                             ColumnCoef c) {
@@ -756,15 +759,15 @@ __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restric
     const double lam = c.kx2[p] + c.ky2[j];
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
-        double cprev = 0.0;
-        for (int t = 0; t < (half ? nz - mid : mid); ++t) {
+        double gam = 0.0;   // 1 + c of the level before (its coefficient `near` is 0 at the wall)
+        const int n = half ? nz - mid : mid;
+        for (int t = 0; t < n; ++t) {
             const int k = half ? nz - 1 - t : t;
-            const double lo = c.lower[k], up = c.upper[k];
-            const double b = -(lo + up) - lam * c.hw[k];
-            const double id = 1.0 / (b - (half ? up : lo) * cprev);
-            cprev = (half ? lo : up) * id;
+            const double near_ = half ? c.upper[k] : c.lower[k], far = half ? c.lower[k] : c.upper[k];
+            const double open = lam * c.hw[k] + near_ * gam, id = -1.0 / (far + open);
+            gam = -open * id;
             mtab[col + (long long)k * sk] = RD(id);
-            ctab[col + (long long)k * sk] = RD(cprev);
+            ctab[col + (long long)k * sk] = RD(t < n - 1 ? far * id : gam);
         }
     }
 }
@@ -773,8 +776,8 @@ __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restric
 // from the bottom up to level mid - 1, the other from the top down to mid; with
 // d, c the eliminated value and coefficient each warp ends on, the two unknowns
 // at the meeting are phi = (d - c d') / (1 - c c') of their own and the other's
-// (the twisted factorisation; 1 - c c' > 0, the pivots of a diagonally dominant
-// column), and each warp substitutes back through its own half.  The solve is
+// (the twisted factorisation), with g = 1 + c: 1 - c c' = g + g' - g g', no difference
+// of close numbers; and each warp substitutes back through its own half.  The solve is
 // bound by the latency of the FP64 recurrence at 1.7 warps a scheduler, and this
 // halves the chain and doubles the warps (128 x 64 x 93 FP32 23 -> 20 us a launch,
 // 256 x 256 x 128 FP64 42 -> 39); in FP32 at 256 x 256 x 128 (37 us) the levels'
@@ -836,16 +839,17 @@ __global__ void __launch_bounds__(64) thomas_tw_kernel(Geo g, cplx<R>* S, Column
     }
     thomas_wait<0>();
     // the meeting
-    const double cm = on ? (double)ctab[at(n - 1)] : 0.0;
+    const double cm = on ? (double)ctab[at(n - 1)] : 1.0;   // g = 1 + c
     xch[(half * 3 + 0) * 32 + lane] = dr;
     xch[(half * 3 + 1) * 32 + lane] = di;
     xch[(half * 3 + 2) * 32 + lane] = cm;
     __syncthreads();
     if (!on) return;
     const int o = 1 - half;
-    const double den = 1.0 / (1.0 - cm * xch[(o * 3 + 2) * 32 + lane]);
-    dr = (dr - cm * xch[(o * 3 + 0) * 32 + lane]) * den;
-    di = (di - cm * xch[(o * 3 + 1) * 32 + lane]) * den;
+    const double co = xch[(o * 3 + 2) * 32 + lane], den = 1.0 / (cm + co - cm * co);
+    const double odr = xch[(o * 3 + 0) * 32 + lane], odi = xch[(o * 3 + 1) * 32 + lane];
+    dr = (dr + odr - cm * odr) * den;
+    di = (di + odi - cm * odi) * den;
     S[at(n - 1)] = cmk<R>(R(dr), R(di));
     // back through this half, levels n - 2 .. 0; slot u holds level n - 2 - u modulo D
     auto refetch = [&](int u) {
