@@ -16,10 +16,9 @@
 //   fftz_solve periodic z: forward transform, scale by nrm/lambda (zero mean
 //              mode), inverse transform -- one pass (src/PressureSolvers.jl:128-138,
 //              :162-174)
-//   thomas_tw  walls in z: per horizontal wavenumber the tridiagonal solve in
-//              FP64 from both ends with tabulated factors, the mean mode
-//              integrated (src/PressureSolvers.jl:650-661, :754-805); thomas: one
-//              way, the factors recomputed (the allocation-free entry)
+//   thomas     walls in z: per horizontal wavenumber the tridiagonal solve in
+//              FP64 with the factors recomputed on the fly, the mean mode
+//              integrated (src/PressureSolvers.jl:650-661, :754-805)
 //   ifftx      c2r along x into the potential phi (interior array)
 //
 // The transforms are Stockham autosort FFTs of in-register DFTs of radix 16, 8
@@ -634,13 +633,17 @@ struct ColumnCoef {
 // streams its column through a shared-memory ring with cp.async, THOMAS_PF
 // levels ahead of the recurrence, and waits (cp.async.wait_group) for exactly
 // the level it needs, so the loads overlap the FP64 recurrence instead of
-// exposing one memory latency per level.  The forward-elimination values go in
-// place over S (each overwrites the level it came from after that level was
-// read); the recurrence itself runs in FP64, and an FP32 step's stored
-// intermediates carry the rounding of the FP32 spectrum they came from.
-// thomas_kernel, the allocation-free entry's, has no scratch for factors: it
-// forms them on the way and keeps the modified upper diagonal c'_k in shared
-// memory [nz][32].
+// exposing one memory latency per level.  The forward-elimination values d'_k
+// go to dsc, a column scratch of the spectrum's layout in precision RD (dsc
+// may alias S when RD is S's type: d'_k overwrites the level it came from
+// after that level was read).  The modified upper diagonal c'_k goes either
+// to an RD scratch of the same layout (CPG: streamed back with d'_k, so a CTA
+// needs only its rings and every column warp of the grid is resident at
+// once) or to shared memory [nz][32] (no scratch: the allocation-free entry).
+// The recurrence itself runs in FP64 whatever RD is; the FP32-mixed step
+// stores d' and c' in FP32 in place (S and an FP32 c' array), so the stored
+// intermediates carry the rounding of the FP32 spectrum they came from and
+// the solve moves 40 bytes an element instead of 64.
 constexpr int THOMAS_PF = 16;
 // the largest nz whose column state fits a CTA's 227 KB of shared memory
 #define AEO_COLUMN_NZ_MAX 800
@@ -671,211 +674,53 @@ __device__ __forceinline__ void thomas_wait() { asm volatile("cp.async.wait_grou
 inline unsigned thomas_blocks(const Geo& g) {
     return 1u + (unsigned)(((long long)g.ny * (g.nx / 2 + 1) + 31) / 32);
 }
-// Shared memory of thomas_kernel: the d' ring [THOMAS_PF][32] of cplx<double>,
-// c' [nz][32], then the lower, upper and h vectors [nz] each; at least the mean
-// mode's 5 nz + 1.
-inline size_t thomas_smem(const Geo& g) {
-    return (size_t)THOMAS_PF * 32 * 2 * sizeof(double) + (size_t)std::max(g.nz * 35, 5 * g.nz + 1) * sizeof(double);
+// Shared memory: the d' ring [THOMAS_PF][32] of cplx<double>, then (CPG) the
+// c' ring [THOMAS_PF][32] of double or (shared c') c' [nz][32], then the
+// lower, upper and h vectors [nz] each; at least the mean mode's 5 nz + 1.
+inline size_t thomas_smem(const Geo& g, bool cpg) {
+    const size_t ring = (size_t)THOMAS_PF * 32 * 2 * sizeof(double);
+    const size_t cols = cpg ? (size_t)THOMAS_PF * 32 * sizeof(double) + (size_t)g.nz * 3 * sizeof(double)
+                            : (size_t)g.nz * 35 * sizeof(double);
+    const size_t mean = (size_t)(5 * g.nz + 1) * sizeof(double);
+    return ring + (cols > mean ? cols : mean);
 }
 
-// the mean mode (_mean_mode!, src/PressureSolvers.jl:780-805), real: a warp
-// loads the column into shared memory, each lane takes a run of its levels, and the
-// sums and the double integration are the runs' sums and scans over the lanes; sm
-// holds 5 nz + 1 doubles.  (On one lane the three chains of nz FP64 additions
-// outlasted the other columns of a small grid: 128 x 64 x 93 FP32 20 us a launch,
-// now 18.5; larger grids' other columns take longer.)
-__device__ __forceinline__ double lane_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-// the sum of the lanes before this one
-__device__ __forceinline__ double lane_scan(double v, int lane) {
-    double s = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double t = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += t;
-    }
-    s = __shfl_up_sync(0xffffffffu, s, 1);
-    return lane ? s : 0.0;
-}
-template <typename R>
-__device__ __forceinline__ void thomas_mean(cplx<R>* S, long long sk, int nz, int lane, double* sm, const ColumnCoef& c) {
-    double* sv = sm;             // [nz] the column's real parts
-    double* ph = sv + nz;        // [nz] the integrated profile
-    double* me = ph + nz;        // [nz] measures
-    double* io = me + nz;        // [nz + 1] iota
-    double* ga = io + nz + 1;    // [nz] gauge weights
-    for (int k = lane; k < nz; k += 32) {
-        sv[k] = (double)S[k * sk].x;
-        me[k] = c.meas[k];
-        ga[k] = c.gauge[k];
-    }
-    for (int k = lane; k <= nz; k += 32) io[k] = c.iota[k];
-    __syncwarp();
-    const int run = (nz + 31) / 32, k0 = min(lane * run, nz), k1 = min(k0 + run, nz);
-    double v = 0.0;
-    for (int k = k0; k < k1; ++k) v += sv[k] * me[k];
-    const double mb = lane_sum(v) / c.meas_sum;
-    v = 0.0;
-    for (int k = k0; k < k1; ++k) v += (sv[k] - mb) * me[k];
-    double F = lane_scan(v, lane), acc = 0.0;   // F: the flux below level k
-    for (int k = k0; k < k1; ++k) {
-        if (k > 0) acc += F * io[k];
-        ph[k] = acc;
-        F += (sv[k] - mb) * me[k];
-    }
-    acc = lane_scan(acc, lane);
-    v = 0.0;
-    for (int k = k0; k < k1; ++k) {
-        ph[k] += acc;
-        v += ph[k] * ga[k];
-    }
-    const double sh = lane_sum(v) / c.gauge_sum;
-    __syncwarp();
-    for (int k = lane; k < nz; k += 32) S[k * sk] = cmk<R>(R(ph[k] - sh), R(0));
-}
-
-// The elimination factors of every non-mean column, once per grid, for an
-// elimination from both ends that meets above level mid = nz/2: the multiplier
-// m_k of level k and the coefficient c_k = (up_k below, lo_k from mid on) m_k of
-// its neighbour on the far side, in precision RD at the spectrum's layout (mtab,
-// ctab).  They depend on the column's coefficients and its eigenvalue
-// kx^2 + ky^2 only, so the solves of a run stream them instead of recomputing
-// the division chain.  The elimination runs on g_k = 1 + c_k, whose recurrence adds
-// positive terms only: the pivot is -(far + lambda h + near g), where the textbook
-// form takes two numbers close to each other apart on the longest waves.  At the
-// meeting's two levels ctab holds g.
+// The elimination factors of every non-mean column, once per grid: the
+// multiplier m_k = 1 / (b_k - lo_k c'_{k-1}) of level k and c'_k = up_k m_k,
+// in precision RD at the spectrum's layout (mtab, ctab).  They depend on the
+// column's coefficients and its eigenvalue kx^2 + ky^2 only, so the solves
+// of a run stream them instead of recomputing the division chain; the FP64
+// arithmetic and its order are those of the solve kernel's own elimination,
+// so an FP64 table reproduces it exactly.
 template <typename RD>
 __global__ void __launch_bounds__(256) thomas_factor_kernel(Geo g, RD* __restrict__ mtab, RD* __restrict__ ctab,
                                                             ColumnCoef c) {
-    const int Mh = g.nx / 2 + 1, nz = g.nz, mid = nz / 2;
+    const int Mh = g.nx / 2 + 1;
     const long long sk = (long long)g.ny * g.sp;
     const long long id0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id0 == 0 || id0 >= (long long)g.ny * Mh) return;
     const int p = (int)(id0 % Mh), j = (int)(id0 / Mh);
     const long long col = (long long)j * g.sp + p;
     const double lam = c.kx2[p] + c.ky2[j];
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-        double gam = 0.0;   // 1 + c of the level before (its coefficient `near` is 0 at the wall)
-        const int n = half ? nz - mid : mid;
-        for (int t = 0; t < n; ++t) {
-            const int k = half ? nz - 1 - t : t;
-            const double near_ = half ? c.upper[k] : c.lower[k], far = half ? c.lower[k] : c.upper[k];
-            const double open = lam * c.hw[k] + near_ * gam, id = -1.0 / (far + open);
-            gam = -open * id;
-            mtab[col + (long long)k * sk] = RD(id);
-            ctab[col + (long long)k * sk] = RD(t < n - 1 ? far * id : gam);
-        }
+    double cprev = 0.0;
+    for (int k = 0; k < g.nz; ++k) {
+        const double lo = c.lower[k], up = c.upper[k];
+        const double b = -(lo + up) - lam * c.hw[k];
+        const double den = b - lo * cprev;
+        const double id = 1.0 / den;
+        cprev = up * id;
+        mtab[col + (long long)k * sk] = RD(id);
+        if (k < g.nz - 1) ctab[col + (long long)k * sk] = RD(cprev);
     }
 }
 
-// The factored column solve: two warps take the same 32 columns, one eliminates
-// from the bottom up to level mid - 1, the other from the top down to mid; with
-// d, c the eliminated value and coefficient each warp ends on, the two unknowns
-// at the meeting are phi = (d - c d') / (1 - c c') of their own and the other's
-// (the twisted factorisation), with g = 1 + c: 1 - c c' = g + g' - g g', no difference
-// of close numbers; and each warp substitutes back through its own half.  The solve is
-// bound by the latency of the FP64 recurrence at 1.7 warps a scheduler, and this
-// halves the chain and doubles the warps (128 x 64 x 93 FP32 23 -> 20 us a launch,
-// 256 x 256 x 128 FP64 42 -> 39); in FP32 at 256 x 256 x 128 (37 us) the levels'
-// four passes and the factors' two through L2 are the bound.  Levels stream through a cp.async ring
-// THOMAS_PF ahead, d in place over S, as in thomas_kernel.
-constexpr size_t THOMAS_TW_RING = (size_t)THOMAS_PF * 32 * 3 * sizeof(double);   // a warp's levels and factors
-inline size_t thomas_tw_smem(const Geo& g) {
-    const size_t cols = 2 * THOMAS_TW_RING + (size_t)2 * g.nz * sizeof(double) + 2 * 32 * 3 * sizeof(double);
-    const size_t mean = (size_t)(5 * g.nz + 1) * sizeof(double);
-    return cols > mean ? cols : mean;
-}
-template <typename R>
-__global__ void __launch_bounds__(64) thomas_tw_kernel(Geo g, cplx<R>* S, ColumnCoef c, const R* __restrict__ mtab,
-                                                       const R* __restrict__ ctab) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int D = THOMAS_PF;
-    const int Mh = g.nx / 2 + 1, nz = g.nz, mid = nz / 2;
-    const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
-    const long long sk = (long long)g.ny * g.sp;
-    if (blockIdx.x == 0) {
-        if (half == 0) thomas_mean(S, sk, nz, lane, reinterpret_cast<double*>(smem_raw), c);
-        return;
-    }
-    // this warp's ring of levels [D][32] and factors [D][32]; then the near coefficients
-    // (lo below, up above) of the levels, then the exchange at the meeting
-    cplx<R>* ring = reinterpret_cast<cplx<R>*>(smem_raw + half * THOMAS_TW_RING);
-    R* fring = reinterpret_cast<R*>(smem_raw + half * THOMAS_TW_RING + (size_t)D * 32 * 2 * sizeof(double));
-    double* near_ = reinterpret_cast<double*>(smem_raw + 2 * THOMAS_TW_RING) + half * nz;
-    double* xch = reinterpret_cast<double*>(smem_raw + 2 * THOMAS_TW_RING) + 2 * nz;   // [2][3][32]
-    for (int k = lane; k < nz; k += 32) near_[k] = half ? c.upper[k] : c.lower[k];
-    __syncwarp();
-    const long long id0 = (long long)(blockIdx.x - 1) * 32 + lane;
-    const bool on = id0 != 0 && id0 < (long long)g.ny * Mh;   // (an idle lane still meets the other warp)
-    const long long idc = on ? id0 : 1;
-    const int p = (int)(idc % Mh), j = (int)(idc / Mh);
-    const long long col = (long long)j * g.sp + p;
-    const int n = half ? nz - mid : mid;
-    auto at = [&](int t) { return col + (long long)(half ? nz - 1 - t : t) * sk; };   // the t-th level from this end
-    auto fetch = [&](int t, const R* tab) {
-        if (on && t >= 0 && t < n) {
-            thomas_cp<sizeof(cplx<R>)>(ring + (t % D) * 32 + lane, S + at(t));
-            thomas_cp<sizeof(R)>(fring + (t % D) * 32 + lane, tab + at(t));
-        }
-        thomas_commit();
-    };
-#pragma unroll
-    for (int q = 0; q < D - 1; ++q) fetch(q, mtab);
-    double dr = 0.0, di = 0.0;
-    for (int t = 0; t < n; ++t) {
-        fetch(t + D - 1, mtab);   // into the slot read one level earlier
-        thomas_wait<D - 1>();     // level t has landed
-        if (on) {
-            const cplx<R> s = ring[(t % D) * 32 + lane];
-            const double m = (double)fring[(t % D) * 32 + lane], co = near_[half ? nz - 1 - t : t];
-            dr = ((double)s.x - co * dr) * m;
-            di = ((double)s.y - co * di) * m;
-            if (t < n - 1) S[at(t)] = cmk<R>(R(dr), R(di));
-        }
-    }
-    thomas_wait<0>();
-    // the meeting
-    const double cm = on ? (double)ctab[at(n - 1)] : 1.0;   // g = 1 + c
-    xch[(half * 3 + 0) * 32 + lane] = dr;
-    xch[(half * 3 + 1) * 32 + lane] = di;
-    xch[(half * 3 + 2) * 32 + lane] = cm;
-    __syncthreads();
-    if (!on) return;
-    const int o = 1 - half;
-    const double co = xch[(o * 3 + 2) * 32 + lane], den = 1.0 / (cm + co - cm * co);
-    const double odr = xch[(o * 3 + 0) * 32 + lane], odi = xch[(o * 3 + 1) * 32 + lane];
-    dr = (dr + odr - cm * odr) * den;
-    di = (di + odi - cm * odi) * den;
-    S[at(n - 1)] = cmk<R>(R(dr), R(di));
-    // back through this half, levels n - 2 .. 0; slot u holds level n - 2 - u modulo D
-    auto refetch = [&](int u) {
-        const int t = n - 2 - u;
-        if (t >= 0) {
-            thomas_cp<sizeof(cplx<R>)>(ring + (u % D) * 32 + lane, S + at(t));
-            thomas_cp<sizeof(R)>(fring + (u % D) * 32 + lane, ctab + at(t));
-        }
-        thomas_commit();
-    };
-#pragma unroll
-    for (int q = 0; q < D - 1; ++q) refetch(q);
-    for (int u = 0; u <= n - 2; ++u) {
-        refetch(u + D - 1);
-        thomas_wait<D - 1>();
-        const cplx<R> d = ring[(u % D) * 32 + lane];
-        const double cc = (double)fring[(u % D) * 32 + lane];
-        dr = (double)d.x - cc * dr;
-        di = (double)d.y - cc * di;
-        S[at(n - 2 - u)] = cmk<R>(R(dr), R(di));
-    }
-    thomas_wait<0>();
-}
-
-template <typename R>
-__global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, ColumnCoef c) {
+// FAC: the elimination factors come from thomas_factor_kernel's tables
+// (mtab; cpg holds c'), streamed through the c' ring in the forward pass, so
+// the recurrence is two multiply-adds a level and writes no c'.
+template <typename R, bool CPG, typename RD = double, bool FAC = false>
+__global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, cplx<RD>* dsc, RD* cpg, ColumnCoef c,
+                                                    const RD* __restrict__ mtab = nullptr) {
+    static_assert(!FAC || CPG, "the factored solve streams c' from its table");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int D = THOMAS_PF;
     cplx<double>* ring = reinterpret_cast<cplx<double>*>(smem_raw);   // [D][32], 16-byte entries
@@ -885,11 +730,47 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, ColumnCoe
     const long long sk = (long long)g.ny * g.sp;
     const int nz = g.nz;
     if (blockIdx.x == 0) {
-        thomas_mean(S, sk, nz, lane, after, c);
+        // the mean mode (_mean_mode!, src/PressureSolvers.jl:780-805), real:
+        // the warp loads the column into shared memory, lane 0 runs the
+        // sums and the double integration in the reference's order, the
+        // warp writes the gauged profile back (the serial loops read shared
+        // memory only)
+        double* sv = after;          // [nz] the column's real parts
+        double* ph = sv + nz;        // [nz] the integrated profile
+        double* me = ph + nz;        // [nz] measures
+        double* io = me + nz;        // [nz + 1] iota
+        double* ga = io + nz + 1;    // [nz] gauge weights
+        for (int k = lane; k < nz; k += 32) {
+            sv[k] = (double)S[k * sk].x;
+            me[k] = c.meas[k];
+            ga[k] = c.gauge[k];
+        }
+        for (int k = lane; k <= nz; k += 32) io[k] = c.iota[k];
+        __syncwarp();
+        if (lane == 0) {
+            double mb = 0.0;
+            for (int k = 0; k < nz; ++k) mb += sv[k] * me[k];
+            mb /= c.meas_sum;
+            double F = 0.0, acc = 0.0, prev = sv[0] - mb;
+            ph[0] = 0.0;
+            for (int k = 1; k < nz; ++k) {
+                F += prev * me[k - 1];
+                acc += F * io[k];
+                prev = sv[k] - mb;
+                ph[k] = acc;
+            }
+            double mp = 0.0;
+            for (int k = 0; k < nz; ++k) mp += ph[k] * ga[k];
+            sv[0] = mp / c.gauge_sum;
+        }
+        __syncwarp();
+        const double sh = sv[0];
+        for (int k = lane; k < nz; k += 32) S[k * sk] = cmk<R>(R(ph[k] - sh), R(0));
         return;
     }
-    double* cp = after;                                 // c': [nz][32]
-    double* s_lo = after + 32 * nz;
+    RD* cring = reinterpret_cast<RD*>(after);           // CPG: [D][32] c' ring
+    double* cp = after;                                 // shared c': [nz][32]
+    double* s_lo = CPG ? after + D * 32 : after + 32 * nz;
     double* s_up = s_lo + nz;
     double* s_hw = s_up + nz;
     // the diagonals' per-level coefficients, staged once
@@ -909,35 +790,51 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, ColumnCoe
     cplx<R>* rs = reinterpret_cast<cplx<R>*>(ring);   // this lane's entries at [slot * 32 + lane]
 #pragma unroll
     for (int q = 0; q < D - 1; ++q) {
-        if (q < nz) thomas_cp<sizeof(cplx<R>)>(rs + q * 32 + lane, S + col + q * sk);
+        if (q < nz) {
+            thomas_cp<sizeof(cplx<R>)>(rs + q * 32 + lane, S + col + q * sk);
+            if (FAC) thomas_cp<sizeof(RD)>(cring + q * 32 + lane, mtab + col + q * sk);
+        }
         thomas_commit();
     }
     double cprev = 0.0, dr = 0.0, di = 0.0;
     for (int k = 0; k < nz; ++k) {
         const int kn = k + D - 1;
-        if (kn < nz) thomas_cp<sizeof(cplx<R>)>(rs + (kn % D) * 32 + lane, S + col + (long long)kn * sk);
+        if (kn < nz) {
+            thomas_cp<sizeof(cplx<R>)>(rs + (kn % D) * 32 + lane, S + col + (long long)kn * sk);
+            if (FAC) thomas_cp<sizeof(RD)>(cring + (kn % D) * 32 + lane, mtab + col + (long long)kn * sk);
+        }
         thomas_commit();
         thomas_wait<D - 1>();   // level k has landed
         const cplx<R> s = rs[(k % D) * 32 + lane];
         const double lo = s_lo[k];
-        const double up = s_up[k];
-        const double b = -(lo + up) - lam * s_hw[k];
-        const double den = b - lo * cprev;
-        const double id = 1.0 / den;
-        cprev = up * id;
+        double id;
+        if constexpr (FAC) {
+            id = (double)cring[(k % D) * 32 + lane];
+        } else {
+            const double up = s_up[k];
+            const double b = -(lo + up) - lam * s_hw[k];
+            const double den = b - lo * cprev;
+            id = 1.0 / den;
+            cprev = up * id;
+        }
         dr = ((double)s.x - lo * dr) * id;   // lo = 0 at k = 0
         di = ((double)s.y - lo * di) * id;
         if (k < nz - 1) {
-            cp[k * 32 + lane] = cprev;
-            S[col + (long long)k * sk] = cmk<R>(R(dr), R(di));
+            if (!FAC) {
+                if (CPG) cpg[col + (long long)k * sk] = RD(cprev);
+                else cp[k * 32 + lane] = cprev;
+            }
+            dsc[col + (long long)k * sk] = cmk<RD>(RD(dr), RD(di));
         }
     }
     thomas_wait<0>();
     S[col + (long long)(nz - 1) * sk] = cmk<R>(R(dr), R(di));
-    // back substitution over k = nz-2 .. 0, the d' values streamed alike (slot t
-    // holds level nz-2-t modulo D)
+    // back substitution over k = nz-2 .. 0, the d' (and c') values streamed
+    // alike (slot t holds level nz-2-t modulo D)
+    cplx<RD>* dring = reinterpret_cast<cplx<RD>*>(ring);
     auto fetch = [&](int slot, int k) {
-        thomas_cp<sizeof(cplx<R>)>(rs + slot * 32 + lane, S + col + (long long)k * sk);
+        thomas_cp<sizeof(cplx<RD>)>(dring + slot * 32 + lane, dsc + col + (long long)k * sk);
+        if (CPG) thomas_cp<sizeof(RD)>(cring + slot * 32 + lane, cpg + col + (long long)k * sk);
     };
 #pragma unroll
     for (int q = 0; q < D - 1; ++q) {
@@ -951,8 +848,8 @@ __global__ void __launch_bounds__(32) thomas_kernel(Geo g, cplx<R>* S, ColumnCoe
         if (kn >= 0) fetch(tn % D, kn);
         thomas_commit();
         thomas_wait<D - 1>();
-        const cplx<R> d = rs[(t % D) * 32 + lane];
-        const double cc = cp[k * 32 + lane];
+        const cplx<RD> d = dring[(t % D) * 32 + lane];
+        const double cc = CPG ? (double)cring[(t % D) * 32 + lane] : cp[k * 32 + lane];
         dr = (double)d.x - cc * dr;
         di = (double)d.y - cc * di;
         S[col + (long long)k * sk] = cmk<R>(R(dr), R(di));

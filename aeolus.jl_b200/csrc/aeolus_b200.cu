@@ -1517,12 +1517,14 @@ struct Core : CoreBase {
                                        (size_t)tpx_z * g.nz * sizeof(cplx<R>), st>>>(g, S, tw, NT, tpx_z, kx2, ky2, kz2, nrm);
             });
         } else {
-            const size_t smt = thomas_tw_smem(g);
-            reg_smem(thomas_tw_kernel<R>, smt);
-            // d in place in S; the factors from the tables made at set-up
-            const R* ftab = reinterpret_cast<const R*>(cps);
+            size_t smt = thomas_smem(g, true);
+            if (smt > 48 * 1024)
+                cudaFuncSetAttribute(thomas_kernel<R, true, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smt);
+            // d' in place in S; the factors m and c' from the tables made at set-up
+            R* ftab = reinterpret_cast<R*>(cps);
             const long long ns = (long long)g.sp * g.ny * g.nz;
-            thomas_tw_kernel<R><<<thomas_blocks(g), 64, smt, st>>>(g, S, cc, ftab, ftab + ns);
+            thomas_kernel<R, true, R, true><<<thomas_blocks(g), 32, smt, st>>>(g, S, S, ftab + ns, cc, ftab);
         }
         CKL();
         mark(AEO_K_ZSOLVE);

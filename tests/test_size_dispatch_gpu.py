@@ -176,59 +176,6 @@ def test_column_solve_of_every_depth(nz, precision, tol):
     assert rel(s.pressure_solve(b), o.pressure_solve(b)) <= tol
 
 
-@pytest.mark.parametrize("nz", [8, 65, 128])
-@pytest.mark.parametrize("precision,eps", [("fp64", 2.0 ** -53), ("fp32_mixed", 2.0 ** -24)])
-def test_column_solve_keeps_the_longest_waves(nz, precision, eps):
-    """Waves of ten thousand depths, whose columns are singular but for lambda h^2 of 1e-10, against an elimination in
-    extended precision that adds positive terms only.  Tolerance: the transforms' eps log2(N) and the column's eps nz
-    of |b|, grown by 1/lambda_min (the 2-norm of the inverse)."""
-    g = regular_grid((16, 8, nz), (1e4, 1e4, 1.0), bc_z="wall")
-    b = np.random.default_rng(nz).standard_normal((nz, 8, 16))
-    b -= b.mean(axis=(1, 2), keepdims=True)
-    ky, kx = (4 / h ** 2 * np.sin(np.pi * np.arange(n) / n) ** 2 for h, n in ((g.dy, 8), (g.dx, 16)))
-    lam = (ky[:, None] + kx[None, :]).astype(np.longdouble)
-    lam[0, 0] = 1.0
-    bh = np.fft.fft2(b).astype(np.clongdouble)
-    far = np.longdouble(1) / np.longdouble(g.dz) ** 2
-    d, c, gam = [], [], np.zeros_like(lam)
-    for k in range(nz):
-        up, lo = (far if k < nz - 1 else 0 * far), (far if k else 0 * far)
-        rest = lam + lo * gam
-        m = -1 / (up + rest)
-        d.append((bh[k] - (lo * d[-1] if k else 0)) * m)
-        c.append(up * m)
-        gam = -rest * m
-    x = [d[-1]]
-    for k in range(nz - 2, -1, -1):
-        x.append(d[k] - c[k] * x[-1])
-    xh = np.array(x[::-1])
-    xh[:, 0, 0] = 0
-    want = np.fft.ifft2(xh.astype(np.complex128)).real
-    got = Sim(CoreSpec(grid=g, precision=precision)).pressure_solve(b)
-    got = got - got.mean(axis=(1, 2), keepdims=True)
-    low = float(min(lam.ravel()[1:]))
-    bound = (2 * np.log2(g.ncells) + nz) * eps * np.linalg.norm(b) / (low * np.linalg.norm(want))
-    assert rel(got, want) <= bound
-
-
-@pytest.mark.parametrize("steps", [1, 2, 3, 5])
-def test_a_run_of_steps_is_its_single_steps(steps):
-    """Direct solvers launch a graph a step, the PCG solver a graph of pairs: both are the single steps' bits."""
-    g = regular_grid((16, 16, 8), (1.0, 1.0, 1.0), bc_z="wall")
-    for kw in ({}, {"precision": "fp32_mixed"}, {"solver": "pcg"}):
-        out = []
-        for calls in ([steps], [1] * steps):
-            s = Sim(CoreSpec(grid=g, nu=1e-3, **kw))
-            if "solver" in kw:
-                s.set_pcg(None, tol=1e-8, maxit=100)
-            s.set_state(*random_state(g, 9, 0.3))
-            s.project()
-            for n in calls:
-                s.step_rk3(1e-3, n)
-            out.append([s.get_field(n) for n in ("u", "v", "w", "theta", "p")])
-        assert all(np.array_equal(a, b) for a, b in zip(*out))
-
-
 # ---- the centred sweeps: persistent CTAs over (tile, level) items, 64 (FP32) or 32 (FP64) columns by 8 rows -----
 @pytest.mark.parametrize("size,wall", [((8, 4, 5), True), ((32, 8, 4), False), ((64, 16, 13), True), ((128, 4, 33), True),
                                        ((32, 32, 64), False)])
