@@ -365,3 +365,21 @@ def test_host_arrays_pageable_pinned_and_from_threads(shape):
     for t in th:
         t.join()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 5])
+def test_a_run_of_steps_is_its_single_steps(steps):
+    """Direct solvers launch a graph a step, the PCG solver a graph of pairs: both are the single steps' bits."""
+    g = regular_grid((16, 16, 8), (1.0, 1.0, 1.0), bc_z="wall")
+    for kw in ({}, {"precision": "fp32_mixed"}, {"solver": "pcg"}):
+        out = []
+        for calls in ([steps], [1] * steps):
+            s = Sim(CoreSpec(grid=g, nu=1e-3, **kw))
+            if "solver" in kw:
+                s.set_pcg(None, tol=1e-8, maxit=100)
+            s.set_state(*random_state(g, 9, 0.3))
+            s.project()
+            for n in calls:
+                s.step_rk3(1e-3, n)
+            out.append([s.get_field(n) for n in ("u", "v", "w", "theta", "p")])
+        assert all(np.array_equal(a, b) for a, b in zip(*out))
