@@ -1386,8 +1386,8 @@ struct Core : CoreBase {
                 SweepArgs<R> b = a;
                 using PS = PairShape<R, SG>;
                 using TS = TileShape<R, ADV, SG>;
-                if constexpr (ADV == 0 && (!kap || PS::KAPPA)) {
-                    // centred, persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
+                if constexpr (ADV == 0 && sizeof(R) == sizeof(float)) {
+                    // centred FP32 (FP64 here moved the stretched layer's pressure by 3.5e-12), persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
                     const int ntx = (g.nx + PS::TX - 1) / PS::TX, nty = (g.ny + PS::TY - 1) / PS::TY;
                     const int items = ntx * nty * g.nz;
                     const dim3 grid((unsigned)std::min(items, PS::CTAS_PER_SM * nsm));
