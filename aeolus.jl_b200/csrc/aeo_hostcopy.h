@@ -7,14 +7,20 @@
 // rate and overlaps the link.  Arrays that are small or already pinned take the
 // plain call.
 //
-// The pinned buffers (LANES x 2 x CHUNK, 12 MiB) belong to the live handles
-// together: the first one allocates them, the last one gives them back, and a
-// mutex lets one copy at a time use them.
+// The pinned buffers (LANES x 2 x CHUNK, 12 MiB) belong together to the live handles
+// that have use for them: the first such handle pins them, the last one gives them back,
+// and a mutex lets one copy at a time use them.  Pinning huge pages and giving them back
+// takes 3.0 ms (7.2 ms by cudaHostAlloc), what the lanes save on PAYS bytes (6.3 MB go up
+// in 0.59 ms and down in 0.40 ms by the plain call); a handle asks for them once its
+// pageable copies come to that much.  So creating a handle pins nothing, one that copies
+// little pays for nothing, and where pinned memory is refused the plain call serves.
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -24,35 +30,12 @@
 
 class HostStage {
 public:
-    static constexpr size_t CHUNK = size_t(1) << 20, SMALL = size_t(2) << 20;
+    static constexpr size_t CHUNK = size_t(1) << 20, SMALL = size_t(2) << 20, PAYS = size_t(40) << 20;
     static constexpr int LANES = 6;
 
-    // the live handles' buffers
-    static std::shared_ptr<HostStage> get(cudaError_t* e) {
-        static std::mutex m;
-        static std::weak_ptr<HostStage> live;
-        std::lock_guard<std::mutex> lock(m);
-        *e = cudaSuccess;
-        std::shared_ptr<HostStage> s = live.lock();
-        if (s) return s;
-        try {
-            s = std::make_shared<HostStage>();
-        } catch (const std::bad_alloc&) {
-            *e = cudaErrorMemoryAllocation;
-            return nullptr;
-        }
-        *e = cudaHostAlloc(reinterpret_cast<void**>(&s->pin_), LANES * 2 * CHUNK, cudaHostAllocPortable);
-        if (*e != cudaSuccess) { s->pin_ = nullptr; return nullptr; }
-        live = s;
-        return s;
-    }
-    ~HostStage() {
-        if (pin_) cudaFreeHost(pin_);
-    }
-
-    // src (host) -> dst (device) on st; returns when src has been read
+    // src (host) -> dst (device) on st; returns when a pageable src has been read
     cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
-        if (bytes < SMALL || pinned(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        if (bytes < SMALL || pinned(src) || !buffers(bytes)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
         return lanes(bytes, device, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
             std::memcpy(pin, static_cast<const char*>(src) + at, n);
             cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + at, pin, n, cudaMemcpyHostToDevice, st);
@@ -61,7 +44,7 @@ public:
     }
     // src (device) -> dst (host), ordered on st; returns when dst is complete
     cudaError_t download(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
-        if (bytes < SMALL || pinned(dst)) {
+        if (bytes < SMALL || pinned(dst) || !buffers(bytes)) {
             cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
             return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
         }
@@ -72,8 +55,53 @@ public:
     }
 
 private:
-    char* pin_ = nullptr;
-    std::mutex use_;
+    struct Buffers {
+        char* pin = nullptr;
+        std::mutex use;
+        ~Buffers() {
+            if (!pin) return;
+            cudaHostUnregister(pin);
+            std::free(pin);
+        }
+    };
+    std::shared_ptr<Buffers> buf_;
+    size_t plain_ = 0;   // bytes of this handle's pageable copies so far
+
+    // the live handles' buffers, where there are none made if `make`; null without, or where pinned
+    // memory is refused
+    static std::shared_ptr<Buffers> shared(bool make) {
+        static std::mutex m;
+        static std::weak_ptr<Buffers> live;
+        std::lock_guard<std::mutex> lock(m);
+        std::shared_ptr<Buffers> s = live.lock();
+        if (s || !make) return s;
+        try {
+            s = std::make_shared<Buffers>();
+        } catch (const std::bad_alloc&) {
+            return nullptr;
+        }
+        const size_t n = LANES * 2 * CHUNK;
+        void* p = std::aligned_alloc(size_t(2) << 20, n);
+        if (!p) return nullptr;
+        madvise(p, n, MADV_HUGEPAGE);
+        if (cudaHostRegister(p, n, cudaHostRegisterPortable) != cudaSuccess) {
+            cudaGetLastError();
+            std::free(p);
+            return nullptr;
+        }
+        s->pin = static_cast<char*>(p);
+        live = s;
+        return s;
+    }
+    // whether this copy takes the lanes (after a refusal the count starts again)
+    bool buffers(size_t bytes) {
+        if (buf_) return true;
+        plain_ += bytes;
+        const bool make = plain_ >= PAYS;
+        if (make) plain_ = 0;
+        buf_ = shared(make);
+        return buf_ != nullptr;
+    }
 
     static bool pinned(const void* p) {
         cudaPointerAttributes a{};
@@ -86,7 +114,7 @@ private:
     // passed, before the buffer's next chunk and at the end.
     template <class Go, class Done>
     cudaError_t lanes(size_t bytes, int device, Go go, Done done) {
-        std::lock_guard<std::mutex> lock(use_);
+        std::lock_guard<std::mutex> lock(buf_->use);
         const size_t nc = (bytes + CHUNK - 1) / CHUNK;
         const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
         const int nl = (int)std::min<size_t>(nc, (size_t)std::min(LANES, std::max(1, hw / 2)));
@@ -100,7 +128,7 @@ private:
                 if (held[b] == nc) return;
                 if (e == cudaSuccess) e = cudaEventSynchronize(ev[b]);
                 const size_t at = held[b] * CHUNK;
-                if (e == cudaSuccess) done(pin_ + (size_t)(2 * l + b) * CHUNK, at, std::min(CHUNK, bytes - at));
+                if (e == cudaSuccess) done(buf_->pin + (size_t)(2 * l + b) * CHUNK, at, std::min(CHUNK, bytes - at));
                 held[b] = nc;
             };
             int b = 0;
@@ -108,7 +136,7 @@ private:
                 finish(b);
                 if (e != cudaSuccess) break;
                 const size_t at = c * CHUNK;
-                e = go(pin_ + (size_t)(2 * l + b) * CHUNK, at, std::min(CHUNK, bytes - at), ev[b]);
+                e = go(buf_->pin + (size_t)(2 * l + b) * CHUNK, at, std::min(CHUNK, bytes - at), ev[b]);
                 if (e == cudaSuccess) held[b] = c;
             }
             finish(b);

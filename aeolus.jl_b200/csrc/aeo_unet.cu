@@ -114,7 +114,7 @@ struct aeo_unet {
     double* rbuf = nullptr;             // device residual / target for host-array calls
     double* ebuf = nullptr;
     int* derr = nullptr;
-    std::shared_ptr<HostStage> stage;   // the pageable host arrays' way to the device
+    HostStage stage;                    // the pageable host arrays' way to the device
     cudaStream_t st_up = nullptr;       // the target's upload, beside the forward pass
     cudaEvent_t ev_free = nullptr, ev_up = nullptr;
 
@@ -142,9 +142,6 @@ struct aeo_unet {
         CK(cudaStreamCreateWithFlags(&st_up, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&ev_free, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&ev_up, cudaEventDisableTiming));
-        cudaError_t se = cudaSuccess;
-        stage = HostStage::get(&se);
-        CK(se);
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         for (int l = 0; l < 3; ++l) {
             const int f = 1 << l;
@@ -548,12 +545,12 @@ aeo_status aeo_unet_apply(aeo_unet* h, const double* r, double* z) {
     if (!r || !z) { h->err = "r and z must not be NULL"; return AEO_ERR_ARGUMENT; }
     std::string& err = h->err;
     const size_t bytes = sizeof(double) * (size_t)h->n[0];
-    CK(h->stage->upload(h->rbuf, r, bytes, h->device, h->st));
+    CK(h->stage.upload(h->rbuf, r, bytes, h->device, h->st));
     if (aeo_status s = h->forward_(h->rbuf)) return s;
     un::widen_kernel<<<grid_for(h->n[0]), 256, 0, h->st>>>(h->z, h->ebuf, h->n[0]);
     CKL();
     if (aeo_status s = h->check_err()) return s;
-    CK(h->stage->download(z, h->ebuf, bytes, h->device, h->st));
+    CK(h->stage.download(z, h->ebuf, bytes, h->device, h->st));
     return AEO_OK;
 }
 
@@ -566,9 +563,9 @@ aeo_status aeo_unet_gradients(aeo_unet* h, const double* r, const double* e, dou
     // the target goes up beside the forward pass, which does not read it
     CK(cudaEventRecord(h->ev_free, h->st));
     CK(cudaStreamWaitEvent(h->st_up, h->ev_free, 0));
-    CK(h->stage->upload(h->rbuf, r, bytes, h->device, h->st));
+    CK(h->stage.upload(h->rbuf, r, bytes, h->device, h->st));
     if (aeo_status s = h->forward_(h->rbuf)) return s;
-    CK(h->stage->upload(h->ebuf, e, bytes, h->device, h->st_up));
+    CK(h->stage.upload(h->ebuf, e, bytes, h->device, h->st_up));
     CK(cudaEventRecord(h->ev_up, h->st_up));
     CK(cudaStreamWaitEvent(h->st, h->ev_up, 0));
     if (aeo_status s = h->backward(h->ebuf)) return s;

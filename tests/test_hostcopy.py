@@ -1,0 +1,181 @@
+"""The pageable arrays' copies (aeo_hostcopy.h) on the host, against a stand-in of the CUDA runtime whose transfers
+run only when something waits for them, and which refuses or fails calls on demand."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "aeolus.jl_b200", "csrc")
+
+RUNTIME = r"""
+#pragma once
+#include <condition_variable>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <mutex>
+#include <vector>
+enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorUnknown = 999 };
+enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+enum { cudaHostRegisterPortable = 1, cudaEventDisableTiming = 2 };
+enum cudaMemoryType { cudaMemoryTypeUnregistered = 0, cudaMemoryTypeHost = 1 };
+struct cudaPointerAttributes { cudaMemoryType type; };
+
+namespace fake {
+struct Transfer { void* dst; const void* src; size_t n; bool done = false; };
+struct Stream { std::vector<Transfer> queue; };
+struct Event { Stream* s = nullptr; size_t upto = 0; };
+inline std::mutex m;
+inline char* pin = nullptr;
+inline size_t pin_bytes = 0;
+inline int allocs = 0, frees = 0, copies = 0, plain = 0, records = 0;
+inline bool refuse = false;
+inline int fail_copy = -1, fail_record = -1, fail_create = -1, creates = 0;
+inline std::function<void()> at_wait;
+inline bool of_pin(const void* p) { return pin && p >= pin && p < pin + pin_bytes; }
+inline void run(Stream* s, size_t upto) {
+    for (size_t q = 0; q < upto; ++q) {
+        Transfer& t = s->queue[q];
+        if (!t.done) { std::memcpy(t.dst, t.src, t.n); t.done = true; }
+    }
+}
+inline int in_flight(Stream* s) {
+    int n = 0;
+    for (auto& t : s->queue) n += !t.done && (of_pin(t.src) || of_pin(t.dst));
+    return n;
+}
+}  // namespace fake
+typedef fake::Stream* cudaStream_t;
+typedef fake::Event* cudaEvent_t;
+
+inline cudaError_t cudaGetLastError() { return cudaSuccess; }
+inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+inline cudaError_t cudaHostRegister(void* p, size_t n, unsigned) {
+    std::lock_guard<std::mutex> l(fake::m);
+    if (fake::refuse) return cudaErrorMemoryAllocation;
+    ++fake::allocs;
+    fake::pin = static_cast<char*>(p);
+    fake::pin_bytes = n;
+    return cudaSuccess;
+}
+inline cudaError_t cudaHostUnregister(void*) {
+    std::lock_guard<std::mutex> l(fake::m);
+    ++fake::frees;
+    fake::pin = nullptr;
+    return cudaSuccess;
+}
+inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+    a->type = cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+// a pageable copy has read its source (or, to the host, is complete) when it returns; a pinned one is only queued
+inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+    std::lock_guard<std::mutex> l(fake::m);
+    if (fake::copies++ == fake::fail_copy) return cudaErrorUnknown;
+    st->queue.push_back({d, s, n});
+    if (!fake::of_pin(d) && !fake::of_pin(s)) {
+        ++fake::plain;
+        fake::run(st, st->queue.size());
+    }
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    std::lock_guard<std::mutex> l(fake::m);
+    if (fake::creates++ == fake::fail_create) return cudaErrorUnknown;
+    *e = new fake::Event;
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
+inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    std::lock_guard<std::mutex> l(fake::m);
+    if (fake::records++ == fake::fail_record) return cudaErrorUnknown;
+    e->s = s;
+    e->upto = s->queue.size();
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    if (fake::at_wait) fake::at_wait();
+    std::lock_guard<std::mutex> l(fake::m);
+    fake::run(e->s, e->upto);
+    return cudaSuccess;
+}
+inline cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    std::lock_guard<std::mutex> l(fake::m);
+    fake::run(s, s->queue.size());
+    return cudaSuccess;
+}
+"""
+
+HEAD = r"""
+#include "cuda_runtime.h"
+#include "aeo_hostcopy.h"
+#include <chrono>
+#include <cstdio>
+#include <future>
+#include <atomic>
+#define REQUIRE(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::_Exit(1); } } while (0)
+const size_t MB = size_t(1) << 20;
+std::vector<char> bytes(size_t n, int seed) {
+    std::vector<char> a(n);
+    unsigned x = 2463534242u + seed;
+    for (auto& c : a) { x ^= x << 13; x ^= x >> 17; x ^= x << 5; c = (char)x; }
+    return a;
+}
+"""
+
+PROGRAMS = {
+    # a handle pins nothing until its pageable copies have paid for the buffers; the last one gives them back
+    "kept": r"""
+int main() {
+    fake::Stream st;
+    auto a = bytes(HostStage::PAYS + 12345, 1);
+    std::vector<char> d(a.size()), b(a.size());
+    {
+        HostStage one, two;
+        REQUIRE(fake::allocs == 0);
+        const size_t small = HostStage::SMALL - 1, half = HostStage::PAYS / 2;
+        for (int q = 0; q < 50; ++q) REQUIRE(one.upload(d.data(), a.data(), small, 0, &st) == cudaSuccess);
+        REQUIRE(one.upload(d.data(), a.data(), half, 0, &st) == cudaSuccess && fake::allocs == 0);
+        REQUIRE(one.upload(d.data(), a.data(), half, 0, &st) == cudaSuccess && fake::allocs == 1);
+        const int plain = fake::plain;
+        REQUIRE(one.upload(d.data(), a.data(), a.size(), 0, &st) == cudaSuccess);
+        REQUIRE(two.download(b.data(), d.data(), a.size(), 0, &st) == cudaSuccess);
+        REQUIRE(b == a && fake::allocs == 1 && fake::plain == plain && fake::in_flight(&st) == 0);
+    }
+    REQUIRE(fake::frees == 1);
+    HostStage three;   // a first array of that size is worth them at once
+    REQUIRE(three.download(b.data(), d.data(), a.size(), 0, &st) == cudaSuccess && fake::allocs == 2);
+}
+""",
+    # where pinned memory is refused the copies still work
+    "refused": r"""
+int main() {
+    fake::Stream st;
+    fake::refuse = true;
+    auto a = bytes(HostStage::PAYS + 1, 2);
+    std::vector<char> d(a.size()), b(a.size());
+    HostStage s;
+    for (int q = 0; q < 3; ++q) {
+        REQUIRE(s.upload(d.data(), a.data(), a.size(), 0, &st) == cudaSuccess);
+        REQUIRE(s.download(b.data(), d.data(), a.size(), 0, &st) == cudaSuccess);
+    }
+    REQUIRE(b == a && fake::allocs == 0);
+    fake::refuse = false;
+    REQUIRE(s.upload(d.data(), a.data(), a.size(), 0, &st) == cudaSuccess && fake::allocs == 1);
+}
+""",
+}
+
+
+@pytest.mark.parametrize("name", sorted(PROGRAMS))
+def test_host_copy(tmp_path, name):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    (tmp_path / "cuda_runtime.h").write_text(RUNTIME)
+    (tmp_path / "main.cpp").write_text(HEAD + PROGRAMS[name])
+    exe = str(tmp_path / "main")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(tmp_path), "-I", CSRC, "-o", exe,
+                    str(tmp_path / "main.cpp")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

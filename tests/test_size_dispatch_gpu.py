@@ -335,8 +335,8 @@ def test_unet_gradients_where_every_level_takes_x_segments(shape):
 
 @pytest.mark.parametrize("shape", [(128, 16, 8), (128, 64, 32), (128, 48, 44), (256, 64, 56)])
 def test_host_arrays_pageable_pinned_and_from_threads(shape):
-    """Below and above the size that takes the pinned lanes, whole and ragged chunks: the same bits as from pinned
-    arrays, and from several handles at once."""
+    """Below and above the size that takes the pinned lanes, whole and ragged chunks, as often as it takes until a
+    handle uses the lanes: the same bits as from pinned arrays, and from several handles at once."""
     import threading
     import torch
     from aeolus_b200.unet import UNet
@@ -356,8 +356,9 @@ def test_host_arrays_pageable_pinned_and_from_threads(shape):
     got = [None] * 3
 
     def work(q):
-        for _ in range(3):
+        for _ in range(3 + (40 << 20) // (2 * rs[q].nbytes)):   # the lanes' buffers are worth 40 MiB of plain copies
             got[q] = np.array(nets[q].apply(rs[q]))
+            assert np.array_equal(got[q], want[q])
 
     th = [threading.Thread(target=work, args=(q,)) for q in range(3)]
     for t in th:
