@@ -36,7 +36,7 @@ public:
     // src (host) -> dst (device) on st; returns when a pageable src has been read
     cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
         if (bytes < SMALL || pinned(src) || !buffers(bytes)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-        return lanes(bytes, device, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
+        return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
             std::memcpy(pin, static_cast<const char*>(src) + at, n);
             cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + at, pin, n, cudaMemcpyHostToDevice, st);
             return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
@@ -48,7 +48,7 @@ public:
             cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
             return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
         }
-        return lanes(bytes, device, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
+        return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
             cudaError_t e = cudaMemcpyAsync(pin, static_cast<const char*>(src) + at, n, cudaMemcpyDeviceToHost, st);
             return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
         }, [=](char* pin, size_t at, size_t n) { std::memcpy(static_cast<char*>(dst) + at, pin, n); });
@@ -111,9 +111,10 @@ private:
 
     // Lane l takes the chunks l, l + nl, ... through its two buffers: go(buffer, offset,
     // bytes, event) starts a chunk, done(buffer, offset, bytes) runs once its event has
-    // passed, before the buffer's next chunk and at the end.
+    // passed, before the buffer's next chunk and at the end.  After an error what was already
+    // enqueued on st is waited for: the buffers are the next copy's.
     template <class Go, class Done>
-    cudaError_t lanes(size_t bytes, int device, Go go, Done done) {
+    cudaError_t lanes(size_t bytes, int device, cudaStream_t st, Go go, Done done) {
         std::lock_guard<std::mutex> lock(buf_->use);
         const size_t nc = (bytes + CHUNK - 1) / CHUNK;
         const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
@@ -157,7 +158,10 @@ private:
         for (int l = 1; l < nl; ++l)
             if (th[l].joinable()) th[l].join();
         for (int l = 0; l < nl; ++l)
-            if (err[l] != cudaSuccess) return err[l];
+            if (err[l] != cudaSuccess) {
+                cudaStreamSynchronize(st);
+                return err[l];
+            }
         return cudaSuccess;
     }
 };

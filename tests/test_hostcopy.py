@@ -114,8 +114,9 @@ HEAD = r"""
 #include <cstdio>
 #include <future>
 #include <atomic>
-#define REQUIRE(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::_Exit(1); } } while (0)
-const size_t MB = size_t(1) << 20;
+#define REQUIRE(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::fflush(stdout); std::_Exit(1); } } while (0)
+// in the place of the library's: one lane, or all of them
+unsigned std::thread::hardware_concurrency() noexcept { return CORES; }
 std::vector<char> bytes(size_t n, int seed) {
     std::vector<char> a(n);
     unsigned x = 2463534242u + seed;
@@ -148,6 +149,31 @@ int main() {
     REQUIRE(three.download(b.data(), d.data(), a.size(), 0, &st) == cudaSuccess && fake::allocs == 2);
 }
 """,
+    # a call that fails leaves no transfer under way through the buffers, which the next copy uses (on one core too,
+    # where one thread has all chunks and no other one waits for them)
+    "failed": r"""
+int main() {
+    auto a = bytes(HostStage::PAYS + 4321, 3);
+    std::vector<char> d(a.size()), b(a.size());
+    HostStage keep;
+    fake::Stream st;
+    REQUIRE(keep.upload(d.data(), a.data(), a.size(), 0, &st) == cudaSuccess && fake::allocs == 1);
+    for (int which = 0; which < 3; ++which)
+        for (int at : {0, 1, 5, 11, 20})
+            for (bool up : {true, false}) {
+                fake::Stream s1;
+                if (which == 0) fake::fail_copy = fake::copies + at;
+                if (which == 1) fake::fail_record = fake::records + at;
+                if (which == 2) fake::fail_create = fake::creates + (at & 1);
+                cudaError_t e = up ? keep.upload(d.data(), a.data(), a.size(), 0, &s1) : keep.download(b.data(), d.data(), a.size(), 0, &s1);
+                REQUIRE(e == cudaErrorUnknown);
+                REQUIRE(fake::in_flight(&s1) == 0);
+                fake::fail_copy = fake::fail_record = fake::fail_create = -1;
+                REQUIRE(keep.upload(d.data(), a.data(), a.size(), 0, &s1) == cudaSuccess);
+                REQUIRE(keep.download(b.data(), d.data(), a.size(), 0, &s1) == cudaSuccess && b == a);
+            }
+}
+""",
     # where pinned memory is refused the copies still work
     "refused": r"""
 int main() {
@@ -168,14 +194,15 @@ int main() {
 }
 
 
+@pytest.mark.parametrize("cores", [1, 12])
 @pytest.mark.parametrize("name", sorted(PROGRAMS))
-def test_host_copy(tmp_path, name):
+def test_host_copy(tmp_path, name, cores):
     if shutil.which("g++") is None:
         pytest.skip("no host compiler")
     (tmp_path / "cuda_runtime.h").write_text(RUNTIME)
     (tmp_path / "main.cpp").write_text(HEAD + PROGRAMS[name])
     exe = str(tmp_path / "main")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(tmp_path), "-I", CSRC, "-o", exe,
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", f"-DCORES={cores}", "-I", str(tmp_path), "-I", CSRC, "-o", exe,
                     str(tmp_path / "main.cpp")], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
