@@ -9,11 +9,12 @@
 //
 // The pinned buffers (LANES x 2 x CHUNK, 12 MiB) belong together to the live handles
 // that have use for them: the first such handle pins them, the last one gives them back,
-// and a mutex lets one copy at a time use them.  Pinning huge pages and giving them back
-// takes 3.0 ms (7.2 ms by cudaHostAlloc), what the lanes save on PAYS bytes (6.3 MB go up
-// in 0.59 ms and down in 0.40 ms by the plain call); a handle asks for them once its
-// pageable copies come to that much.  So creating a handle pins nothing, one that copies
-// little pays for nothing, and where pinned memory is refused the plain call serves.
+// and one copy at a time uses them (a copy that finds them in use goes the plain way).
+// Pinning huge pages and giving them back takes 3.0 ms (7.2 ms by cudaHostAlloc), what the
+// lanes save on PAYS bytes (6.3 MB go up in 0.59 ms and down in 0.40 ms by the plain call);
+// a handle asks for them once its pageable copies come to that much.  So creating a handle
+// pins nothing, one that copies little pays for nothing, and where pinned memory is refused
+// the plain call serves.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,23 +36,23 @@ public:
 
     // src (host) -> dst (device) on st; returns when a pageable src has been read
     cudaError_t upload(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
-        if (bytes < SMALL || pinned(src) || !buffers(bytes)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-        return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
-            std::memcpy(pin, static_cast<const char*>(src) + at, n);
-            cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + at, pin, n, cudaMemcpyHostToDevice, st);
-            return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
-        }, [](char*, size_t, size_t) {});
+        if (Turn turn{*this, src, bytes})
+            return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
+                std::memcpy(pin, static_cast<const char*>(src) + at, n);
+                cudaError_t e = cudaMemcpyAsync(static_cast<char*>(dst) + at, pin, n, cudaMemcpyHostToDevice, st);
+                return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
+            }, [](char*, size_t, size_t) {});
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
     }
     // src (device) -> dst (host), ordered on st; returns when dst is complete
     cudaError_t download(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
-        if (bytes < SMALL || pinned(dst) || !buffers(bytes)) {
-            cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
-            return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-        }
-        return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
-            cudaError_t e = cudaMemcpyAsync(pin, static_cast<const char*>(src) + at, n, cudaMemcpyDeviceToHost, st);
-            return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
-        }, [=](char* pin, size_t at, size_t n) { std::memcpy(static_cast<char*>(dst) + at, pin, n); });
+        if (Turn turn{*this, dst, bytes})
+            return lanes(bytes, device, st, [=](char* pin, size_t at, size_t n, cudaEvent_t ev) -> cudaError_t {
+                cudaError_t e = cudaMemcpyAsync(pin, static_cast<const char*>(src) + at, n, cudaMemcpyDeviceToHost, st);
+                return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
+            }, [=](char* pin, size_t at, size_t n) { std::memcpy(static_cast<char*>(dst) + at, pin, n); });
+        cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
     }
 
 private:
@@ -103,6 +104,16 @@ private:
         return buf_ != nullptr;
     }
 
+    // Whether a copy of the host array at p has the buffers: held while it runs, never waited for (another copy,
+    // of another device perhaps, has them: the plain call is no slower than waiting).
+    struct Turn {
+        std::unique_lock<std::mutex> lock;
+        Turn(HostStage& s, const void* p, size_t bytes) {
+            if (bytes >= SMALL && !pinned(p) && s.buffers(bytes)) lock = std::unique_lock<std::mutex>(s.buf_->use, std::try_to_lock);
+        }
+        explicit operator bool() const { return lock.owns_lock(); }
+    };
+
     static bool pinned(const void* p) {
         cudaPointerAttributes a{};
         if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
@@ -115,7 +126,6 @@ private:
     // enqueued on st is waited for: the buffers are the next copy's.
     template <class Go, class Done>
     cudaError_t lanes(size_t bytes, int device, cudaStream_t st, Go go, Done done) {
-        std::lock_guard<std::mutex> lock(buf_->use);
         const size_t nc = (bytes + CHUNK - 1) / CHUNK;
         const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
         const int nl = (int)std::min<size_t>(nc, (size_t)std::min(LANES, std::max(1, hw / 2)));

@@ -174,6 +174,31 @@ int main() {
             }
 }
 """,
+    # while one copy has the buffers, another handle's goes the plain way and does not wait for it
+    "busy": r"""
+int main() {
+    fake::Stream s1, s2;
+    auto a = bytes(HostStage::PAYS, 4), b = bytes(HostStage::PAYS, 5);
+    std::vector<char> da(a.size()), db(a.size()), back(a.size());
+    HostStage one, two;
+    REQUIRE(one.upload(da.data(), a.data(), a.size(), 0, &s1) == cudaSuccess);
+    REQUIRE(two.upload(db.data(), b.data(), b.size(), 0, &s2) == cudaSuccess && fake::allocs == 1);
+    std::promise<void> go;
+    auto gate = go.get_future().share();
+    std::atomic<int> held{0};
+    fake::at_wait = [&] { ++held; gate.wait(); };
+    auto first = std::async(std::launch::async, [&] { return one.upload(da.data(), a.data(), a.size(), 0, &s1); });
+    while (!held) std::this_thread::yield();
+    std::fill(db.begin(), db.end(), 0);
+    auto second = std::async(std::launch::async, [&] {
+        cudaError_t e = two.upload(db.data(), b.data(), b.size(), 0, &s2);
+        return e == cudaSuccess ? two.download(back.data(), db.data(), b.size(), 0, &s2) : e;
+    });
+    const bool through = second.wait_for(std::chrono::seconds(20)) == std::future_status::ready;
+    go.set_value();
+    REQUIRE(through && first.get() == cudaSuccess && second.get() == cudaSuccess && da == a && back == b);
+}
+""",
     # where pinned memory is refused the copies still work
     "refused": r"""
 int main() {
