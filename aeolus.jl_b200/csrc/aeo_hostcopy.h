@@ -23,10 +23,10 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 
 class HostStage {
@@ -160,8 +160,8 @@ private:
         for (int l = 1; l < nl; ++l) {
             try {
                 th[l] = std::thread(lane, l);
-            } catch (const std::system_error&) {
-                lane(l);   // no thread to be had: this one does the lane's chunks
+            } catch (const std::exception&) {
+                lane(l);   // no thread (or no memory for one) to be had: this one does the lane's chunks
             }
         }
         lane(0);

@@ -15,6 +15,7 @@ RUNTIME = r"""
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <new>
 #include <vector>
 enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorUnknown = 999 };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
@@ -83,10 +84,10 @@ inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyK
 inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     std::lock_guard<std::mutex> l(fake::m);
     if (fake::creates++ == fake::fail_create) return cudaErrorUnknown;
-    *e = new fake::Event;
+    *e = new (std::malloc(sizeof(fake::Event))) fake::Event;
     return cudaSuccess;
 }
-inline cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; return cudaSuccess; }
+inline cudaError_t cudaEventDestroy(cudaEvent_t e) { std::free(e); return cudaSuccess; }
 inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
     std::lock_guard<std::mutex> l(fake::m);
     if (fake::records++ == fake::fail_record) return cudaErrorUnknown;
@@ -197,6 +198,30 @@ int main() {
     const bool through = second.wait_for(std::chrono::seconds(20)) == std::future_status::ready;
     go.set_value();
     REQUIRE(through && first.get() == cudaSuccess && second.get() == cudaSuccess && da == a && back == b);
+}
+""",
+    # a lane whose thread cannot be had, for want of threads or of memory, runs on the calling one
+    "threads": r"""
+thread_local bool starved = false;
+void* operator new(size_t n) {
+    void* p = starved ? nullptr : std::malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+int main() {
+    fake::Stream st;
+    st.queue.reserve(1 << 12);
+    auto a = bytes(HostStage::PAYS + 99, 6);
+    std::vector<char> d(a.size()), b(a.size());
+    HostStage s;
+    REQUIRE(s.upload(d.data(), a.data(), a.size(), 0, &st) == cudaSuccess);
+    std::fill(d.begin(), d.end(), 0);
+    starved = true;
+    const cudaError_t up = s.upload(d.data(), a.data(), a.size(), 0, &st), down = s.download(b.data(), d.data(), a.size(), 0, &st);
+    starved = false;
+    REQUIRE(up == cudaSuccess && down == cudaSuccess && b == a);
 }
 """,
     # where pinned memory is refused the copies still work
