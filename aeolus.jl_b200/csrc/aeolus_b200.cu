@@ -96,10 +96,9 @@ struct CoreBase {
     std::string err;
     cudaStream_t st = nullptr;
     Geo g{};
-    int launches = 0;
     virtual ~CoreBase() {}
     // kernels of one RK3 step (solver = PCG: with the last solve's iteration count)
-    virtual int step_launches() { return launches; }
+    virtual aeo_status step_launches(int* out) = 0;
     void fail(const std::string& m) { err = m; }
     virtual aeo_status init(const double* zf, const double* wc, const double* wf, const double* thf) = 0;
     virtual aeo_status set_field(int id, const double* host) = 0;
@@ -221,7 +220,7 @@ struct Core : CoreBase {
     double* d_dynpart = nullptr;
     int dyn_nb = 0;
     double dyn_d2 = 0.0;   // Delta^2 = (dx dy dz)^(2/3)
-    // the kernels of the dynamic coefficient of the state in `in` (3 launches)
+    // the kernels of the dynamic coefficient of the state in `in`
     aeo_status enqueue_dynamic(R* const* in) {
         const long long ns = (long long)dws.sx * dws.sy * (g.nz + 2);
         germano_pass1_kernel<R><<<(unsigned)std::min<long long>((ns + 255) / 256, 148LL * 16), 256, 0, st>>>(
@@ -242,7 +241,6 @@ struct Core : CoreBase {
         CKL();
         return AEO_OK;
     }
-    int dyn_launches() const { return dyn() ? 3 : 0; }
     // the Lagrangian closure: its memories (two sets, LagArgs), the committed
     // set and initialised flag on the device (and a copy of them taken before
     // an adaptive step, put back when the step is retried), C0, theta, the
@@ -250,7 +248,6 @@ struct Core : CoreBase {
     LagArgs<R> lagA{};
     int* d_lag_state = nullptr;
     double lag_c0 = 0.16, lag_theta = 1.5, lag_mt = 0.0;
-    int lag_launches() const { return lag() ? 4 : 0; }   // per step
     // advance_sgs! of the state in `in` (halos filled): passes 1 and 2 with
     // the memory update, the coefficient's halos, the flip
     aeo_status enqueue_lag_commit(R* const* in) {
@@ -332,7 +329,6 @@ struct Core : CoreBase {
     // return to, the coefficients
     R *d_tke = nullptr, *d_tk2 = nullptr, *d_tkt = nullptr, *d_tke_keep = nullptr;
     TkeArgs tkeA{};
-    int tke_launches() const { return tke() ? 8 : 0; }   // per step
     aeo_status set_tke(double c_eps0, double c_eps1, double c_l, int exact) override {
         if (!tke()) { fail("set_tke: the domain's closure is not the TKE closure"); return AEO_ERR_STATE; }
         if (!(c_eps0 >= 0) || !(c_eps1 >= 0) || !(c_l > 0) || !std::isfinite(c_eps0) || !std::isfinite(c_eps1) ||
@@ -812,7 +808,6 @@ struct Core : CoreBase {
             wchunk = chunk(WPairShape::TX, WPairShape::TY, WPairShape::CTAS_PER_SM * nsm, 64, 6);
         }
         CK(cudaStreamSynchronize(st));
-        launches = 3 * (9 + dyn_launches()) + lag_launches() + tke_launches();
         return AEO_OK;
     }
 
@@ -906,12 +901,40 @@ struct Core : CoreBase {
         return make_pcg(ax, ay, az);
     }
 
-    // a PCG substage: sweep, cc_div, the solve graph, cc_correct, halo fill
-    int step_launches() override {
-        if (!pcg) return launches;
+    // the kernels of a step as its graph was captured; the three solves' iterations
+    // (the conditional nodes' bodies) by the last solve's count
+    int step_nodes = 0;
+    aeo_status count_nodes(cudaGraph_t gr) {
+        size_t n = 0;
+        CK(cudaGraphGetNodes(gr, nullptr, &n));
+        std::vector<cudaGraphNode_t> nodes(n);
+        CK(cudaGraphGetNodes(gr, nodes.data(), &n));
+        step_nodes = 0;
+        for (cudaGraphNode_t q : nodes) {
+            cudaGraphNodeType t;
+            const cudaError_t e = cudaGraphNodeGetType(q, &t);
+            if (e == cudaErrorUnknown) {   // the answer of this runtime for a conditional node
+                cudaGetLastError();
+                continue;
+            }
+            CK(e);
+            step_nodes += t == cudaGraphNodeTypeKernel;
+        }
+        return AEO_OK;
+    }
+    aeo_status step_launches(int* out) override {
+        cudaGraphExec_t ge;
+        if (aeo_status e = graph_for(false, &ge)) return e;
+        *out = step_nodes;
+        if (!pcg) return AEO_OK;
         aeo_mg_stats o{};
-        if (cudaStreamSynchronize(st) != cudaSuccess || aeo_mg_read_stats(mg, &o)) return 0;
-        return 3 * (4 + dyn_launches() + aeo_mg_launches_per_solve(mg, o.iterations)) + lag_launches() + tke_launches();
+        CK(cudaStreamSynchronize(st));
+        if (aeo_status e = aeo_mg_read_stats(mg, &o)) {
+            fail(std::string("launches_per_step: ") + aeo_mg_last_error(mg));
+            return e;
+        }
+        *out += 3 * (aeo_mg_launches_per_solve(mg, o.iterations) - aeo_mg_launches_per_solve(mg, 0));
+        return AEO_OK;
     }
 
     // the implicit IBM correction after every predictor (aeo_set_ibm)
@@ -925,7 +948,6 @@ struct Core : CoreBase {
         drop_graphs();   // the step graphs gain or lose the correction
         if (!mask) {
             ibm_mask = nullptr;
-            launches = 3 * (9 + dyn_launches()) + lag_launches() + tke_launches();
             return AEO_OK;
         }
         std::vector<unsigned char> m((size_t)g.nin);
@@ -941,7 +963,6 @@ struct Core : CoreBase {
         CK(cudaStreamSynchronize(st));
         ibm_mask = ibm_alloc;
         ibm_tau = tau;
-        launches = 3 * (10 + dyn_launches()) + lag_launches() + tke_launches();
         return AEO_OK;
     }
 
@@ -1697,8 +1718,10 @@ struct Core : CoreBase {
             cudaError_t ce = cudaStreamEndCapture(st, &gr);
             if (e) { if (gr) cudaGraphDestroy(gr); return e; }
             if (ce != cudaSuccess) { fail(std::string("graph capture: ") + cudaGetErrorString(ce)); return AEO_ERR_CUDA; }
-            cudaError_t ie = cudaGraphInstantiate(&ge, gr, 0);
+            if (!pick) e = count_nodes(gr);
+            cudaError_t ie = e ? cudaSuccess : cudaGraphInstantiate(&ge, gr, 0);
             cudaGraphDestroy(gr);
+            if (e) return e;
             if (ie != cudaSuccess) { ge = nullptr; fail(std::string("graph instantiate: ") + cudaGetErrorString(ie)); return AEO_ERR_CUDA; }
         }
         *out = ge;
@@ -2597,9 +2620,9 @@ aeo_status aeo_profile_step(aeo_sim* h, double dt, double* ms_per_class, int32_t
 }
 
 aeo_status aeo_launches_per_step(aeo_sim* h, int32_t* out) {
-    if (!h || !out) return AEO_ERR_ARGUMENT;
-    *out = h->core->step_launches();
-    return AEO_OK;
+    ENTER(h);
+    if (!out) { h->core->fail("launches_per_step: NULL argument"); return AEO_ERR_ARGUMENT; }
+    return h->core->step_launches(out);
 }
 
 void* aeo_stream(aeo_sim* h) { return h ? (void*)h->core->st : nullptr; }

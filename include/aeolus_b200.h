@@ -262,8 +262,8 @@ aeo_status aeo_advect_positive(aeo_sim* h, const double* u, const double* v, con
 aeo_status aeo_advect_positive_device(aeo_sim* h, const void* u, const void* v, const void* w, const void* phi,
                                       void* tend, double dt, int32_t scheme, int32_t accumulate);
 
-/* Number of kernel launches one RK3 step issues (for launch accounting).
-   solver = AEO_SOLVER_PCG: counted with the iteration count of the last
+/* Number of kernel launches one RK3 step issues (for launch accounting),
+   counted in the step's captured graph.  solver = AEO_SOLVER_PCG: counted with the iteration count of the last
    pressure solve for all three substages (synchronises the stream). */
 aeo_status aeo_launches_per_step(aeo_sim* h, int32_t* out);
 
