@@ -1,4 +1,4 @@
-"""launches_per_step against the kernels that the runtime's trace of a step holds."""
+"""launches_per_step, and what bench.py counts for a solve and a tracer, against the kernels that the runtime's trace of a step holds."""
 import numpy as np
 import pytest
 
@@ -43,3 +43,31 @@ def test_launches_of_a_step_are_the_traced_ones(kw, size):
     got = traced(lambda: s.step_rk3(1e-4))
     assert len(got) == s.launches_per_step(), sorted(got)
     assert count in (None, len(got))
+
+
+@pytest.mark.parametrize("precond", ["vcycle", "jacobi", "identity"])
+def test_launches_of_a_solve(precond):
+    """Two kernels to begin with, two for the mean's shift, and the iterations between them."""
+    import torch
+    from aeolus_b200.multigrid import MGPreconditionedCG
+    n = (32, 16, 8)
+    s = MGPreconditionedCG(n, (1.0,) * 3, tol=1e-8, maxit=200, precond=precond)
+    b = torch.randn(n[::-1], dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    x = torch.empty_like(b)
+    s.solve_device(b.data_ptr(), x.data_ptr())
+    stats = []
+    got = traced(lambda: stats.append(s.solve_device(b.data_ptr(), x.data_ptr())))
+    assert len(got) == 4 + stats[0]["iterations"] * s.launches_per_iteration, sorted(got)
+
+
+def test_launches_of_a_tracer():
+    import torch
+    from aeolus_b200.simulation import Simulation
+    g = regular_grid((64, 16, 16), (1.0, 1.0, 1.0))
+    s = Simulation(CoreSpec(grid=g))
+    a = [torch.rand(g.storage_shape, dtype=torch.float64, device="cuda") for _ in range(4)]
+    t = torch.zeros_like(a[0])
+    go = lambda: (s.advect_positive_device(*a, t, 1e-3, "weno_z5", accumulate=False), s.synchronize())
+    go()
+    got = traced(go)
+    assert len(got) == 2, got
