@@ -222,11 +222,16 @@ struct Met {
     __device__ __forceinline__ R spf(int k) const { return lv(LV_SPF, k); }
 };
 
-// 1/x for x in the normal range (the WENO weights' denominators, the Poisson
-// eigenvalues).  FP32: rcp.approx (1 ulp).  FP64: the hardware's approximation
-// (its upper 32 bits, 20 bits good) and one third-order step of Newton's
-// series, r (1 + e + e^2) with e = 1 - x r: the error e^3 is below 2^-53.  Four
-// operations and no branch, against the ten-odd of an IEEE division.
+// 1/x (the WENO weights' denominators, the Poisson eigenvalues).  FP32:
+// rcp.approx (1 ulp).  FP64: the hardware's approximation, taken from and
+// given in the upper 32 bits (|e| < 2^-19, e = 1 - x r), and the geometric
+// series' first three terms, r (1 + e + e^2): what is left out is e^3 < 2^-57 of
+// the result, the two inner roundings are below 2^-70 of it and the last one is
+// half an ulp, together less than 0.57 ulp.  (Measured over all exponents: 0.93
+// and 0.501 ulp.)  Four operations and no branch, against the ten-odd of an IEEE
+// division.  For normal x whose reciprocal is
+// normal: subnormal numbers count as 0, beyond that range FP32 gives 0 or inf
+// and FP64 0 for a subnormal reciprocal and NaN for a subnormal, zero or infinite x.
 __device__ __forceinline__ float wrcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

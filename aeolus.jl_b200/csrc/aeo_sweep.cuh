@@ -71,7 +71,9 @@ struct WScalar { using type = VT; };   // the scalar type of a value or of a pai
 //   4 beta_2 = (3c - d)^2 + 13/3 (d - c)^2,
 // so the value is v3 plus a weighted mean of differences: a uniform field
 // comes back exactly, and the whole takes 40 operations (weights' scale 4 is
-// exact and cancels in tau / (beta + eps)).
+// exact and cancels in tau / (beta + eps)).  4 beta is at most 33.4 times the
+// largest difference squared and has to have a normal reciprocal: differences
+// below 1.5e18 in FP32.
 template <class VT, int ADV>
 __device__ __forceinline__ VT weno5_left(VT v1, VT v2, VT v3, VT v4, VT v5) {
     using R = typename WScalar<VT>::type;
