@@ -25,7 +25,7 @@
 // nx (ny+1) nz, nx ny (nz+1)); R on the interior cells.
 #pragma once
 
-#include "aeo_sweep_wpair.cuh"   // PairVal, the paired reconstruction
+#include "aeo_sweep_wpair.cuh"   // the paired reconstruction
 
 struct PosGeo {
     int nx, ny, nz, hx, hy, hz;
@@ -47,7 +47,8 @@ __device__ __forceinline__ long long pos_sidx(const PosGeo& g, int i, int j, int
 // that the ratios read no flux from memory and form no L twice.
 // Bound by the reconstruction's instructions (three faces a cell).
 template <typename R> struct PosTile {
-    static constexpr int N = PairVal<R>::N, TX = 32 * N, TY = 8, ROWT = 32 * TY, THREADS = ROWT + 32;
+    using VT = typename std::conditional<sizeof(R) == 4, F2, double>::type;   // a thread's values
+    static constexpr int N = sizeof(R) == 4 ? 2 : 1, TX = 32 * N, TY = 8, ROWT = 32 * TY, THREADS = ROWT + 32;
     static constexpr int PW = TX + 6, PH = TY + 6, PSZ = PW * PH, RING = 5;
 };
 template <typename R, int S>
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(PosTile<R>::THREADS, 2) pos_flux_ratio_kernel(
     const double* __restrict__ dtp, int zc, R* __restrict__ Fx, R* __restrict__ Fy, R* __restrict__ Fz,
     R* __restrict__ Rr) {
     using T = PosTile<R>;
-    using VT = typename PairVal<R>::VT;
+    using VT = typename T::VT;
     constexpr int N = T::N;
     __shared__ R ring[T::RING][T::PSZ];
     __shared__ R xFs[2][T::TY][T::TX + 1], xLs[2][T::TY][T::TX + 1], yFs[2][T::TY + 1][T::TX], yLs[2][T::TY + 1][T::TX];

@@ -1405,17 +1405,17 @@ struct Core : CoreBase {
                 constexpr int CLOS = cl;
                 constexpr bool kap = CLOS == 1 || CLOS == 3;
                 SweepArgs<R> b = a;
-                using PS = PairShape<R, SG>;
-                using TS = TileShape<R, ADV, SG>;
                 if constexpr (ADV == 0 && sizeof(R) == sizeof(float)) {
-                    // centred FP32 (FP64 here moved the stretched layer's pressure by 3.5e-12), persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
+                    // centred FP32, persistent: the SMs' worth of CTAs, each an equal range of (tile, level) items
+                    using PS = PairShape<SG>;
                     const int ntx = (g.nx + PS::TX - 1) / PS::TX, nty = (g.ny + PS::TY - 1) / PS::TY;
                     const int items = ntx * nty * g.nz;
                     const dim3 grid((unsigned)std::min(items, PS::CTAS_PER_SM * nsm));
                     if (kap) b.kofs = PS::KT_OFS;
-                    sweep_go(sweep_pair_kernel<R, SG, AN, UN, CLOS>, grid, dim3(PS::TXT, PS::TY),
+                    sweep_go(sweep_pair_kernel<SG, AN, UN, CLOS>, grid, dim3(PS::TXT, PS::TY),
                              kap ? PS::SMEM_AMD : PS::SMEM, tmaps[s_in], b, ntx, items, d_flag);
                 } else {
+                    using TS = TileShape<R, ADV, SG>;
                     const dim3 grid((g.nx + TS::TX - 1) / TS::TX, (g.ny + TS::TY - 1) / TS::TY, (g.nz + kchunk - 1) / kchunk);
                     if (kap) b.kofs = TS::KT_OFS;
                     sweep_go(sweep_tile_kernel<R, ADV, SG, AN, UN, CLOS>, grid, dim3(TS::NT), kap ? TS::SMEM_AMD : TS::SMEM,
