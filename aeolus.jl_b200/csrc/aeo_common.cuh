@@ -223,15 +223,15 @@ struct Met {
 };
 
 // 1/x (the WENO weights' denominators, the Poisson eigenvalues).  FP32:
-// rcp.approx (1 ulp).  FP64: the hardware's approximation, taken from and
-// given in the upper 32 bits (|e| < 2^-19, e = 1 - x r), and the geometric
-// series' first three terms, r (1 + e + e^2): what is left out is e^3 < 2^-57 of
-// the result, the two inner roundings are below 2^-70 of it and the last one is
-// half an ulp, together less than 0.57 ulp.  (Measured over all exponents: 0.93
-// and 0.501 ulp.)  Four operations and no branch, against the ten-odd of an IEEE
-// division.  For normal x whose reciprocal is
-// normal: subnormal numbers count as 0, beyond that range FP32 gives 0 or inf
-// and FP64 0 for a subnormal reciprocal and NaN for a subnormal, zero or infinite x.
+// rcp.approx (1 ulp).  FP64: the hardware's approximation, taken from and given
+// in the upper 32 bits (|e| < 2^-19, e = 1 - x r), and the geometric series'
+// first three terms, r (1 + e + e^2): what is left out is e^3 < 2^-57 of the
+// result, the two inner roundings are below 2^-70 of it and the last one is half
+// an ulp, together less than 0.57 ulp.  (Measured over all exponents: 0.93 and
+// 0.501 ulp.)  Four operations and no branch, against the ten-odd of an IEEE
+// division.  For normal x whose reciprocal is normal: subnormal numbers count as
+// 0, beyond that range FP32 gives 0 or inf, FP64 0 for a subnormal reciprocal and
+// NaN for a subnormal, zero or infinite x.
 __device__ __forceinline__ float wrcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

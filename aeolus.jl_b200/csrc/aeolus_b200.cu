@@ -195,7 +195,7 @@ struct Core : CoreBase {
     std::vector<double> h_dzc, h_dzf, h_wc, h_wf;
     double dz_min = 0.0;
     cudaGraphExec_t gexec[2][2] = {};   // [with CFL pick][parity of cur]
-    // n steps as one launch: a WHILE node over pairs of steps [parity of cur],
+    // PCG: n steps as one launch, a WHILE node over pairs of steps [parity of cur],
     // its body captured on st_loop, the pair count in d_steps
     cudaGraphExec_t gmulti[2] = {};
     cudaStream_t st_loop = nullptr;
@@ -1728,11 +1728,11 @@ struct Core : CoreBase {
         return AEO_OK;
     }
 
-    // The graph of n steps: WHILE(pairs left) { step cur -> cur^1; step cur^1 -> cur }.
+    // The graph of n PCG steps: WHILE(pairs left) { step cur -> cur^1; step cur^1 -> cur }.
     aeo_status multi_graph_for(cudaGraphExec_t* out) {
         cudaGraphExec_t& ge = gmulti[cur];
         if (!ge) {
-            if (pcg) CK(cudaDeviceSynchronize());   // as graph_for: the handle's set-up is complete
+            CK(cudaDeviceSynchronize());   // as graph_for: the handle's set-up is complete
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
             aeo_status e = AEO_OK;
             cudaError_t ce = cudaSuccess;

@@ -142,10 +142,11 @@ aeo_status aeo_get_field_f32(aeo_sim* h, int32_t field, float* host);
 
 /* nsteps projected SSP-RK3 steps of size dt: step_rk3! of the Boussinesq
  * core (src/Simulations.jl:843-904) or of the sound-proof core
- * (src/Anelastic.jl:1905-1948).  The whole step is one CUDA graph; with
- * nsteps >= 2 the pairs of steps run as one launch of a graph whose
- * conditional WHILE node loops over a two-step body (an odd last step is
- * launched on its own), bit-identical to single steps. */
+ * (src/Anelastic.jl:1905-1948).  The whole step is one CUDA graph, launched
+ * nsteps times.  With solver = AEO_SOLVER_PCG and nsteps >= 2 the pairs of
+ * steps run as one launch of a graph whose conditional WHILE node loops over a
+ * two-step body (an odd last step is launched on its own), bit-identical to
+ * single steps. */
 aeo_status aeo_step_rk3(aeo_sim* h, double dt, int32_t nsteps);
 
 /* nsteps forward-Euler projection steps: step! (src/Simulations.jl:481-650,
@@ -219,7 +220,9 @@ aeo_status aeo_kinetic_energy(aeo_sim* h, double* out);
 aeo_status aeo_max_divergence(aeo_sim* h, double* out);
 
 /* Device-resident stepping for benchmarks and graph-captured drivers: the
- * same as aeo_step_rk3 but returns without synchronising the stream. */
+ * same as aeo_step_rk3 but returns without synchronising the stream, once its
+ * launches are enqueued (a run of so many direct-solver steps that the stream's
+ * launch queue fills up waits for room in it). */
 aeo_status aeo_step_rk3_async(aeo_sim* h, double dt, int32_t nsteps);
 aeo_status aeo_synchronize(aeo_sim* h);
 

@@ -165,7 +165,7 @@ def test_column_projection_at_every_row_length(size, core, stretched):
     assert rel(s64.pressure_solve(b), o.pressure_solve(b)) <= 1e-12
 
 
-# ---- the Thomas solve from both ends: every remainder of its unrolled loops ------------------------------------
+# ---- the column solve: depths below, at and above its ring of levels --------------------------------------------
 @pytest.mark.parametrize("nz", [2, 3, 4, 5, 6, 7, 8, 9, 15, 16, 17, 31, 64, 93])
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("fp32_mixed", 1e-4)])
 def test_column_solve_of_every_depth(nz, precision, tol):
@@ -176,7 +176,7 @@ def test_column_solve_of_every_depth(nz, precision, tol):
     assert rel(s.pressure_solve(b), o.pressure_solve(b)) <= tol
 
 
-# ---- the centred sweeps: persistent CTAs over (tile, level) items, 64 (FP32) or 32 (FP64) columns by 8 rows -----
+# ---- the centred sweeps: FP32 persistent CTAs over (64 x 8 tile, level) items, FP64 32 x 8 tiles in chunks of levels
 @pytest.mark.parametrize("size,wall", [((8, 4, 5), True), ((32, 8, 4), False), ((64, 16, 13), True), ((128, 4, 33), True),
                                        ((32, 32, 64), False)])
 @pytest.mark.parametrize("sgs", [None, "smagorinsky", "vreman", "sigma", "dynamic", "amd"])
@@ -305,7 +305,7 @@ def test_positive_tendency_over_ragged_tiles(size, scheme):
                 assert (phi + dt * got)[g.interior].min() >= -1e-14
 
 
-# ---- the halo written with the correction (nz >= 4) or by the shell's fill, where rows and columns have several images
+# ---- the halo fill where rows and columns have several images ----------------------------------------------------
 @pytest.mark.parametrize("size,bc_z", [((4, 4, 4), "periodic"), ((4, 4, 4), "wall"), ((8, 4, 8), "periodic"),
                                        ((4, 8, 5), "wall"), ((16, 4, 3), "wall"), ((8, 8, 2), "wall"), ((64, 32, 7), "wall")])
 @pytest.mark.parametrize("scheme", ["centred", "weno_z5"])
@@ -369,18 +369,21 @@ def test_host_arrays_pageable_pinned_and_from_threads(shape):
 
 
 @pytest.mark.parametrize("steps", [1, 2, 3, 5])
-def test_a_run_of_steps_is_its_single_steps(steps):
-    """Direct solvers launch a graph a step, the PCG solver a graph of pairs: both are the single steps' bits."""
+@pytest.mark.parametrize("kw", [{}, {"precision": "fp32_mixed"}, {"solver": "pcg"}], ids=lambda kw: "-".join(kw.values()))
+def test_a_run_of_steps_against_the_oracle(steps, kw):
+    """The direct solvers' graph a step and the PCG solver's graph of pairs: the state after a run of odd and even
+    length, p included (written in a step's last substage only), is the oracle's."""
     g = regular_grid((16, 16, 8), (1.0, 1.0, 1.0), bc_z="wall")
-    for kw in ({}, {"precision": "fp32_mixed"}, {"solver": "pcg"}):
-        out = []
-        for calls in ([steps], [1] * steps):
-            s = Sim(CoreSpec(grid=g, nu=1e-3, **kw))
-            if "solver" in kw:
-                s.set_pcg(None, tol=1e-8, maxit=100)
-            s.set_state(*random_state(g, 9, 0.3))
-            s.project()
-            for n in calls:
-                s.step_rk3(1e-3, n)
-            out.append([s.get_field(n) for n in ("u", "v", "w", "theta", "p")])
-        assert all(np.array_equal(a, b) for a, b in zip(*out))
+    s, o = Sim(CoreSpec(grid=g, nu=1e-3, **kw)), OracleSimulation(CoreSpec(grid=g, nu=1e-3, solver=kw.get("solver")))
+    for q in (s, o):
+        if "solver" in kw:
+            q.set_pcg(None, tol=1e-12, maxit=100)
+        q.set_state(*random_state(g, 9, 0.3))
+        q.project()
+        q.step_rk3(1e-3, steps)
+    fp64 = "precision" not in kw
+    for n in ("u", "v", "w", "theta", "p"):
+        want = o.get_field(n)[g.interior]
+        # the pressure is phi / dt: the solve's tolerance (1e-12 of the divergence) or the FP32 divergence's rounding over it
+        tol = (1e-11 if n != "p" else 1e-8) if fp64 else (1e-5 if n != "p" else 1e-3)
+        assert rel(s.get_field(n)[g.interior], want) <= tol, n
