@@ -293,6 +293,9 @@ __global__ void pcg_init_kernel(const double* __restrict__ b, double* __restrict
         if (S->bnorm == 0.0) {
             S->status = MG_ZERO_RHS;
             S->done = 3;
+        } else if (S->rnorm <= S->tol * S->bnorm) {   // a tolerance of 1 or more: before the first iteration, and without one
+            S->status = MG_CONVERGED;
+            S->done = 1;
         } else {
             S->status = MG_MAXIT;
             S->done = 0;
@@ -462,12 +465,6 @@ __global__ void pcg_rz_kernel(const double* __restrict__ r, const Z* __restrict_
         if (first) {
             S->rz = rzn;
             S->beta = 0.0;
-            S->rnorm = sqrt(t[0]);
-            S->rprev = S->rnorm;
-            if (S->rnorm <= S->tol * S->bnorm) {
-                S->status = MG_CONVERGED;
-                S->done = 1;
-            }
         } else {
             if (flex) {
                 double zAp = t[4] - (S->project ? m * t[5] : 0.0);

@@ -280,8 +280,10 @@ def test_cg_loop_counts_and_ends(n, precond):
         assert st["status"] == "converged" and st["residual"] <= 1e-6 * st["bnorm"]
     x, st = s.solve(np.zeros_like(b))
     assert st["status"] == "zero_rhs" and st["iterations"] == 0 and not x.any()
-    x, st = make(tol=2.0, maxit=5).solve(b)
-    assert st["status"] == "converged" and st["iterations"] == 0 and not x.any()
+    for tol, maxit, status in ((2.0, 5, "converged"), (1.0, 1, "converged"), (2.0, 0, "converged"), (0.5, 0, "maxit")):
+        x, st = make(tol=tol, maxit=maxit).solve(b)
+        assert st["status"] == status and st["iterations"] == 0 and not x.any(), (tol, maxit)
+        assert st["residual"] == st["bnorm"] > 0
 
 
 # ---- the positivity-preserving advection: tiles of 64 (FP32) or 32 columns by 8 rows, chunks of levels ----------
