@@ -4,17 +4,19 @@
 // on the calling thread, 11 GB/s on the hosts measured; the link does 50.  Here a
 // few threads copy the array's chunks into pinned buffers (two a thread) and
 // enqueue each chunk's transfer, so that the host copy runs at the memory's
-// rate and overlaps the link.  Arrays that are small or already pinned take the
-// plain call.
+// rate and overlaps the link.  Arrays that are already pinned take the plain call,
+// and so do those below SMALL, where starting the threads costs what they save: an
+// apply of the network, two copies (ms, plain and by lanes), takes 0.63 and 0.74 on
+// arrays of 2.1 MB, 1.43 and 1.47 on 6.3, 2.15 and 1.98 on 12.6, 3.98 and 3.15 on 25,
+// 16.8 and 7.0 on 50.
 //
 // The pinned buffers (LANES x 2 x CHUNK, 12 MiB) belong together to the live handles
 // that have use for them: the first such handle pins them, the last one gives them back,
 // and one copy at a time uses them (a copy that finds them in use goes the plain way).
 // Pinning huge pages and giving them back takes 3.0 ms (7.2 ms by cudaHostAlloc), what the
-// lanes save on PAYS bytes (6.3 MB go up in 0.59 ms and down in 0.40 ms by the plain call);
-// a handle asks for them once its pageable copies come to that much.  So creating a handle
-// pins nothing, one that copies little pays for nothing, and where pinned memory is refused
-// the plain call serves.
+// lanes save on 30 to 80 MB of 50 MB arrays; a handle asks for them once its pageable
+// copies come to PAYS.  So creating a handle pins nothing, one that copies little pays for
+// nothing, and where pinned memory is refused the plain call serves.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,7 +33,7 @@
 
 class HostStage {
 public:
-    static constexpr size_t CHUNK = size_t(1) << 20, SMALL = size_t(2) << 20, PAYS = size_t(40) << 20;
+    static constexpr size_t CHUNK = size_t(1) << 20, SMALL = size_t(8) << 20, PAYS = size_t(40) << 20;
     static constexpr int LANES = 6;
 
     // src (host) -> dst (device) on st; returns when a pageable src has been read

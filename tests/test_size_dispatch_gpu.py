@@ -335,7 +335,7 @@ def test_unet_gradients_where_every_level_takes_x_segments(shape):
 
 
 
-@pytest.mark.parametrize("shape", [(128, 16, 8), (128, 64, 32), (128, 48, 44), (256, 64, 56)])
+@pytest.mark.parametrize("shape", [(128, 16, 8), (128, 64, 32), (256, 64, 56), (512, 64, 32), (256, 48, 92)])
 def test_host_arrays_pageable_pinned_and_from_threads(shape):
     """Below and above the size that takes the pinned lanes, whole and ragged chunks, as often as it takes until a
     handle uses the lanes: the same bits as from pinned arrays, and from several handles at once."""
