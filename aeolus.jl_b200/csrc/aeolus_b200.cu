@@ -344,13 +344,17 @@ struct Core : CoreBase {
     }
     // the limited tendency of a[3] in the flow a[0 .. 2]: chunks of levels such that the tiles
     // fill the SMs several times over, at least eight levels each (a chunk computes one z
-    // face more than it has levels)
+    // face more than it has levels); where that leaves SMs without a CTA, as many chunks as
+    // make one wave: there the levels of a chunk, one after the other, are what a call waits for
+    // (FP32 32^3: 37 us in chunks of eight levels, 23 in chunks of one; 64^3: 40 and 29)
     template <int SCH>
     void launch_positive(const PosGeo& pg, const R* const* a, const double* dtp, R* tend, int accumulate) {
         using T = PosTile<R>;
         const unsigned tx = (unsigned)((g.nx + T::TX - 1) / T::TX), ty = (unsigned)((g.ny + T::TY - 1) / T::TY);
-        const int want = (int)((16LL * nsm + (long long)tx * ty - 1) / ((long long)tx * ty));
-        const int nc = std::max(1, std::min(want, g.nz / 8)), zc = (g.nz + nc - 1) / nc;
+        const long long tiles = (long long)tx * ty;
+        const int want = (int)((16LL * nsm + tiles - 1) / tiles);
+        const int wave = (int)std::min<long long>(g.nz, 2LL * nsm / tiles);   // two CTAs an SM
+        const int nc = std::max({1, std::min(want, g.nz / 8), wave}), zc = (g.nz + nc - 1) / nc;
         const dim3 grid(tx, ty, (unsigned)((g.nz + zc - 1) / zc));
         pos_flux_ratio_kernel<R, SCH><<<grid, T::THREADS, 0, st>>>(pg, a[0], a[1], a[2], a[3], dtp, zc, pos_fx, pos_fy, pos_fz, pos_r);
         pos_apply_kernel<R><<<grid, T::THREADS, 0, st>>>(pg, a[0], a[1], a[2], a[3], pos_fx, pos_fy, pos_fz, pos_r, zc, tend, accumulate);

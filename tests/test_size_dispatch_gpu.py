@@ -286,9 +286,10 @@ def test_cg_loop_counts_and_ends(n, precond):
         assert st["residual"] == st["bnorm"] > 0
 
 
-# ---- the positivity-preserving advection: tiles of 64 (FP32) or 32 columns by 8 rows, chunks of levels ----------
+# ---- the positivity-preserving advection: tiles of 64 (FP32) or 32 columns by 8 rows, chunks of one level (few tiles)
+# to a dozen, whole and ragged
 @pytest.mark.parametrize("size", [(8, 4, 3), (16, 8, 9), (64, 8, 8), (32, 16, 33), (128, 32, 40), (64, 4, 70),
-                                  (256, 4, 24)])
+                                  (256, 4, 24), (128, 64, 25), (256, 128, 40), (256, 64, 100)])
 @pytest.mark.parametrize("scheme", ["weno_z5", "weno_js5"])
 def test_positive_tendency_over_ragged_tiles(size, scheme):
     g = regular_grid(size, (1.0, 0.8, 0.6), bc_z="wall")
