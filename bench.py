@@ -61,12 +61,11 @@ import numpy as np  # noqa: E402
 
 HBM_FALLBACK_GBS = 6650.0
 # DRAM bytes (read + write) of one sweep launch of the CBL 256x256x128 FP32-mixed
-# step, from an ncu capture of `python bench.py --steps 2 --warmup 3`
-# (profiles/sweep_pair_kernel_cbl256_fp32.md)
-CBL_SWEEP_DRAM_BYTES = 315824640 + 109399552
+# step, from an ncu capture (profiles/sweep_pair_kernel_cbl256_fp32.md)
+CBL_SWEEP_DRAM_BYTES = 317773312 + 108520192
 # ... and of one finest red-black colour pass of the urban 256x256x96 FP32-mixed
-# solve (profiles/mg_vcycle_urban256x256x96_fp32.md): 69.4 MB read + 1.3 MB written
-URBAN_RBGS_DRAM_BYTES = 70.7e6
+# solve (profiles/mg_vcycle_urban256x256x96_fp32.md): 69.3 MB read + 1.3 MB written
+URBAN_RBGS_DRAM_BYTES = 70.6e6
 
 
 # ----------------------------------------------------------------------------- workloads
